@@ -204,7 +204,7 @@ LinePart make_part(int L, int nlines) {
     LinePart lp;
     lp.L = L;
     lp.nlines = nlines;
-    lp.red0 = 0;
+    lp.red0 = lp.pcr0 = 0;
     // chunks of at least 16 rows and at most 256 chunks per line (the
     // reduced system of 2P rows is solved by one block)
     lp.m = std::max(16, (L + 255) / 256);
@@ -654,6 +654,8 @@ int fw_create(const fw_params *p, fw_ctx **out) {
     c->py = make_part(p->Nglob, p->Mglob);
     c->px.red0 = 0;
     c->py.red0 = (long long)c->px.nlines * 2 * c->px.P * 6;
+    c->px.pcr0 = 0;
+    c->py.pcr0 = fw::lsf_line(c->px) ? (long long)c->px.nlines * fw::pcr_words(c->px) : 0;
     c->ncand_cap = (p->Mglob + 2) * (p->Nglob + 2);
     // the factored solve assumes tmp2 = 1 + Gamma1*MASK9*(-b1-2*b2)/h^2*dep^2
     // never vanishes, which holds for -b1-2*b2 >= 0 (Beta_ref in [-2, 0])
@@ -1316,11 +1318,15 @@ int fw_sync(fw_ctx *c) {
 namespace {
 
 const char kCkMagic[8] = {'F', 'W', 'C', 'K', 'P', 'T', '0', '1'};
+// 0: every factor at its cell; 1: x factors chunk-interleaved (fw::fac_at),
+// the reduction's multipliers kept (fw::pcr_factor)
+const int32_t kCkFactors = 1;
 
 struct CkHeader {
     char magic[8];
     uint32_t sizeof_params, sizeof_grid;
-    int32_t precision, pad;
+    int32_t precision;
+    int32_t factors;  // layout of the line solver's factors in the arena (kCkFactors)
     uint64_t arena_bytes, band_bytes;  // band_bytes: each of Cm and Sm
     int64_t off_mask, off_maskn, off_age, off_agen;
     double EtaBlowVal;
@@ -1447,6 +1453,7 @@ int fw_checkpoint(fw_ctx *c, const char *path) {
     h.sizeof_params = (uint32_t)sizeof(fw_params);
     h.sizeof_grid = (uint32_t)sizeof(Grid);
     h.precision = c->p.precision;
+    h.factors = kCkFactors;
     h.arena_bytes = c->arena_bytes;
     h.band_bytes = band_bytes(c, c->g);
     h.EtaBlowVal = c->EtaBlowVal;
@@ -1538,6 +1545,11 @@ int fw_restore(fw_ctx *c, const char *path) {
     }
     c->g = g;
     c->EtaBlowVal = h.EtaBlowVal;
+    if (h.factors != kCkFactors) {
+        // another layout's factors: factor again at the next solve
+        const int one = 1;
+        if ((rc = upload_array(c, fp64 ? c->fd.m9_dirty : c->ff.m9_dirty, &one, sizeof(one))) != FW_OK) return rc;
+    }
     if (c->graph) {
         cudaGraphExecDestroy(c->graph);
         c->graph = nullptr;

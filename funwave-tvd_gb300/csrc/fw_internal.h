@@ -75,7 +75,8 @@ struct Fields {
     T *Depth, *Depthx, *Depthy, *Cd, *SPONGE, *CD4;
     T *P, *Q, *Fx, *Fy, *Gx, *Gy;
     T *A, *B, *C, *E;                 // mixed: exchanged Uxx+Vxy, DUxx+DVxy, Uxy+Vyy, DUxy+DVyy
-    T *Uxx, *Vxy, *Uxy, *Vyy, *DUxx, *DVxy, *DUxy, *DVyy;  // FP64: the exchanged terms themselves
+    // FP64: the exchanged terms themselves; mixed: the line solver's reduction multipliers
+    T *Uxx, *Vxy, *Uxy, *Vyy, *DUxx, *DVxy, *DUxy, *DVyy;
     T *U4, *V4, *U1p, *V1p, *Udisp, *Vdisp;  // Udisp = U1pp+U2+U3
     T *ETAx, *ETAy, *ETAT;
     T *AGE, *AGEn, *nu;               // AGE ping-pong (old / new)
@@ -141,6 +142,7 @@ struct LinePart {
     int P;       // chunks per line
     long long red0;  // offset (doubles) of this direction's rows in the factorisation scratch
     int lgm;         // log2(m) when m is a power of two, else -1
+    long long pcr0;  // offset (floats) of this direction's reduction multipliers (mixed)
 };
 
 // launchers (fw_kernels.cu), all asynchronous on the context stream
@@ -173,6 +175,20 @@ void convert_out_f32(fw_ctx *c, const double *field, float *staging, int w, int 
 
 // Host context behind the opaque C handle.
 namespace fw {
+// rows of a chunk of the lines that k_linesolve takes (32 to 4096 rows, and 16)
+constexpr int LSF_M = 16;
+__host__ __device__ __forceinline__ bool lsf_line(const LinePart &lp) { return lp.m == LSF_M; }
+// the cyclic reduction of n = 2P reduced rows: its steps, and the words that
+// one line's multipliers take (pcr_factor)
+__host__ __device__ __forceinline__ int pcr_steps(int n) {
+    int st = 0;
+    while ((1 << st) < n) st++;
+    return st;
+}
+__host__ __device__ __forceinline__ int pcr_words(const LinePart &lp) {
+    const int n = 2 * lp.P;
+    return (2 * pcr_steps(n) + 1) * ((n + 3) & ~3);
+}
 // tensor maps of the flux kernels' TMA-staged tiles: U V HU HV Eta U4 V4 and
 // MASK, for one direction and tile height (the box shape is part of a map)
 // and one of the two MASK buffers

@@ -1596,6 +1596,17 @@ __device__ __forceinline__ void tri_ac_row(const Grid &g, const Fields<T> &f, co
     }
 }
 
+// where row k of line l keeps its factors: its cell, except that the x lines
+// of LSF_M-row chunks keep the rows of equal offset in their chunks side by
+// side, so that neighbouring threads, which own neighbouring chunks, load
+// neighbouring words; the last chunk's rows past LSF_M keep their place
+template <int DIR> __device__ __forceinline__ size_t fac_at(const Grid &g, const LinePart &lp, int l, int k) {
+    if (DIR == 1) return IDX(g.ib + l, g.jb + k);
+    const size_t row = (size_t)(g.jb + l) * g.pitch;
+    if (lp.m != LSF_M) return row + g.ib + k;
+    return row + (k < LSF_M * lp.P ? (k % LSF_M) * lp.P + k / LSF_M : k);
+}
+
 __device__ __forceinline__ void split2(double v, float &hi, float &lo) {
     hi = (float)v;
     lo = (float)(v - (double)hi);
@@ -1618,7 +1629,7 @@ __device__ __forceinline__ void fac_a_body(const Grid &g, const Fields<T> &f, co
         tri_ac<T, DIR>(g, f, i, j, a, c, it);
         if (!PER && k == 0) a = 0.0;
         if (!PER && k == lp.L - 1) c = 0.0;
-        const size_t q = IDX(i, j);
+        const size_t q = fac_at<DIR>(g, lp, l, k);
         split2(a, f.fac_ah[DIR][q], f.fac_al[DIR][q]);
         split2(c, f.fac_ch[DIR][q], f.fac_cl[DIR][q]);
         it_[q] = (float)it;
@@ -1626,11 +1637,12 @@ __device__ __forceinline__ void fac_a_body(const Grid &g, const Fields<T> &f, co
     double as, cs, its, ae, ce, ite;
     tri_ac_row<T, DIR, PER>(g, f, lp, l, s, as, cs, its);
     tri_ac_row<T, DIR, PER>(g, f, lp, l, e, ae, ce, ite);
-    int i, j;
-    line_cell<DIR>(g, l, s, i, j);
-    A_[IDX(i, j)] = 1.0f;
-    line_cell<DIR>(g, l, e, i, j);
-    A_[IDX(i, j)] = 1.0f;
+    // a chunk's first and last row: constants with which the sweeps pass them by
+    for (int k = s; k <= e; k += max(1, e - s)) {
+        const size_t q = fac_at<DIR>(g, lp, l, k);
+        A_[q] = 1.0f;
+        lr_[q] = cp_[q] = p_[q] = q_[q] = 0.0f;
+    }
     if (s == 0) as = 0.0;
     if (e == lp.L - 1) ce = 0.0;
     double lo_s, di_s, up_s, lo_e, di_e, up_e;
@@ -1646,8 +1658,7 @@ __device__ __forceinline__ void fac_a_body(const Grid &g, const Fields<T> &f, co
             cp = upper * r;
             pp = ((k == s + 1 ? a : 0.0) - lower * pp) * r;
             qp = ((k == e - 1 ? c : 0.0) - lower * qp) * r;
-            line_cell<DIR>(g, l, k, i, j);
-            const size_t q = IDX(i, j);
+            const size_t q = fac_at<DIR>(g, lp, l, k);
             A_[q] = (float)r;
             lr_[q] = (float)(lower * r);
             cp_[q] = (float)cp;
@@ -1657,8 +1668,7 @@ __device__ __forceinline__ void fac_a_body(const Grid &g, const Fields<T> &f, co
         }
         double pn = 0.0, qn = 0.0, p1 = 0.0, q1 = 0.0, pl = 0.0, ql = 0.0;
         for (int k = e - 1; k >= s + 1; k--) {
-            line_cell<DIR>(g, l, k, i, j);
-            const size_t q = IDX(i, j);
+            const size_t q = fac_at<DIR>(g, lp, l, k);
             const double cpk = cbuf[q];
             const double pk = pbuf[q] - cpk * pn, qk = qbuf[q] - cpk * qn;
             p_[q] = (float)pk;
@@ -1741,11 +1751,11 @@ __device__ __forceinline__ void fac_b_body(const Grid &g, const Fields<T> &f, co
         for (int k = 0; k < n; k++) {
             const double rhs = k == 0 ? 1.0 / (1.0 + c_end) : (k == n - 1 ? -1.0 / (1.0 + a_beg) : 0.0);
             z = (rhs - red[k * 6 + 3] * z) * red[k * 6 + 4];
-            red[k * 6 + 0] = z;
+            red[k * 6 + 4] = z;
         }
         double x = 0.0, x0 = 0.0, xl = 0.0;
         for (int k = n - 1; k >= 0; k--) {
-            x = red[k * 6 + 0] - red[k * 6 + 5] * x;
+            x = red[k * 6 + 4] - red[k * 6 + 5] * x;
             fl.x2[k] = (float)x;
             if (k == n - 1) xl = x;
             if (k == 0) x0 = x;
@@ -1756,10 +1766,72 @@ __device__ __forceinline__ void fac_b_body(const Grid &g, const Fields<T> &f, co
     }
 }
 
+// The multipliers of the parallel cyclic reduction of a line's reduced rows,
+// constant like the factors: per step a and b (n4 words each), then the last
+// diagonal; the operations are pcr_solve's.  They lie in the planes that only
+// the FP64 mode's dispersion terms use (eight consecutive planes from Uxx; at
+// most 19/8 words per cell and direction), x lines first.
+template <typename T, int DIR>
+__device__ __forceinline__ float *pcr_line(const Fields<T> &f, const LinePart &lp, int l) {
+    return (float *)f.Uxx + lp.pcr0 + (size_t)l * pcr_words(lp);
+}
+// one line by a block of 128 threads; sh: 6 x 2P words
+template <typename T, int DIR>
+__device__ void pcr_factor(const Fields<T> &f, const LinePart &lp, int l, float *sh) {
+    const int n = 2 * lp.P, n4 = (n + 3) & ~3;
+    const double *red = f.red + lp.red0 + (size_t)l * n * 6;
+    float *out = pcr_line<T, DIR>(f, lp, l);
+    float *lo = sh, *di = sh + n, *up = sh + 2 * n, *lo2 = sh + 3 * n, *di2 = sh + 4 * n, *up2 = sh + 5 * n;
+    __syncthreads();  // the previous line's readers
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        lo[k] = (float)((k > 0) ? red[k * 6 + 0] : 0.0);
+        di[k] = (float)red[k * 6 + 1];
+        up[k] = (float)((k < n - 1) ? red[k * 6 + 2] : 0.0);
+    }
+    __syncthreads();
+    for (int st = 1; st < n; st <<= 1) {
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            const int km = k - st, kp = k + st;
+            float a = 0.0f, b = 0.0f, nlo = 0.0f, nup = 0.0f;
+            float nd = di[k];
+            if (km >= 0) {
+                a = -lo[k] / di[km];
+                nlo = a * lo[km];
+                nd += a * up[km];
+            }
+            if (kp < n) {
+                b = -up[k] / di[kp];
+                nup = b * up[kp];
+                nd += b * lo[kp];
+            }
+            lo2[k] = nlo;
+            di2[k] = nd;
+            up2[k] = nup;
+            out[k] = a;
+            out[n4 + k] = b;
+        }
+        out += 2 * n4;
+        __syncthreads();
+        float *t;
+        t = lo; lo = lo2; lo2 = t;
+        t = di; di = di2; di2 = t;
+        t = up; up = up2; up2 = t;
+    }
+    for (int k = threadIdx.x; k < n; k += blockDim.x) out[k] = di[k];
+}
+
+// blocks [0, nb) factor the reduced rows, one line per thread; the others take
+// the reduction's multipliers, one line per block at a time (both read words
+// 0..2 of the reduced rows, and only the first write words 3..5)
 template <typename T, int DIR, bool PER>
-__global__ void __launch_bounds__(128) k_fac_b(Grid g, Fields<T> f, LinePart lp) {
+__global__ void __launch_bounds__(128) k_fac_b(Grid g, Fields<T> f, LinePart lp, int nb) {
+    extern __shared__ float shp[];
     if (!*f.m9_dirty) return;
-    fac_b_body<T, DIR, PER>(g, f, lp, blockIdx.x * blockDim.x + threadIdx.x);
+    if ((int)blockIdx.x < nb) {
+        fac_b_body<T, DIR, PER>(g, f, lp, blockIdx.x * blockDim.x + threadIdx.x);
+        return;
+    }
+    for (int l = blockIdx.x - nb; l < lp.nlines; l += gridDim.x - nb) pcr_factor<T, DIR>(f, lp, l, shp);
 }
 
 // both directions in one launch each: blocks [0, nbx) factor x, the rest y
@@ -1770,23 +1842,36 @@ __global__ void __launch_bounds__(128) k_fac_a_xy(Grid g, Fields<T> f, LinePart 
     else fac_a_body<T, 1, PERY>(g, f, py, (blockIdx.x - nbx) * blockDim.x + threadIdx.x);
 }
 template <typename T, bool PERY>
-__global__ void __launch_bounds__(128) k_fac_b_xy(Grid g, Fields<T> f, LinePart px, LinePart py, int nbx) {
+__global__ void __launch_bounds__(128) k_fac_b_xy(Grid g, Fields<T> f, LinePart px, LinePart py, int nbx, int nby) {
+    extern __shared__ float shp[];
     if (!*f.m9_dirty) return;
-    if ((int)blockIdx.x < nbx) fac_b_body<T, 0, false>(g, f, px, blockIdx.x * blockDim.x + threadIdx.x);
-    else fac_b_body<T, 1, PERY>(g, f, py, (blockIdx.x - nbx) * blockDim.x + threadIdx.x);
+    const int b = blockIdx.x - nbx - nby;
+    if ((int)blockIdx.x < nbx) {
+        fac_b_body<T, 0, false>(g, f, px, blockIdx.x * blockDim.x + threadIdx.x);
+    } else if (b < 0) {
+        fac_b_body<T, 1, PERY>(g, f, py, (blockIdx.x - nbx) * blockDim.x + threadIdx.x);
+    } else {
+        const int nx = lsf_line(px) ? px.nlines : 0, ny = lsf_line(py) ? py.nlines : 0;
+        for (int l = b; l < nx + ny; l += gridDim.x - nbx - nby) {
+            if (l < nx) pcr_factor<T, 0>(f, px, l, shp);
+            else pcr_factor<T, 1>(f, py, l - nx, shp);
+        }
+    }
 }
 
 static __global__ void k_fac_clear(int *dirty) { *dirty = 0; }
 
 // compensated r = d - (a x(k-1) + x(k) + c x(k+1)) with a = ah + al, c = ch + cl
+// Every operation is written as rounded (no contraction left to the
+// compiler), so that all callers get the same bits.
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-    s = a + b;
-    const float bb = s - a;
-    e = (a - (s - bb)) + (b - bb);
+    s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 __device__ __forceinline__ void two_prod(float a, float b, float &p, float &e) {
-    p = a * b;
-    e = fmaf(a, b, -p);
+    p = __fmul_rn(a, b);
+    e = __fmaf_rn(a, b, -p);
 }
 __device__ __forceinline__ float residual(float d, float x, float xm, float xp, float ah, float al, float ch,
                                           float cl) {
@@ -1796,7 +1881,8 @@ __device__ __forceinline__ float residual(float d, float x, float xm, float xp, 
     two_prod(ch, xp, v, e3);
     two_sum(t, -u, t2, e4);
     two_sum(t2, -v, t3, e5);
-    return t3 + ((((e1 + e4) + e5) - e2) - e3 - al * xm - cl * xp);
+    const float lo = __fsub_rn(__fsub_rn(__fadd_rn(__fadd_rn(e1, e4), e5), e2), e3);
+    return __fadd_rn(t3, __fmaf_rn(-cl, xp, __fmaf_rn(-al, xm, lo)));
 }
 
 // Parallel cyclic reduction of n reduced rows lo x(k-1) + di x(k) +
@@ -1852,10 +1938,7 @@ template <int PASS> __device__ __forceinline__ float *red_rhs(double *red, const
     return (float *)red + (PASS == 0 ? 0 : (size_t)lp.nlines * 2 * lp.P);
 }
 
-// M > 0: chunks of exactly M rows are walked in registers (all loads first,
-// the sweep values stored once); other chunks, and M = 0, walk the loop.
-// Both do the same operations in the same order.
-template <typename T, int DIR, bool PER, int PASS, int M>
+template <typename T, int DIR, bool PER, int PASS>
 __global__ void __launch_bounds__(128) k_sol_a(Grid g, Fields<T> f, LinePart lp) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= lp.nlines * lp.P) return;
@@ -1885,42 +1968,6 @@ __global__ void __launch_bounds__(128) k_sol_a(Grid g, Fields<T> f, LinePart lp)
     line_cell<DIR>(g, l, e, i, j);
     const float de = dval(e, IDX(i, j));
     float rs = ds, re = de;
-    if constexpr (M > 2) {
-        if (e - s + 1 == M) {
-            const size_t stride = DIR == 0 ? 1 : (size_t)g.pitch;
-            line_cell<DIR>(g, l, s, i, j);
-            const size_t q0 = IDX(i, j);
-            float dv[M], av[M], lv[M], cv[M], yv[M];
-#pragma unroll
-            for (int k = 1; k < M - 1; k++) {
-                const size_t q = q0 + (size_t)k * stride;
-                dv[k] = dval(s + k, q);
-                av[k] = A_[q];
-                lv[k] = lr_[q];
-                cv[k] = cp_[q];
-            }
-            float yp = 0.0f;
-#pragma unroll
-            for (int k = 1; k < M - 1; k++) {
-                yp = dv[k] * av[k] - lv[k] * yp;
-                yv[k] = yp;
-            }
-            float yn = 0.0f;
-#pragma unroll
-            for (int k = M - 2; k >= 1; k--) {
-                yn = yv[k] - cv[k] * yn;
-                yv[k] = yn;
-            }
-#pragma unroll
-            for (int k = 1; k < M - 1; k++) ys[q0 + (size_t)k * stride] = yv[k];
-            rs = ds - fl.cs[ch] * yv[1];
-            re = de - fl.ae[ch] * yv[M - 2];
-            float *red = red_rhs<PASS>(f.red, lp) + ((size_t)l * 2 * lp.P + 2 * ch);
-            red[0] = rs;
-            red[1] = re;
-            return;
-        }
-    }
     if (e - s >= 2) {
         float yp = 0.0f;
         for (int k = s + 1; k <= e - 1; k++) {
@@ -1968,9 +2015,8 @@ __global__ void __launch_bounds__(512) k_sol_b(Grid g, Fields<T> f, LinePart lp)
     for (int k = threadIdx.x; k < n; k += blockDim.x) red[k] = PER ? r[k] + beta * fl.x2[k] : r[k];
 }
 
-// PASS 0: x0 -> tp scratch; PASS 1: out = x0 + correction.  M > 0: chunks
-// of exactly M rows with all loads first (as k_sol_a).
-template <typename T, int DIR, int PASS, int M>
+// PASS 0: x0 -> tp scratch; PASS 1: out = x0 + correction
+template <typename T, int DIR, int PASS>
 __global__ void __launch_bounds__(128) k_sol_c(Grid g, Fields<T> f, LinePart lp) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= lp.nlines * lp.P) return;
@@ -1984,28 +2030,6 @@ __global__ void __launch_bounds__(128) k_sol_c(Grid g, Fields<T> f, LinePart lp)
     const float *ys = (const float *)f.ty;
     float *x0 = (float *)f.tp;
     T *out = DIR == 0 ? f.U : f.V;
-    if constexpr (M > 2) {
-        if (e - s + 1 == M) {
-            const size_t stride = DIR == 0 ? 1 : (size_t)g.pitch;
-            int i, j;
-            line_cell<DIR>(g, l, s, i, j);
-            const size_t q0 = IDX(i, j);
-            float xv[M], x0v[M];
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const size_t q = q0 + (size_t)k * stride;
-                xv[k] = (k == 0) ? xs : (k == M - 1) ? xe : ys[q] - p_[q] * xs - q_[q] * xe;
-                if (PASS == 1) x0v[k] = x0[q];
-            }
-#pragma unroll
-            for (int k = 0; k < M; k++) {
-                const size_t q = q0 + (size_t)k * stride;
-                if (PASS == 0) x0[q] = xv[k];
-                else out[q] = (T)(x0v[k] + xv[k]);
-            }
-            return;
-        }
-    }
     for (int k = s; k <= e; k++) {
         int i, j;
         line_cell<DIR>(g, l, k, i, j);
@@ -2048,14 +2072,8 @@ __host__ __device__ __forceinline__ size_t lsx_smem_floats(int L, int P) {
     return (size_t)6 * (lsx_pad(L) + 1) + (size_t)L + 16 * (size_t)P;
 }
 
-// KPT > 0: lines of at most 256 x KPT cells; every global value a thread
-// needs later (the reconstruction's p, q and the residual's a, c pairs of
-// its cells k = tid + 256 j, the reduced rows and the chunk's spike ends)
-// is loaded into registers at the start, together with the staging loads,
-// so that the block waits for global memory once instead of once per phase.
-// KPT = 0: any length, loads where they are used.
-template <typename T, int KPT>
-__global__ void __launch_bounds__(256, KPT > 0 ? 3 : 1) k_linesolve_x(Grid g, Fields<T> f, LinePart lp, int clear_dirty) {
+template <typename T>
+__global__ void __launch_bounds__(256) k_linesolve_x(Grid g, Fields<T> f, LinePart lp, int clear_dirty) {
     extern __shared__ float shf[];
     const int l = blockIdx.x;
     // the factorisation of this stage is complete: the MASK9 change flag
@@ -2083,32 +2101,6 @@ __global__ void __launch_bounds__(256, KPT > 0 ? 3 : 1) k_linesolve_x(Grid g, Fi
     const int s = ch * m;
     const int e = (ch == P - 1) ? L - 1 : s + m - 1;
     const int n = 2 * P;
-    constexpr int KR = KPT > 0 ? KPT : 1;
-    float rP[KR], rQ[KR], rAH[KR], rAL[KR], rCH[KR], rCL[KR];
-    float lo_r = 0.0f, di_r = 0.0f, up_r = 0.0f, cs_r = 0.0f, ae_r = 0.0f;
-    if constexpr (KPT > 0) {
-#pragma unroll
-        for (int q = 0; q < KPT; q++) {
-            const int k = threadIdx.x + q * 256;
-            if (k < L) {
-                rP[q] = Pp[k];
-                rQ[q] = Qq[k];
-                rAH[q] = AH[k];
-                rAL[q] = AL[k];
-                rCH[q] = CH[k];
-                rCL[q] = CL[k];
-            }
-        }
-        if ((int)threadIdx.x < n) {
-            lo_r = fl.lo[threadIdx.x];
-            di_r = fl.di[threadIdx.x];
-            up_r = fl.up[threadIdx.x];
-        }
-        if (ch < P) {
-            cs_r = fl.cs[ch];
-            ae_r = fl.ae[ch];
-        }
-    }
     for (int k = threadIdx.x; k < L; k += blockDim.x) {
         const int q = lsx_pad(k);
         const float dv = (float)rhs[k] * IT[k];
@@ -2136,24 +2128,16 @@ __global__ void __launch_bounds__(256, KPT > 0 ? 3 : 1) k_linesolve_x(Grid g, Fi
                     yn = y[q] - CP[q] * yn;
                     y[q] = yn;
                 }
-                rs = rs - (KPT > 0 ? cs_r : fl.cs[ch]) * y[lsx_pad(s + 1)];
-                re = re - (KPT > 0 ? ae_r : fl.ae[ch]) * y[lsx_pad(e - 1)];
+                rs = rs - fl.cs[ch] * y[lsx_pad(s + 1)];
+                re = re - fl.ae[ch] * y[lsx_pad(e - 1)];
             }
             rr[2 * ch] = rs;
             rr[2 * ch + 1] = re;
         }
-        if constexpr (KPT > 0) {
-            if ((int)threadIdx.x < n) {
-                pb[threadIdx.x] = lo_r;
-                pb[n + threadIdx.x] = di_r;
-                pb[2 * n + threadIdx.x] = up_r;
-            }
-        } else {
-            for (int k = threadIdx.x; k < n; k += blockDim.x) {
-                pb[k] = fl.lo[k];
-                pb[n + k] = fl.di[k];
-                pb[2 * n + k] = fl.up[k];
-            }
+        for (int k = threadIdx.x; k < n; k += blockDim.x) {
+            pb[k] = fl.lo[k];
+            pb[n + k] = fl.di[k];
+            pb[2 * n + k] = fl.up[k];
         }
         __syncthreads();
         pcr_solve(pb, pb + n, pb + 2 * n, rr, pb + 3 * n, pb + 4 * n, pb + 5 * n, pb + 6 * n, n);
@@ -2164,15 +2148,7 @@ __global__ void __launch_bounds__(256, KPT > 0 ? 3 : 1) k_linesolve_x(Grid g, Fi
             if (pass == 0) x0[k] = x;
             else f.U[row + k] = (T)(x0[k] + x);
         };
-        if constexpr (KPT > 0) {
-#pragma unroll
-            for (int q = 0; q < KPT; q++) {
-                const int k = threadIdx.x + q * 256;
-                if (k < L) recon(k, rP[q], rQ[q]);
-            }
-        } else {
-            for (int k = threadIdx.x; k < L; k += blockDim.x) recon(k, Pp[k], Qq[k]);
-        }
+        for (int k = threadIdx.x; k < L; k += blockDim.x) recon(k, Pp[k], Qq[k]);
         __syncthreads();
         if (pass == 0) {
             auto resid = [&](int k, float ah, float al, float chv, float cl) {
@@ -2180,16 +2156,405 @@ __global__ void __launch_bounds__(256, KPT > 0 ? 3 : 1) k_linesolve_x(Grid g, Fi
                 const int q = lsx_pad(k);
                 d[q] = residual(dn[q], x0[k], xm, xp, ah, al, chv, cl);
             };
-            if constexpr (KPT > 0) {
+            for (int k = threadIdx.x; k < L; k += blockDim.x) resid(k, AH[k], AL[k], CH[k], CL[k]);
+            __syncthreads();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The mixed u/v recovery of one direction in one kernel, for lines of 32 to
+// 4096 rows (chunks of LSF_M rows).  A thread owns one chunk of one line and
+// keeps its rows in registers from the right-hand side to the result: sweeps,
+// reduced system, reconstruction, compensated residual, and the same again on
+// the residual.  HBM sees the right-hand side, the constant factors and the
+// result once each: 56 B per cell.
+//   x lines: a block takes a few whole lines.  Their factors lie chunk-
+//   interleaved (fac_at), so the 32 chunks of a warp load neighbouring words;
+//   the right-hand side and the result cross shared memory between the
+//   coalesced order and the chunks' (lsx_pad keeps that free of conflicts).
+//   y lines: a block takes up to 8 neighbouring columns, a whole 32-byte
+//   sector of each row, times the chunks of a line; lines of more than 32
+//   chunks (512 rows) are shared by a cluster of 2, 4 or 8 blocks.  The
+//   reduced rows of a column go to one block of the cluster through
+//   distributed shared memory (each block owns 8 / nc of the columns), are
+//   solved there and come back.
+// The reduced system (2P rows of a line, at most 512 rows per block: a chunk's
+// pair per thread) is solved by parallel cyclic reduction with the multipliers
+// that the factorisation left (pcr_factor), staged in shared memory at the
+// start.
+// REM: the line's length is no multiple of LSF_M.  Its last chunk has up to
+// 31 rows, whose rows past the 16th belong to a thread of their own; the two
+// hand the sweeps' running value to each other through shared memory.  All
+// threads then sweep 16 rows without a test: the constants of a chunk's first
+// and last row (fac_a_body) and the zeros beside them pass those rows by, and
+// a remainder thread repeats its last row's.
+// What bounds it is memory latency (16 warps to an SM at 128 registers), so
+// the loads of a phase are issued together (ld_now).  The operations and
+// their order are those of k_sol_a .. k_resid, which the other lines take, so
+// that the results are the same bit for bit.
+// Measured with the two early-exit factor launches (us, before -> after; x
+// took one 256-thread block per line, y seven kernels moving 95 B per cell):
+// 2048 x 2048 x 119 -> 75, y 138 -> 94; 4096 x 4096 x 1160 -> 247, y 424 ->
+// 330; 250 x 500 x 28 -> 20, y 72 -> 25 (the 20-row last chunks walked global
+// memory); 1024 x 1024 x 41 -> 23, y 51 -> 29.
+// ---------------------------------------------------------------------------
+constexpr int LSF_T = 256;     // most threads of a block
+constexpr int LSF_COLS = 8;    // columns of a y block
+struct LsfShape {
+    int nline;  // lines of a block
+    int nch;    // threads of a line in a block (its chunks, and the remainder rows' thread)
+    int slots;  // lines whose reduced rows a block solves
+    int nc;     // blocks of a cluster
+    int nblk;   // blocks of the grid
+    int nt;     // threads of a block: its lines' chunks, in whole warps
+};
+
+// the address of a shared-memory word of this block in block `rank` of the cluster
+__device__ __forceinline__ float *cluster_peer(float *p, int rank) {
+    uint64_t q;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+    return reinterpret_cast<float *>(q);
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// a read-only load that stays where it is written, ahead of later barriers
+__device__ __forceinline__ float ld_now(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+// 16 bytes to shared memory without a register, and the wait for all of them
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// shared memory of a block, in floats: the reduction's multipliers, the
+// reduced right-hand sides twice, the solved pairs of the block's chunks with
+// a neighbour on either side, the remainder rows' exchange and, for x, the
+// staged lines
+static size_t lsf_smem_floats(int dir, const LinePart &lp, const LsfShape &S) {
+    return (size_t)S.slots * pcr_words(lp) + (size_t)2 * S.slots * 2 * lp.P + (size_t)S.nline * (2 * S.nch + 4) +
+           (size_t)4 * S.nline + (dir == 0 ? (size_t)S.nline * (lsx_pad(lp.L) + 1) : 0);
+}
+
+template <typename T, int DIR, bool PER, bool REM>
+__global__ void __launch_bounds__(LSF_T, 2) k_linesolve(Grid g, Fields<T> f, LinePart lp, LsfShape S, int clear_dirty) {
+    extern __shared__ __align__(16) float shf[];
+    constexpr int M = LSF_M;
+    const int P = lp.P, L = lp.L, n = 2 * P, tid = threadIdx.x, NT = blockDim.x;
+    const int PT = P + (REM ? 1 : 0);  // threads of a line
+    const bool clus = DIR == 1 && S.nc > 1;
+    if (clus) cluster_arrive();  // every block of the cluster has started before the first remote store
+    const int rank = clus ? (int)(blockIdx.x % (unsigned)S.nc) : 0;
+    const int grp = clus ? (int)(blockIdx.x / (unsigned)S.nc) : (int)blockIdx.x;
+    // the factorisation of this stage is complete: the MASK9 change flag
+    // can be reset for UPDATE_MASK to set again
+    if (clear_dirty && blockIdx.x == 0 && tid == 0) *f.m9_dirty = 0;
+    const int nred = S.slots * n, steps = pcr_steps(n), n4 = (n + 3) & ~3, pw = pcr_words(lp);
+    float *MUL = shf;                  // [slots][pw]
+    float *R0 = MUL + S.slots * pw, *R1 = R0 + nred;
+    const int rw = 2 * S.nch + 4;
+    float *res = R1 + nred;            // per line: -, left neighbour, the chunks' pairs, right neighbour, -
+    float *ex = res + S.nline * rw;    // [4][nline]
+    float *stage = ex + 4 * S.nline;   // x: the block's lines
+    const int SW = lsx_pad(L) + 1;
+
+    // this thread's line and chunk (y: consecutive threads on consecutive columns)
+    const int ln = DIR == 0 ? tid / PT : tid % S.nline;
+    const int cl = DIR == 0 ? tid - ln * PT : tid / S.nline;
+    const int ct = rank * S.nch + cl;       // chunk, or P: the remainder rows of chunk P-1
+    // x: a block's lines from grp*nline; y: its columns from nline*grp of the
+    // plane (sector-aligned), of which the interior ones are lines
+    const int l0 = grp * S.nline - (DIR == 0 ? 0 : g.ib), l = l0 + ln;
+    const bool on = ln < S.nline && cl < S.nch && ct < PT && l >= 0 && l < lp.nlines;
+    const bool rem = REM && on && ct == P, last = REM && on && ct == P - 1;
+    const int ch = rem ? P - 1 : ct;
+    const int s = ct * M, nr = rem ? L - s : M;   // this thread's first row and its rows
+    constexpr int K0 = REM ? 0 : 1, K1 = REM ? M : M - 1;  // rows that the sweeps walk
+    const int fst = DIR == 0 ? (rem ? 1 : P) : g.pitch;
+    // offset of row k's factors from the first row's (of the last row for the
+    // rows that a remainder does not have: loaded, never used)
+#define LSF_OFF(k) ((REM ? min((k), nr - 1) : (k)) * fst)
+    const size_t fq = on ? fac_at<DIR>(g, lp, l, s) : 0;
+
+    // the multipliers, in flight until the first reduction
+    for (int q = tid; q < S.slots * (pw / 4); q += NT) {
+        const int slot = q / (pw / 4);
+        const int rl = DIR == 0 ? l0 + slot : l0 + slot * S.nc + rank;
+        if (rl >= 0 && rl < lp.nlines) copy16_async(MUL + 4 * q, pcr_line<T, DIR>(f, lp, rl) + 4 * (q - slot * (pw / 4)));
+    }
+    // the right-hand side (x: staged below), normalised, and the sweeps' constants
+    float d[M], y[M], x0[M], av[M], lv[M], cv[M];
+    if (on) {
+        const float *IT = f.fac_it[DIR] + fq, *FA = f.fac_A[DIR] + fq, *LR = f.fac_lr[DIR] + fq, *CP = f.fac_cp[DIR] + fq;
 #pragma unroll
-                for (int q = 0; q < KPT; q++) {
-                    const int k = threadIdx.x + q * 256;
-                    if (k < L) resid(k, rAH[q], rAL[q], rCH[q], rCL[q]);
-                }
-            } else {
-                for (int k = threadIdx.x; k < L; k += blockDim.x) resid(k, AH[k], AL[k], CH[k], CL[k]);
+        for (int k = 0; k < M; k++) {
+            if (DIR == 1) d[k] = ld_now((const float *)f.rhs_y + fq + LSF_OFF(k));
+            x0[k] = ld_now(IT + LSF_OFF(k));
+        }
+#pragma unroll
+        for (int k = K0; k < K1; k++) {
+            av[k] = ld_now(FA + LSF_OFF(k));
+            lv[k] = ld_now(LR + LSF_OFF(k));
+            cv[k] = ld_now(CP + LSF_OFF(k));
+        }
+    }
+    float cs = 0.0f, ae = 0.0f, sc0 = 1.0f, sc1 = 1.0f;
+    if (on) {
+        const FacLine fl = fac_line(f.fac_red[DIR], lp, l);
+        cs = ld_now(fl.cs + ch);
+        ae = ld_now(fl.ae + ch);
+        if (PER) {
+            if (ch == 0) sc0 = 1.0f / (1.0f + ld_now(fl.tail + 0));      // row 0: d / (1 + c_end)
+            if (ch == P - 1) sc1 = 1.0f / (1.0f + ld_now(fl.tail + 1));  // row L-1: d / (1 + a_beg)
+        }
+    }
+    if (DIR == 0) {
+        const int nl = min(S.nline, lp.nlines - l0);
+        for (int q = 0; q < nl; q++) {
+            const T *src = f.rhs_x + (size_t)(g.jb + l0 + q) * g.pitch + g.ib;
+#pragma unroll 4
+            for (int k = tid; k < L; k += NT) stage[q * SW + lsx_pad(k)] = (float)ro(src + k);
+        }
+        __syncthreads();
+    }
+    if (on) {
+#pragma unroll
+        for (int k = 0; k < M; k++)
+            d[k] = __fmul_rn(DIR == 0 ? stage[ln * SW + lsx_pad(s + (REM ? min(k, nr - 1) : k))] : d[k], x0[k]);
+    }
+    // the reduced rows this thread solves: the pair of chunk rc of line rl (slot rsl)
+    const int rsl = tid / P, rc = tid - rsl * P;
+    const int rl = DIR == 0 ? l0 + rsl : l0 + rsl * S.nc + rank;
+    const bool ron = rsl < S.slots && rl >= 0 && rl < lp.nlines;
+
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++) {
+        // the chunk's forward and backward sweep
+        auto forward = [&](float yp) {
+#pragma unroll
+            for (int k = K0; k < K1; k++) {
+                yp = __fmaf_rn(d[k], av[k], -__fmul_rn(lv[k], yp));  // rounded as in k_sol_a
+                y[k] = yp;
+            }
+            return yp;
+        };
+        auto backward = [&](float yn) {
+#pragma unroll
+            for (int k = K1 - 1; k >= K0; k--) {
+                yn = __fmaf_rn(-cv[k], yn, y[k]);
+                y[k] = yn;
+            }
+            return yn;
+        };
+        float rs = 0.0f, re = 0.0f, yn = 0.0f;
+        if (on && !rem) {
+            const float yp = forward(0.0f);
+            if (last) ex[ln] = yp;
+        }
+        if (REM) {
+            // the last chunk: forward through both of its threads, then back
+            __syncthreads();
+            if (rem) {
+                const float yp = ex[ln];
+                forward(yp);
+                ex[S.nline + ln] = backward(0.0f);
+                float de = d[0], ye = yp;  // d of the chunk's last row, y of the one before
+#pragma unroll
+                for (int k = 1; k < M; k++)
+                    if (k == nr - 1) {
+                        de = d[k];
+                        ye = y[k - 1];
+                    }
+                ex[2 * S.nline + ln] = ye;
+                ex[3 * S.nline + ln] = __fmul_rn(de, sc1);
             }
             __syncthreads();
+            if (last) yn = ex[S.nline + ln];
+        }
+        if (on && !rem) {
+            backward(yn);
+            rs = __fmul_rn(d[0], sc0) - cs * y[1];
+            re = REM && last ? ex[3 * S.nline + ln] - ae * ex[2 * S.nline + ln]
+                             : __fmul_rn(d[M - 1], sc1) - ae * y[M - 2];
+        }
+        if (clus && pass == 0) cluster_wait();
+        if (on && !rem) {
+            // the reduced right-hand sides, to the block that solves this line
+            float *dst = R0 + (DIR == 0 ? ln : ln / S.nc) * n + 2 * ch;
+            if (clus) dst = cluster_peer(dst, ln % S.nc);
+            dst[0] = rs;
+            dst[1] = re;
+        }
+        if (on) {
+            // the reconstruction's constants arrive while the reduced system is solved
+            const float *PP = f.fac_p[DIR] + fq, *QQ = f.fac_q[DIR] + fq;
+#pragma unroll
+            for (int k = K0; k < K1; k++) {
+                av[k] = ld_now(PP + LSF_OFF(k));
+                lv[k] = ld_now(QQ + LSF_OFF(k));
+            }
+        }
+        if (pass == 0) copies_wait();
+        if (clus) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+        // parallel cyclic reduction
+        float *r = R0 + 2 * tid, *r2 = R1 + 2 * tid;
+        const float *m = MUL + rsl * pw + 2 * rc;
+        float2 rr = make_float2(0.0f, 0.0f);
+        if (ron) {
+            rr = *(const float2 *)r;
+            // neighbours one row away: a pair's rows are each other's
+            const float2 a = *(const float2 *)m, b = *(const float2 *)(m + n4);
+            float x = rr.x, y_ = rr.y;
+            if (rc > 0) x += a.x * r[-1];
+            x += b.x * rr.y;
+            y_ += a.y * rr.x;
+            if (rc < P - 1) y_ += b.y * r[2];
+            rr = make_float2(x, y_);
+            *(float2 *)r2 = rr;
+        }
+        __syncthreads();
+        for (int st = 1; st < steps; st++) {
+            float *t = r;
+            r = r2;
+            r2 = t;
+            m += 2 * n4;
+            if (ron) {
+                // whole pairs: 2^st rows are 2^(st-1) chunks
+                const int dist = 1 << st, dc = dist >> 1;
+                const float2 a = *(const float2 *)m, b = *(const float2 *)(m + n4);
+                if (rc >= dc) {
+                    const float2 v = *(const float2 *)(r - dist);
+                    rr.x += a.x * v.x;
+                    rr.y += a.y * v.y;
+                }
+                if (rc + dc < P) {
+                    const float2 v = *(const float2 *)(r + dist);
+                    rr.x += b.x * v.x;
+                    rr.y += b.y * v.y;
+                }
+                *(float2 *)r2 = rr;
+            }
+            __syncthreads();
+        }
+        if (ron) {
+            const float2 di = *(const float2 *)(m + 2 * n4);
+            rr = make_float2(rr.x / di.x, rr.y / di.y);
+        }
+        if (PER) {  // Sherman-Morrison with both ends of the line's solution
+            if (ron && rc == 0) r[0] = rr.x;
+            if (ron && rc == P - 1) r[1] = rr.y;
+            __syncthreads();
+            if (ron) {
+                const FacLine fl = fac_line(f.fac_red[DIR], lp, rl);
+                const float *z = r - 2 * rc;
+                const float beta = (ro(fl.tail + 0) * z[0] - ro(fl.tail + 1) * z[n - 1]) / ro(fl.tail + 2);
+                rr.x = rr.x + beta * ro(fl.x2 + 2 * rc);
+                rr.y = rr.y + beta * ro(fl.x2 + 2 * rc + 1);
+            }
+        }
+        if (ron) {
+            // to the chunk's own pair and, at the end of a block's chunks (or
+            // of a periodic line), to the neighbour's outer place
+            const int q = clus ? rc / S.nch : 0, cq = rc - q * S.nch;
+            float *own = res + (DIR == 0 ? rsl : rsl * S.nc + rank) * rw;
+            auto at = [&](int blk, int pos) { return clus ? cluster_peer(own + pos, blk) : own + pos; };
+            *(float2 *)at(q, 2 + 2 * cq) = rr;
+            if (clus && rc < P - 1 && cq == S.nch - 1) *at(q + 1, 1) = rr.y;
+            if (clus && rc > 0 && cq == 0) *at(q - 1, 2 + 2 * S.nch) = rr.x;
+            if (PER && rc == P - 1) *at(0, 1) = rr.y;
+            if (PER && rc == 0) {
+                const int ql = clus ? (P - 1) / S.nch : 0;
+                *at(ql, 2 + 2 * (P - ql * S.nch)) = rr.x;
+            }
+        }
+        if (clus) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
+        // reconstruction; after the first pass the residual in d's place
+        const float *rv = res + ln * rw + 2 + 2 * (ch - rank * S.nch);
+        const float xs = on ? rv[0] : 0.0f, xe = on ? rv[1] : 0.0f;
+        float xl = on && (PER || ch > 0) ? rv[-1] : 0.0f, xr = on && (PER || ch < P - 1) ? rv[2] : 0.0f;
+        if (on) {
+#pragma unroll
+            for (int k = K0; k < K1; k++) y[k] = y[k] - av[k] * xs - lv[k] * xe;
+            if (!rem) y[0] = xs;
+            if (!REM || !(rem || last)) y[M - 1] = xe;
+            if (REM) {
+#pragma unroll
+                for (int k = 0; k < M; k++)
+                    if (rem && k >= nr - 1) y[k] = xe;
+            }
+        }
+        if (REM && pass == 0) {
+            // the last chunk's two threads are each other's neighbours
+            if (last) ex[2 * S.nline + ln] = y[M - 1];
+            if (rem) ex[3 * S.nline + ln] = y[0];
+            __syncthreads();
+            if (rem) xl = ex[2 * S.nline + ln];
+            if (last) xr = ex[3 * S.nline + ln];
+        }
+        if (on) {
+            if (pass == 0) {
+                const float *AH = f.fac_ah[DIR] + fq, *AL = f.fac_al[DIR] + fq, *CH = f.fac_ch[DIR] + fq,
+                            *CL = f.fac_cl[DIR] + fq;
+                // rows whose coefficients are loaded together
+                constexpr int HB = 8;
+#pragma unroll
+                for (int k0 = 0; k0 < M; k0 += HB) {
+                    float ah[HB], al[HB], ch_[HB], cl_[HB];
+#pragma unroll
+                    for (int q = 0; q < HB; q++) {
+                        ah[q] = ld_now(AH + LSF_OFF(k0 + q));
+                        al[q] = ld_now(AL + LSF_OFF(k0 + q));
+                        ch_[q] = ld_now(CH + LSF_OFF(k0 + q));
+                        cl_[q] = ld_now(CL + LSF_OFF(k0 + q));
+                    }
+#pragma unroll
+                    for (int q = 0; q < HB; q++) {
+                        const int k = k0 + q;
+                        const float xm = k > 0 ? y[k > 0 ? k - 1 : 0] : xl;
+                        const float xp = k < M - 1 && (!REM || k < nr - 1) ? y[k < M - 1 ? k + 1 : k] : xr;
+                        d[k] = residual(d[k], y[k], xm, xp, ah[q], al[q], ch_[q], cl_[q]);
+                        x0[k] = y[k];
+                    }
+                }
+                // the sweeps' constants again (L2)
+                const float *FA = f.fac_A[DIR] + fq, *LR = f.fac_lr[DIR] + fq, *CP = f.fac_cp[DIR] + fq;
+#pragma unroll
+                for (int k = K0; k < K1; k++) {
+                    av[k] = ld_now(FA + LSF_OFF(k));
+                    lv[k] = ld_now(LR + LSF_OFF(k));
+                    cv[k] = ld_now(CP + LSF_OFF(k));
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < M; k++)
+                    if (!REM || k < nr) {
+                        const float x = x0[k] + y[k];
+                        if (DIR == 0) stage[ln * SW + lsx_pad(s + k)] = x;
+                        else f.V[fq + (size_t)k * fst] = (T)x;
+                    }
+            }
+        }
+    }
+#undef LSF_OFF
+    if (DIR == 0) {
+        __syncthreads();
+        const int nl = min(S.nline, lp.nlines - l0);
+        for (int q = 0; q < nl; q++) {
+            T *dst = f.U + (size_t)(g.jb + l0 + q) * g.pitch + g.ib;
+            for (int k = tid; k < L; k += NT) dst[k] = (T)stage[q * SW + lsx_pad(k)];
         }
     }
 }
@@ -3401,6 +3766,59 @@ template <typename T> void launch_sources_debug(fw_ctx *c) {
     note(c);
 }
 
+// blocks of the factorisation's launch that take the reduction's multipliers
+constexpr int PCR_BLOCKS = 4 * 152;
+// the blocks of k_linesolve: x lines as many to a block as its threads hold,
+// y columns 8 to a block, but fewer while the grid would not reach every SM
+static LsfShape lsf_shape(int dir, const Grid &g, const LinePart &lp) {
+    constexpr int SMS = 152;
+    LsfShape S;
+    const int PT = lp.P + (lp.L % LSF_M ? 1 : 0);  // threads of a line
+    if (dir == 0) {
+        S.nc = 1;
+        S.nline = std::max(1, std::min(LSF_T / PT, (lp.nlines + SMS - 1) / SMS));
+        S.nch = PT;
+        S.slots = S.nline;
+        S.nblk = (lp.nlines + S.nline - 1) / S.nline;
+    } else {
+        S.nc = PT > 128 ? 8 : PT > 64 ? 4 : PT > 32 ? 2 : 1;
+        S.nline = LSF_COLS;
+        if (S.nc == 1)
+            while (S.nline > 2 && (g.ie + S.nline) / S.nline < SMS) S.nline /= 2;
+        S.nch = (PT + S.nc - 1) / S.nc;
+        // the last chunk and its remainder rows in the same block (P is then
+        // no multiple of nch; nch stays below 32 where it grows)
+        if (PT > lp.P && lp.P % S.nch == 0) S.nch++;
+        S.slots = S.nline / S.nc;
+        S.nblk = (g.ie + S.nline) / S.nline * S.nc;  // columns 0 .. ie
+    }
+    // (every reduced pair has a thread too: slots x P <= nline x nch); at least
+    // 128 for the staging loops
+    S.nt = std::max(128, (S.nline * S.nch + 31) / 32 * 32);
+    return S;
+}
+
+template <typename T, int DIR, bool PER>
+static void launch_linesolve(fw_ctx *c, const LinePart &lp, bool clear_dirty) {
+    const LsfShape S = lsf_shape(DIR, c->g, lp);
+    auto kern = lp.L % LSF_M ? k_linesolve<T, DIR, PER, true> : k_linesolve<T, DIR, PER, false>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)S.nblk);
+    cfg.blockDim = dim3((unsigned)S.nt);
+    cfg.dynamicSmemBytes = lsf_smem_floats(DIR, lp, S) * sizeof(float);
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)S.nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = S.nc > 1 ? 1 : 0;
+    if (cfg.dynamicSmemBytes > 48 * 1024)
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+    cudaLaunchKernelEx(&cfg, kern, c->g, c->F<T>(), lp, S, clear_dirty ? 1 : 0);
+    note(c);
+}
+
 template <typename T, int DIR, bool PER>
 static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clear_dirty = false) {
     const Grid &g = c->g;
@@ -3408,15 +3826,20 @@ static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clea
     if constexpr (sizeof(T) == sizeof(float)) if (c->factored) {
         if (fac) {
             k_fac_a<T, DIR, PER><<<(nt + 127) / 128, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_fac_b<T, DIR, PER><<<(lp.nlines + 127) / 128, 128, 0, c->stream>>>(g, c->F<T>(), lp);
+            const int nb = (lp.nlines + 127) / 128;
+            const int nm = lsf_line(lp) ? std::min(lp.nlines, PCR_BLOCKS) : 0;
+            k_fac_b<T, DIR, PER><<<nb + nm, 128, nm ? 12 * lp.P * sizeof(float) : 0, c->stream>>>(g, c->F<T>(), lp, nb);
             note(c, 2);
         }
+        if (lsf_line(lp)) {
+            launch_linesolve<T, DIR, PER>(c, lp, clear_dirty);
+            return clear_dirty;
+        }
+        // lines of more than 4096 rows
         const size_t smem = lsx_smem_floats(lp.L, lp.P) * sizeof(float);
         if (DIR == 0 && !PER && lp.P <= 256 && smem <= 200 * 1024) {
-            // lines of up to 2048 cells keep their per-cell coefficients in registers
-            auto kern = lp.L <= 2048 ? k_linesolve_x<T, 8> : k_linesolve_x<T, 0>;
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<lp.nlines, 256, smem, c->stream>>>(g, c->F<T>(), lp, clear_dirty ? 1 : 0);
+            if (smem > 48 * 1024) cudaFuncSetAttribute(k_linesolve_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            k_linesolve_x<T><<<lp.nlines, 256, smem, c->stream>>>(g, c->F<T>(), lp, clear_dirty ? 1 : 0);
             note(c);
             return clear_dirty;
         }
@@ -3424,24 +3847,13 @@ static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clea
         const int nb = std::min(512, ((2 * lp.P + 31) / 32) * 32);
         const size_t sb = (size_t)16 * lp.P * sizeof(float);
         const unsigned ga = (unsigned)((nt + 127) / 128);
-        // chunks of 16 rows (lines of 512 cells and more) walk in registers
-        if (lp.m == 16) {
-            k_sol_a<T, DIR, PER, 0, 16><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_b<T, DIR, PER, 0><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_c<T, DIR, 0, 16><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_resid<T, DIR, PER><<<gi, B2D, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_a<T, DIR, PER, 1, 16><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_b<T, DIR, PER, 1><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_c<T, DIR, 1, 16><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-        } else {
-            k_sol_a<T, DIR, PER, 0, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_b<T, DIR, PER, 0><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_c<T, DIR, 0, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_resid<T, DIR, PER><<<gi, B2D, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_a<T, DIR, PER, 1, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_b<T, DIR, PER, 1><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
-            k_sol_c<T, DIR, 1, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
-        }
+        k_sol_a<T, DIR, PER, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
+        k_sol_b<T, DIR, PER, 0><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
+        k_sol_c<T, DIR, 0><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
+        k_resid<T, DIR, PER><<<gi, B2D, 0, c->stream>>>(g, c->F<T>(), lp);
+        k_sol_a<T, DIR, PER, 1><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
+        k_sol_b<T, DIR, PER, 1><<<lp.nlines, nb, sb, c->stream>>>(g, c->F<T>(), lp);
+        k_sol_c<T, DIR, 1><<<ga, 128, 0, c->stream>>>(g, c->F<T>(), lp);
         note(c, 7);
         return false;
     }
@@ -3486,12 +3898,14 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
             const int nbx = (c->px.nlines * c->px.P + 127) / 128;
             const int nby = (c->py.nlines * c->py.P + 127) / 128;
             const int lbx = (c->px.nlines + 127) / 128, lby = (c->py.nlines + 127) / 128;
+            const int nm = std::min((lsf_line(c->px) ? c->px.nlines : 0) + (lsf_line(c->py) ? c->py.nlines : 0), PCR_BLOCKS);
+            const size_t sp = nm ? 12 * std::max(lsf_line(c->px) ? c->px.P : 0, lsf_line(c->py) ? c->py.P : 0) * sizeof(float) : 0;
             if (g.periodic) {
                 k_fac_a_xy<T, true><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
-                k_fac_b_xy<T, true><<<lbx + lby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx);
+                k_fac_b_xy<T, true><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
             } else {
                 k_fac_a_xy<T, false><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
-                k_fac_b_xy<T, false><<<lbx + lby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx);
+                k_fac_b_xy<T, false><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
             }
             note(c, 2);
             const bool cleared = launch_tri<T, 0, false>(c, c->px, false, true);
