@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "fw_internal.h"
 #include "fw_tc.cuh"
@@ -482,80 +483,159 @@ template <typename T, int DIR, int FY_ = flux_fy_default<T, DIR>()> struct FluxT
     static constexpr int NP = DIR == 0 ? NPOS : NPOS + 1;  // odd row length for y
 };
 
-template <typename T, int DIR, int FY_ = flux_fy_default<T, DIR>()>
-__global__ void __launch_bounds__(256) k_flux(Grid g, Fields<T> f) {
-    using TL = FluxTile<T, DIR, FY_>;
-    static_assert(TL::FY % TL::BY == 0, "whole faces per thread");
-    constexpr int BX = TL::BX, BY = TL::BY, NTL = TL::NTL, NPOS = TL::NPOS, NP = TL::NP;
-    __shared__ T din[7][NTL][NP];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i0 = g.ib + blockIdx.x * TL::FX, j0 = g.jb + blockIdx.y * TL::FY;
-    const int lo = DIR == 0 ? g.ib : g.jb, hi = DIR == 0 ? g.ie : g.je;
-    const int base = (DIR == 0 ? i0 : j0) - 1;
-    const T *src[7] = {f.U, f.V, f.HU, f.HV, f.Eta, f.U4, f.V4};
-    const int nvar = g.dispersion ? 7 : 5;
-    // 32-bit offsets: the arena planes hold fewer than 2^31 elements
-    const int stride = DIR == 0 ? 1 : g.pitch;
-    // the NTL x NPOS Din positions of the tile, spread over all threads
-    // (consecutive threads on consecutive x for coalesced loads)
-    const int tid = tx + ty * BX;
-    for (int it = tid; it < NTL * NPOS; it += BX * BY) {
-        const int k = DIR == 0 ? it % NPOS : it / NTL;
-        const int ln = DIR == 0 ? it / NPOS : it % NTL;
-        const int p = base + k;
-        const int ci = DIR == 0 ? p : i0 + ln;
-        const int cj = DIR == 0 ? j0 + ln : p;
-        const bool lok = DIR == 0 ? (cj <= g.je) : (ci <= g.ie);
-        if (lok && p >= lo - 1 && p <= hi + 2) {
-            const int o0 = ci + cj * g.pitch - 2 * stride;
-            int m[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) m[q] = ro(f.MASK + (o0 + q * stride));
-#pragma unroll
-            for (int vv = 0; vv < 7; vv++) {
-                if (vv < nvar) {
-                    T v[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) v[q] = ro(src[vv] + (o0 + q * stride));
-                    din[vv][ln][k] = ho_din(v, m);
-                }
-            }
-        }
+// ---------------------------------------------------------------------------
+// FP64 arithmetic beside the FP64 pipe.  GB300 issues double operations at
+// 1/64 of the float rate and integer ones beside them, so comparisons,
+// absolute values and doublings of doubles are done on their bits, and
+// quotients by a divisor whose reciprocal is at hand take one product and two
+// fused operations.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
+__device__ __forceinline__ double dfrom(unsigned long long b) { return __longlong_as_double((long long)b); }
+constexpr unsigned long long D_SIGN = 1ull << 63, D_INF = 0x7ffull << 52;
+__device__ __forceinline__ unsigned long long dmag(double x) { return dbits(x) & ~D_SIGN; }
+
+// a / b rounded to nearest, with y = RN(1/b): q = RN(a y), r = a - b q
+// (exact), RN(q + r y) (Markstein, IBM J. Res. Dev. 34 (1990): correctly
+// rounded when y is, and nothing under- or overflows).  b > 0 lies in
+// [2^-300, 2^300] (the callers' spacings, steps and guarded slopes); an a
+// outside [2^-500, 2^500], zero apart, takes the division.
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+    const unsigned long long m = dmag(a);
+    if (m - ((1023ull - 500) << 52) >= (1000ull << 52)) {
+        if (m == 0) return a;
+        return a / b;
     }
-    __syncthreads();
-    const T g1 = GC(gamma1), g3 = GC(gamma3);
-    for (int r = 0; r < TL::FPT; r++) {
-    const int i = i0 + tx;
-    const int j = j0 + ty + r * BY;
-    if (DIR == 0) {
-        if (i > g.ie + 1 || j > g.je) continue;
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// ---------------------------------------------------------------------------
+// The reconstruction along a line, with every quantity computed once: Din at
+// a cell from its three slopes, and from two neighbouring Din the left state
+// of the face after them and the right state of the face between them.
+// ---------------------------------------------------------------------------
+// Din from the slopes T1 = v(p-1)-v(p-2), T2 = v(p)-v(p-1), T3 = v(p+1)-v(p)
+// (ho_din): the same value as lim3's three slopes.  For slopes of one sign
+// lim3(a, b, c) = s min(|a|, 2|b|, 2|c|) = s min(|a|, 2m) with m the least of
+// the three sizes, else 0; so each limited slope is its own clamped to
+// [2 min(0, max), 2 max(0, min)].
+__device__ __forceinline__ float line_din(float T1, float T2, float T3, bool wet) {
+    const float lo = 2.0f * fminf(0.0f, fmaxf(fmaxf(T1, T2), T3)), hi = 2.0f * fmaxf(0.0f, fminf(fminf(T1, T2), T3));
+    const float D1 = fminf(fmaxf(T1, lo), hi), D2 = fminf(fmaxf(T2, lo), hi), D3 = fminf(fmaxf(T3, lo), hi);
+    const float d = __fmaf_rn(-(1.0f / 6.0f), __fadd_rn(__fmaf_rn(-2.0f, D2, D3), D1), T2);
+    return wet ? d : T2;
+}
+// FP64: the limiting on the bits.  A zero T2 keeps lim3's expressions, whose
+// zeros' signs decide the sign of Din there (vl_guard reads it); so do
+// non-finite slopes.
+__device__ __forceinline__ double line_din(double T1, double T2, double T3, bool wet) {
+    if (!wet) return T2;
+    const unsigned long long m1 = dmag(T1), m2 = dmag(T2), m3 = dmag(T3);
+    const unsigned long long mx = m1 > m2 ? (m1 > m3 ? m1 : m3) : (m2 > m3 ? m2 : m3);
+    if (m2 == 0 || mx >= D_INF) {
+        const double P1 = lim3(T1, T2, T3), P2 = lim3(T2, T3, T1), P3 = lim3(T3, T1, T2);
+        return T2 - 1.0 / 6.0 * (P3 - 2.0 * P2 + P1);
+    }
+    const unsigned long long mn = m1 < m2 ? (m1 < m3 ? m1 : m3) : (m2 < m3 ? m2 : m3);
+    // slopes of both signs, or a zero one: the limited slopes are zero
+    if ((((dbits(T1) ^ dbits(T2)) | (dbits(T1) ^ dbits(T3))) & D_SIGN) || mn == 0) return T2;
+    const unsigned long long two = (mn >> 52) ? mn + (1ull << 52) : mn << 1;  // 2 mn
+    const unsigned long long sg = dbits(T2) & D_SIGN;
+    const double D1 = dfrom(sg | (m1 < two ? m1 : two)), D2 = dfrom(sg | (m2 < two ? m2 : two)),
+                 D3 = dfrom(sg | (m3 < two ? m3 : two));
+    // D3 - 2 D2: the product is exact, so one fused operation rounds the same
+    return __dsub_rn(T2, __dmul_rn(1.0 / 6.0, __dadd_rn(__fma_rn(-2.0, D2, D3), D1)));
+}
+
+// what the two pairs that a cell's Din belongs to share: in FP64 the guarded
+// slope (vl_guard) and its reciprocal
+template <typename T> struct LineSlope;
+template <> struct LineSlope<float> {
+    float t;
+    __device__ __forceinline__ void set(float d) { t = d; }
+};
+template <> struct LineSlope<double> {
+    double t, y;
+    __device__ __forceinline__ void set(double d) {
+        const unsigned long long m = dmag(d);
+        t = m <= dbits(SMALL) ? dfrom((dbits(d) & D_SIGN) | dbits(SMALL)) : d;
+        y = __drcp_rn(t);
+    }
+};
+// vl_phi
+__device__ __forceinline__ double line_phi(double rat) {
+    const double s = __dadd_rn(1.0, rat);
+    if (!(dbits(rat) & D_SIGN)) return __ddiv_rn(__dadd_rn(rat, rat), s);
+    // rat < 0: rat + |rat| = +0 over 1 + rat, or 0 where that is small
+    return ((dbits(s) & D_SIGN) && dmag(s) > dbits(SMALL) && dmag(s) <= D_INF) ? -0.0 : 0.0;
+}
+// the right state of the face between cells (k, k+1) is v(k) minus, the left
+// state of the face after it v(k) plus, what Din of k and k+1 give (ho_lr)
+__device__ __forceinline__ void line_pair(const LineSlope<float> &a, const LineSlope<float> &b, float v, float &R, float &L) {
+    const float h = (a.t * b.t > 0.0f) ? __fdividef(2.0f * a.t * b.t, a.t + b.t) : 0.0f;
+    R = v - 0.5f * h;
+    L = v + 0.5f * h;
+}
+__device__ __forceinline__ void line_pair(const LineSlope<double> &a, const LineSlope<double> &b, double v, double &R, double &L) {
+    double r1, r2;
+    const unsigned long long big = (1023ull + 300) << 52;
+    if (dmag(a.t) < big && dmag(b.t) < big) {
+        // b/a and a/b by the slopes' reciprocals (their signs: Markstein's
+        // steps do not depend on them)
+        const double q1 = __dmul_rn(b.t, a.y), q2 = __dmul_rn(a.t, b.y);
+        r1 = __fma_rn(__fma_rn(-q1, a.t, b.t), a.y, q1);
+        r2 = __fma_rn(__fma_rn(-q2, b.t, a.t), b.y, q2);
     } else {
-        if (i > g.ie || j > g.je + 1) continue;
+        r1 = b.t / a.t;
+        r2 = a.t / b.t;
     }
-    const int own = DIR == 0 ? tx : ty + r * BY;
-    const int line = DIR == 0 ? ty + r * BY : tx;
-    const int fid = i + j * g.pitch;
-    const int cm = fid - stride;  // cell pos-1 (cell pos is fid)
-    const int kf = own + 1;
-    T Lv[7], Rv[7];
-#pragma unroll
-    for (int vv = 0; vv < 7; vv++) {
-        if (vv >= nvar) {
-            Lv[vv] = (T)0;
-            Rv[vv] = (T)0;
-            continue;
-        }
-        ho_lr(ro(src[vv] + (cm)), ro(src[vv] + (fid)), din[vv][line][kf - 1], din[vv][line][kf], din[vv][line][kf + 1], Lv[vv],
-              Rv[vv]);
+    const double A = __dmul_rn(line_phi(r1), a.t), B = __dmul_rn(line_phi(r2), b.t);
+    // 2 x: exact, so van * t doubled is (2 van) * t
+    L = __dadd_rn(v, __dmul_rn(1.0 / 6.0, __dadd_rn(A, __dadd_rn(B, B))));
+    R = __dsub_rn(v, __dmul_rn(1.0 / 6.0, __dadd_rn(__dadd_rn(A, A), B)));
+}
+
+// the three fluxes of a face (hll): in FP64 their common divisor's reciprocal
+// is taken once
+__device__ __forceinline__ void hll3(float SL, float SR, float F0L, float F0R, float U0L, float U0R, float F1L, float F1R,
+                                     float U1L, float U1R, float F2L, float F2R, float U2L, float U2R, float &A,
+                                     float &B, float &C) {
+    const float r = SR - SL, d = fabsf(r) < (float)SMALL ? (float)SMALL : r, sp = SL * SR;
+    const float a = SR * F0L - SL * F0R + sp * (U0R - U0L), b = SR * F1L - SL * F1R + sp * (U1R - U1L),
+                c = SR * F2L - SL * F2R + sp * (U2R - U2L);
+    A = SL >= 0.0f ? F0L : SR <= 0.0f ? F0R : __fdividef(a, d);
+    B = SL >= 0.0f ? F1L : SR <= 0.0f ? F1R : __fdividef(b, d);
+    C = SL >= 0.0f ? F2L : SR <= 0.0f ? F2R : __fdividef(c, d);
+}
+__device__ __forceinline__ void hll3(double SL, double SR, double F0L, double F0R, double U0L, double U0R, double F1L,
+                                     double F1R, double U1L, double U1R, double F2L, double F2R, double U2L,
+                                     double U2R, double &A, double &B, double &C) {
+    const double ds = SR - SL;
+    if (SL >= 0.0 || SR <= 0.0 || !(ds >= SMALL && ds < 0x1p300)) {
+        A = hll(SL, SR, F0L, F0R, U0L, U0R);
+        B = hll(SL, SR, F1L, F1R, U1L, U1R);
+        C = hll(SL, SR, F2L, F2R, U2L, U2R);
+        return;
     }
+    const double y = __drcp_rn(ds), sp = SL * SR;
+    A = div_rcp(SR * F0L - SL * F0R + sp * (U0R - U0L), ds, y);
+    B = div_rcp(SR * F1L - SL * F1R + sp * (U1R - U1L), ds, y);
+    C = div_rcp(SR * F2L - SL * F2R + sp * (U2R - U2L), ds, y);
+}
+
+// one face from its left and right states: wave speeds, HLL and
+// BOUNDARY_CONDITION (walls and dry faces; last write wins).  pos: the face's
+// index along DIR; mL, mR: MASK of the cells pos-1 and pos
+template <typename T, int DIR>
+__device__ __forceinline__ void face_flux(const Grid &g, const T *Lv, const T *Rv, T Dd, T m9, int pos, int mL, int mR,
+                                          T &Pm, T &Nm, T &Tm) {
+    const T g1 = GC(gamma1), g3 = GC(gamma3);
+    const int lo = DIR == 0 ? g.ib : g.jb, hi = DIR == 0 ? g.ie : g.je;
     const T UL = Lv[0], UR = Rv[0], VL = Lv[1], VR = Rv[1], HUL = Lv[2], HUR = Rv[2];
     const T HVL = Lv[3], HVR = Rv[3], EL = Lv[4], ER = Rv[4];
     const T U4L = Lv[5], U4R = Rv[5], V4L = Lv[6], V4R = Rv[6];
-    const T Dd = DIR == 0 ? ro(f.Depthx + (fid)) : ro(f.Depthy + (fid));
     const T HL = EL + Dd, HR = ER + Dd;
-    // MASK9u(Mloc1,:) = MASK9(Mloc,:) (fluxes.F:1333); the faces computed
-    // here never reach that column
-    const T m9 = m2r<T>(ro(f.MASK9 + (fid)));
     const T nL = DIR == 0 ? UL : VL, nR = DIR == 0 ? UR : VR;
     const T tL = DIR == 0 ? VL : UL, tR = DIR == 0 ? VR : UR;
     const T n4L = DIR == 0 ? U4L : V4L, n4R = DIR == 0 ? U4R : V4R;
@@ -582,11 +662,8 @@ __global__ void __launch_bounds__(256) k_flux(Grid g, Fields<T> f) {
     const T U_S = (T)0.5 * (nL + nR) + SQR_PHI_L - SQR_PHI_R;
     const T SL = tmin(nL - SQR_PHI_L, U_S - SQR_PHI_S);
     const T SR = tmax(nR + SQR_PHI_R, U_S + SQR_PHI_S);
-    T Pm = hll(SL, SR, ML, MR, EL, ER);
-    T Nm = hll(SL, SR, NL, NR, qnL, qnR);
-    T Tm = hll(SL, SR, TL, TR, qtL, qtR);
+    hll3(SL, SR, ML, MR, EL, ER, NL, NR, qnL, qnR, TL, TR, qtL, qtR, Pm, Nm, Tm);
     // BOUNDARY_CONDITION: walls, then the dry-cell loop (last write wins)
-    const int pos = DIR == 0 ? i : j;
     const bool wall_on = DIR == 0 || !g.periodic;
     if (wall_on && pos == lo) {
         Pm = (T)0;
@@ -598,7 +675,6 @@ __global__ void __launch_bounds__(256) k_flux(Grid g, Fields<T> f) {
         Nm = press(EL, Dd, g3);
         Tm = (T)0;
     }
-    const int mL = ro(f.MASK + (cm)), mR = ro(f.MASK + (fid));  // cells pos-1 and pos
     if (mL < 1) {
         Pm = (T)0;
         Nm = (pos - 1 != hi) ? press(ER, Dd, g3) * m2r<T>(mR) : (T)0;
@@ -609,24 +685,185 @@ __global__ void __launch_bounds__(256) k_flux(Grid g, Fields<T> f) {
         Nm = (pos != lo) ? press(EL, Dd, g3) * m2r<T>(mL) : (T)0;
         Tm = (T)0;
     }
-    if (DIR == 0) {
-        f.P[fid] = Pm;
-        f.Fx[fid] = Nm;
-        f.Gx[fid] = Tm;
-    } else {
-        f.Q[fid] = Pm;
-        f.Gy[fid] = Nm;
-        f.Fy[fid] = Tm;
+}
+
+// FLUXES along y: a thread walks `strip` faces of one column, keeping each
+// field's last two cells, slopes, Din and the left state of the next face in
+// registers, so that a cell is loaded once and Din, and the pair of Din that
+// two faces share, are computed once.  The next face's cells are loaded while
+// a face is computed (without that, 189 us at 2048 x 2048: 20 warps to an SM
+// do not hide the loads).  The tiles that shared Din through shared memory
+// took 790 instructions per face; this takes 400.  2048 x 2048 float: 121 ->
+// 66 us (the bound: instruction issue); 701 x 937 double: 1493 -> 980 us, of
+// which the FP64 pipe is the bound.
+template <typename T>
+__global__ void __launch_bounds__(128) k_flux_y(Grid g, Fields<T> f, int strip) {
+    const int i = blockIdx.x * 32 + threadIdx.x;
+    const int j0 = g.jb + (blockIdx.y * blockDim.y + threadIdx.y) * strip;
+    if (i < g.ib || i > g.ie || j0 > g.je + 1) return;
+    const int j1 = min(j0 + strip - 1, g.je + 1);
+    const T *const src[7] = {f.U, f.V, f.HU, f.HV, f.Eta, f.U4, f.V4};
+    const bool disp = g.dispersion != 0;
+    T v1[7], v2[7], T1[7], T2[7], L[7];  // cells j-1 (then j) and j+1, their slopes, the next left state
+    LineSlope<T> d[7];
+    int o = i + j0 * g.pitch;
+    // MASK of the cells j-3 .. j+2 of face j, bit 0 the first
+    int mk = 0;
+#pragma unroll
+    for (int q = 0; q < 5; q++) mk |= (int)ro(f.MASK + (o + (q - 3) * g.pitch)) << q;
+#pragma unroll
+    for (int q = 0; q < 7; q++) {
+        if (q >= 5 && !disp) {
+            v1[q] = v2[q] = T1[q] = T2[q] = L[q] = (T)0;
+            d[q].set((T)0);
+            continue;
+        }
+        const T *s = src[q] + o;
+        const T a = ro(s - 3 * g.pitch), b = ro(s - 2 * g.pitch), c = ro(s - g.pitch);
+        v1[q] = ro(s);
+        v2[q] = ro(s + g.pitch);
+        const T Ta = b - a, Tb = c - b;
+        T1[q] = v1[q] - c;
+        T2[q] = v2[q] - v1[q];
+        LineSlope<T> dm;
+        dm.set(line_din(Ta, Tb, T1[q], (mk & 0xf) == 0xf));
+        d[q].set(line_din(Tb, T1[q], T2[q], (mk & 0x1e) == 0x1e));
+        T r;
+        line_pair(dm, d[q], c, r, L[q]);
     }
+    // the cells j+2 and the face's depth and masks, one face ahead
+    T v3[7], Dd = ro(f.Depthy + o);
+    int mq = ro(f.MASK + (o + 2 * g.pitch)), m9 = ro(f.MASK9 + o);
+#pragma unroll
+    for (int q = 0; q < 7; q++) v3[q] = q < 5 || disp ? ro(src[q] + (o + 2 * g.pitch)) : (T)0;
+#pragma unroll 2
+    for (int j = j0; j <= j1; j++, o += g.pitch) {
+        mk |= mq << 5;
+        const bool wet = (mk & 0x3c) == 0x3c;
+        const T Dj = Dd, m9j = m2r<T>(m9);
+        T c3[7];
+#pragma unroll
+        for (int q = 0; q < 7; q++) c3[q] = v3[q];
+        if (j < j1) {
+            const int on = o + g.pitch;
+            Dd = ro(f.Depthy + on);
+            m9 = ro(f.MASK9 + on);
+            mq = ro(f.MASK + (on + 2 * g.pitch));
+#pragma unroll
+            for (int q = 0; q < 7; q++)
+                if (q < 5 || disp) v3[q] = ro(src[q] + (on + 2 * g.pitch));
+        }
+        T Lv[7], Rv[7];
+#pragma unroll
+        for (int q = 0; q < 7; q++) {
+            if (q >= 5 && !disp) {
+                Lv[q] = Rv[q] = (T)0;
+                continue;
+            }
+            const T T3 = c3[q] - v2[q];
+            LineSlope<T> dn;
+            dn.set(line_din(T1[q], T2[q], T3, wet));
+            Lv[q] = L[q];
+            line_pair(d[q], dn, v1[q], Rv[q], L[q]);
+            d[q] = dn;
+            v1[q] = v2[q];
+            v2[q] = c3[q];
+            T1[q] = T2[q];
+            T2[q] = T3;
+        }
+        T Pm, Nm, Tm;
+        face_flux<T, 1>(g, Lv, Rv, Dj, m9j, j, (mk >> 2) & 1, (mk >> 3) & 1, Pm, Nm, Tm);
+        f.Q[o] = Pm;
+        f.Gy[o] = Nm;
+        f.Fy[o] = Tm;
+        mk >>= 1;
+    }
+}
+
+// FLUXES along x: a lane takes two neighbouring cells (one 8- or 16-byte load
+// per field) and their two faces, and gets the neighbours' slopes, Din and
+// left state from the lanes beside it; lanes 2 .. 30 have all they need, so a
+// warp covers FLUX_XW = 58 faces of a row.  2048 x 2048 float: 112 -> 63 us
+// (before: 32 x 8 tiles, Din through shared memory); 701 x 937 double: 1722
+// -> 725 us.
+constexpr int FLUX_XW = 58;
+template <typename T> __device__ __forceinline__ T shup(T x) { return __shfl_up_sync(0xffffffffu, x, 1); }
+template <typename T> __device__ __forceinline__ T shdn(T x) { return __shfl_down_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ LineSlope<float> slope_dn(const LineSlope<float> &a) {
+    LineSlope<float> r;
+    r.t = shdn(a.t);
+    return r;
+}
+__device__ __forceinline__ LineSlope<double> slope_dn(const LineSlope<double> &a) {
+    LineSlope<double> r;
+    r.t = shdn(a.t);
+    r.y = shdn(a.y);
+    return r;
+}
+template <typename T>
+__global__ void __launch_bounds__(128) k_flux_x(Grid g, Fields<T> f, int rows) {
+    using T2 = typename std::conditional<sizeof(T) == sizeof(double), double2, float2>::type;
+    const int lane = threadIdx.x;
+    const int i = FLUX_XW * blockIdx.x - 2 + 2 * lane;  // the lane's cells i, i+1 and the faces before them
+    const int j0 = g.jb + (blockIdx.y * blockDim.y + threadIdx.y) * rows;
+    if (j0 > g.je) return;
+    const int j1 = min(j0 + rows - 1, g.je);
+    const T *const src[7] = {f.U, f.V, f.HU, f.HV, f.Eta, f.U4, f.V4};
+    const bool disp = g.dispersion != 0, mine = lane >= 2 && lane <= 30;
+    // cells left of the plane's rows or past their end are other rows' cells:
+    // loaded (rows 3 .. Nloc-4 of Nloc+1), never used by a face of the domain
+    for (int j = j0; j <= j1; j++) {
+        const int o = i + j * g.pitch;
+        const uchar2 m = __ldg((const uchar2 *)(f.MASK + o));
+        const int mo = (int)m.x | ((int)m.y << 1);
+        // MASK of the cells i-2 .. i+3, bit 0 the first
+        const int mk = shup(mo) | (mo << 2) | (shdn(mo) << 4);
+        const T2 Dd = __ldg((const T2 *)(f.Depthx + o));
+        const uchar2 m9 = __ldg((const uchar2 *)(f.MASK9 + o));
+        T2 vv[7];
+#pragma unroll
+        for (int q = 0; q < 7; q++) vv[q] = q < 5 || disp ? __ldg((const T2 *)(src[q] + o)) : T2{(T)0, (T)0};
+        T La[7], Ra[7], Lb[7], Rb[7];  // faces i and i+1
+#pragma unroll
+        for (int q = 0; q < 7; q++) {
+            const T2 v = vv[q];
+            const T Ta = v.x - shup(v.y), Tb = v.y - v.x;  // v(i)-v(i-1), v(i+1)-v(i)
+            const T Tm = shup(Tb), Tp = shdn(Ta);
+            LineSlope<T> da, db;
+            da.set(line_din(Tm, Ta, Tb, (mk & 0xf) == 0xf));
+            db.set(line_din(Ta, Tb, Tp, (mk & 0x1e) == 0x1e));
+            T Ln;
+            line_pair(da, db, v.x, Ra[q], Lb[q]);
+            line_pair(db, slope_dn(da), v.y, Rb[q], Ln);
+            La[q] = shup(Ln);
+        }
+        if (!mine) continue;
+        T P0, N0, T0, P1, N1, T1;
+        face_flux<T, 0>(g, La, Ra, Dd.x, m2r<T>(m9.x), i, (mk >> 1) & 1, (mk >> 2) & 1, P0, N0, T0);
+        face_flux<T, 0>(g, Lb, Rb, Dd.y, m2r<T>(m9.y), i + 1, (mk >> 2) & 1, (mk >> 3) & 1, P1, N1, T1);
+        if (i >= g.ib && i + 1 <= g.ie + 1) {
+            *(T2 *)(f.P + o) = T2{P0, P1};
+            *(T2 *)(f.Fx + o) = T2{N0, N1};
+            *(T2 *)(f.Gx + o) = T2{T0, T1};
+        } else if (i >= g.ib && i <= g.ie + 1) {
+            f.P[o] = P0;
+            f.Fx[o] = N0;
+            f.Gx[o] = T0;
+        } else if (i + 1 >= g.ib && i + 1 <= g.ie + 1) {
+            f.P[o + 1] = P1;
+            f.Fx[o + 1] = N1;
+            f.Gx[o + 1] = T1;
+        }
     }
 }
 
 // The tile's inputs staged by TMA: one 2-D tensor load of each of U V HU HV
 // Eta U4 V4 (40 cells wide from i0 - 3, FY rows from j0 for x faces or FY+6
 // rows from j0 - 3 for y faces) and of MASK (48 wide), completing on one
-// mbarrier; Din and the faces then read shared memory.  i0 - 3 is a
+// mbarrier; Din of the seven fields is computed once per cell position into
+// shared memory, and each thread finishes its faces from there.  i0 - 3 is a
 // multiple of 32 (ib = 3), so every box starts on a 16-byte boundary.  The
-// same arithmetic as k_flux, so the same results.
+// same results as k_flux_x and k_flux_y, bit for bit.
 template <typename T, int DIR, int FY_> struct FluxStage {
     using TL = FluxTile<T, DIR, FY_>;
     static constexpr int BW = 40, BWM = 48;             // staged columns from i0 - 3
@@ -3634,7 +3871,7 @@ __global__ void __launch_bounds__(256) k_end(Grid g, Fields<T> f, int track_hmax
 // ---------------------------------------------------------------------------
 static inline dim3 grid2(int nx, int ny, dim3 b) { return dim3((nx + b.x - 1) / b.x, (ny + b.y - 1) / b.y); }
 static const dim3 B2D(32, 8);
-// blocks of k_flux: tiles of FX x FY faces over (Mglob+1) x Nglob x-faces
+// blocks of k_flux_tma: tiles of FX x FY faces over (Mglob+1) x Nglob x-faces
 // or Mglob x (Nglob+1) y-faces
 template <typename T, int DIR, int FY_ = flux_fy_default<T, DIR>()> static dim3 flux_grid(const Grid &g) {
     using TL = FluxTile<T, DIR, FY_>;
@@ -3708,13 +3945,6 @@ template <typename T> void launch_dispersion(fw_ctx *c) {
     note(c);
 }
 
-// the compiled flux tile heights: 8, 16 or 32 faces in float; 8 or 16 in
-// double (a 32-high tile of doubles would not fit 48 KB)
-
-template <typename T, int DIR, int FY_> static void flux_at(fw_ctx *c) {
-    k_flux<T, DIR, FY_><<<flux_grid<T, DIR, FY_>(c->g), B2D, 0, c->stream>>>(c->g, c->F<T>());
-}
-
 // the TMA-staged flux kernel with the maps of the current MASK buffer (its
 // shared-memory size is set when the maps are made, outside any capture)
 template <typename T, int DIR, int FY_> static void flux_tma_at(fw_ctx *c) {
@@ -3744,13 +3974,18 @@ template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
         note(c);
         return;
     }
-    if constexpr (sizeof(T) == sizeof(float)) {
-        if (fy == 8) flux_at<T, DIR, 8>(c);
-        else if (fy == 16) flux_at<T, DIR, 16>(c);
-        else flux_at<T, DIR, 32>(c);
+    // the tuned height is what a block of four warps covers along y; halved
+    // while the grid has fewer warps than the SMs take
+    const Grid &g = c->g;
+    const dim3 b(32, 4);
+    if (DIR == 0) {
+        const int rows = std::max(1, fy / 8), nx = (g.ie + FLUX_XW) / FLUX_XW;
+        k_flux_x<T><<<dim3(nx, (g.Nglob + 4 * rows - 1) / (4 * rows)), b, 0, c->stream>>>(g, c->F<T>(), rows);
     } else {
-        if (fy == 8) flux_at<T, DIR, 8>(c);
-        else flux_at<T, DIR, 16>(c);
+        const int nx = (g.ie + 32) / 32;
+        int strip = fy;
+        while (strip > 4 && nx * ((g.Nglob + strip) / strip) < 152 * 16) strip /= 2;
+        k_flux_y<T><<<dim3(nx, (g.Nglob + 4 * strip) / (4 * strip)), b, 0, c->stream>>>(g, c->F<T>(), strip);
     }
     note(c);
 }
