@@ -145,11 +145,20 @@ template <typename T> int get_field(fw_ctx *c, const FieldRef &r, void *host) {
     return cuda_status(c, e);
 }
 
+// a field that the FP64 line solver's kept factors depend on was set: factor
+// again at the next solve (the mixed factors follow MASK9's own changes)
+int refactor_after(fw_ctx *c, const char *name) {
+    if (c->p.precision != FW_PREC_FP64) return FW_OK;
+    if (std::strcmp(name, "Depth") && std::strcmp(name, "MASK9") && std::strcmp(name, "MASK")) return FW_OK;
+    return cuda_status(c, cudaMemsetAsync(c->fd.m9_dirty, 1, sizeof(int), c->stream));
+}
+
 int put_named(fw_ctx *c, const char *name, const void *host) {
     FieldRef r;
     if (c->p.precision == FW_PREC_FP64) {
         if (!find_field<double>(c, name, r)) return FW_ERR_BAD_PARAM;
-        return put_field<double>(c, r, host);
+        const int rc = put_field<double>(c, r, host);
+        return rc == FW_OK ? refactor_after(c, name) : rc;
     }
     if (!find_field<float>(c, name, r)) return FW_ERR_BAD_PARAM;
     int rc = put_field<float>(c, r, host);
@@ -874,7 +883,8 @@ int fw_set_field_f32(fw_ctx *c, const char *name, const float *host) {
         }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    return cuda_status(c, e);
+    if (e != cudaSuccess) return cuda_status(c, e);
+    return refactor_after(c, name);
 }
 
 int fw_get_points(fw_ctx *c, const char *name, int n, const int *I, const int *J, double *out) {
@@ -1711,6 +1721,7 @@ int fw_set_fields(fw_ctx *c, int n, const char *const *names, const void *const 
             e = cudaMemcpy2DAsync(c->ff.DepthD, (size_t)c->g.pitch * sizeof(double), buf + off[k],
                                   (size_t)w * sizeof(double), (size_t)w * sizeof(double), (size_t)h,
                                   cudaMemcpyDeviceToDevice, c->stream);
+        if (e == cudaSuccess && (rc = refactor_after(c, names[k])) != FW_OK) return rc;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_status(c, e);

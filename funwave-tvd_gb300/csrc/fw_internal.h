@@ -74,7 +74,9 @@ struct Fields {
     T *Eta0, *Ubar0, *Vbar0, *U0, *V0;
     T *Depth, *Depthx, *Depthy, *Cd, *SPONGE, *CD4;
     T *P, *Q, *Fx, *Fy, *Gx, *Gy;
-    T *A, *B, *C, *E;                 // mixed: exchanged Uxx+Vxy, DUxx+DVxy, Uxy+Vyy, DUxy+DVyy
+    // mixed: exchanged Uxx+Vxy, DUxx+DVxy, Uxy+Vyy, DUxy+DVyy; FP64: the Thomas
+    // solves' kept factors (c' and 1/den of the x and the y lines)
+    T *A, *B, *C, *E;
     // FP64: the exchanged terms themselves; mixed: the line solver's reduction multipliers
     T *Uxx, *Vxy, *Uxy, *Vyy, *DUxx, *DVxy, *DUxy, *DVyy;
     T *U4, *V4, *U1p, *V1p, *Udisp, *Vdisp;  // Udisp = U1pp+U2+U3

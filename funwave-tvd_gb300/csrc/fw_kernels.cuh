@@ -88,6 +88,33 @@ template <typename T> __device__ __forceinline__ T tmax(T a, T b) { return a > b
 template <typename T> __device__ __forceinline__ T tmin(T a, T b) { return a < b ? a : b; }
 
 // ---------------------------------------------------------------------------
+// FP64 arithmetic beside the FP64 pipe.  GB300 issues double operations at
+// 1/64 of the float rate and integer ones beside them, so comparisons,
+// absolute values and doublings of doubles are done on their bits, and
+// quotients by a divisor whose reciprocal is at hand take one product and two
+// fused operations.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
+__device__ __forceinline__ double dfrom(unsigned long long b) { return __longlong_as_double((long long)b); }
+constexpr unsigned long long D_SIGN = 1ull << 63, D_INF = 0x7ffull << 52;
+__device__ __forceinline__ unsigned long long dmag(double x) { return dbits(x) & ~D_SIGN; }
+
+// a / b rounded to nearest, with y = RN(1/b): q = RN(a y), r = a - b q
+// (exact), RN(q + r y) (Markstein, IBM J. Res. Dev. 34 (1990): correctly
+// rounded when y is, and nothing under- or overflows).  |b| lies in
+// [2^-300, 2^300] (the callers' spacings, steps and coefficients); an a
+// outside [2^-500, 2^500], zero apart, takes the division.
+__device__ __forceinline__ double div_rcp(double a, double b, double y) {
+    const unsigned long long m = dmag(a);
+    if (m - ((1023ull - 500) << 52) >= (1000ull << 52)) {
+        if (m == 0) return dfrom(dbits(a) ^ (dbits(b) & D_SIGN));
+        return a / b;
+    }
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// ---------------------------------------------------------------------------
 // exchange source of a ghost cell (PHI_COLL, serial branches)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int mirror_x(const Grid &g, int i) {
@@ -482,33 +509,6 @@ template <typename T, int DIR, int FY_ = flux_fy_default<T, DIR>()> struct FluxT
     static constexpr int NPOS = NB + 2;                // Din positions per line
     static constexpr int NP = DIR == 0 ? NPOS : NPOS + 1;  // odd row length for y
 };
-
-// ---------------------------------------------------------------------------
-// FP64 arithmetic beside the FP64 pipe.  GB300 issues double operations at
-// 1/64 of the float rate and integer ones beside them, so comparisons,
-// absolute values and doublings of doubles are done on their bits, and
-// quotients by a divisor whose reciprocal is at hand take one product and two
-// fused operations.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
-__device__ __forceinline__ double dfrom(unsigned long long b) { return __longlong_as_double((long long)b); }
-constexpr unsigned long long D_SIGN = 1ull << 63, D_INF = 0x7ffull << 52;
-__device__ __forceinline__ unsigned long long dmag(double x) { return dbits(x) & ~D_SIGN; }
-
-// a / b rounded to nearest, with y = RN(1/b): q = RN(a y), r = a - b q
-// (exact), RN(q + r y) (Markstein, IBM J. Res. Dev. 34 (1990): correctly
-// rounded when y is, and nothing under- or overflows).  b > 0 lies in
-// [2^-300, 2^300] (the callers' spacings, steps and guarded slopes); an a
-// outside [2^-500, 2^500], zero apart, takes the division.
-__device__ __forceinline__ double div_rcp(double a, double b, double y) {
-    const unsigned long long m = dmag(a);
-    if (m - ((1023ull - 500) << 52) >= (1000ull << 52)) {
-        if (m == 0) return a;
-        return a / b;
-    }
-    const double q = __dmul_rn(a, y);
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
-}
 
 // ---------------------------------------------------------------------------
 // The reconstruction along a line, with every quantity computed once: Din at
@@ -1633,6 +1633,138 @@ __global__ void __launch_bounds__(256) k_thomas_rows(Grid g, Fields<T> f, LinePa
     }
 }
 
+// With viscosity breaking MASK9 does not change once it is set, and with it
+// the matrices stay: den and c' of every row depend on Depth, MASK9 and MASK
+// alone.  k_thomas_fac walks the lines once per change (m9_dirty) and keeps c'
+// and RN(1/den), and for periodic lines the second solution (tq); the solves
+// (k_thomas_solve) then divide by den through its reciprocal
+// (div_rcp: the same rounding), which leaves one sum, one product and two
+// fused operations of each row on a line's critical path, and k_thomas_rows
+// prepares d/a alone.  A den outside div_rcp's range keeps 0 for its
+// reciprocal and is divided by.
+// The planes are those that only the mixed mode's dispersion terms use.
+template <typename T, int DIR> __device__ __forceinline__ double *tf_c(const Fields<T> &f) { return (double *)(DIR == 0 ? f.A : f.C); }
+template <typename T, int DIR> __device__ __forceinline__ double *tf_y(const Fields<T> &f) { return (double *)(DIR == 0 ? f.B : f.E); }
+__device__ __forceinline__ bool div_rcp_ok(double b) {
+    const unsigned long long m = dmag(b);
+    return m >= ((1023ull - 300) << 52) && m <= ((1023ull + 300) << 52);
+}
+
+// a, c, 1 + c_end or 1 + a_beg (the scale of a periodic line's end rows, else
+// 1) and tmp2 of row k
+template <typename T, int DIR, bool PER>
+__device__ __forceinline__ void thomas_row(const Grid &g, const Fields<T> &f, const LinePart &lp, int i, int j, double &a,
+                                           double &c, double &sc) {
+    const int k = DIR == 0 ? i - g.ib : j - g.jb;
+    double d;
+    tri_coef<T, DIR>(g, f, i, j, a, c, d);
+    sc = 1.0;
+    if (PER && (k == 0 || k == lp.L - 1)) {
+        double a2, c2;
+        const bool first = k == 0;
+        tri_coef<T, DIR>(g, f, DIR == 0 ? (first ? g.ie : g.ib) : i, DIR == 0 ? j : (first ? g.je : g.jb), a2, c2, d);
+        sc = 1 + (first ? c2 : a2);
+        if (first) c = c / sc;
+        else a = a / sc;
+    }
+}
+
+template <typename T, int DIR, bool PER>
+__device__ __forceinline__ void thomas_ends(const Grid &g, const Fields<T> &f, const LinePart &lp, int l, double &a_beg, double &c_end) {
+    double a, c, d;
+    int i, j;
+    line_cell<DIR>(g, l, 0, i, j);
+    tri_coef<T, DIR>(g, f, i, j, a, c, d);
+    a_beg = a;
+    line_cell<DIR>(g, l, lp.L - 1, i, j);
+    tri_coef<T, DIR>(g, f, i, j, a, c, d);
+    c_end = c;
+}
+template <typename T, int DIR, bool PER>
+__device__ void thomas_fac_body(const Grid &g, const Fields<T> &f, const LinePart &lp, int l) {
+    if (l >= lp.nlines) return;
+    double *FC = tf_c<T, DIR>(f), *FY = tf_y<T, DIR>(f);
+    double cp = 0.0, ep = 0.0, e_first = 0.0, e_last = 0.0;
+    if (PER) {
+        // e = [1/(1+c_end), 0, ..., 0, -1/(1+a_beg)] (tridiagnal.F:207-215)
+        double a_beg, c_end;
+        thomas_ends<T, DIR, PER>(g, f, lp, l, a_beg, c_end);
+        e_first = 1.0 / (1.0 + c_end);
+        e_last = -1.0 / (1.0 + a_beg);
+    }
+    for (int k = 0; k < lp.L; k++) {
+        int i, j;
+        line_cell<DIR>(g, l, k, i, j);
+        double a, c, sc;
+        thomas_row<T, DIR, PER>(g, f, lp, i, j, a, c, sc);
+        double y = 0.0;
+        if (k > 0 && a != 0.0) {
+            const double den = 1.0 / a - cp;
+            cp = (c / a) / den;
+            if (div_rcp_ok(den)) y = 1.0 / den;
+            // e/a: 0/a is a zero with the sign of a; the last row's a is scaled
+            if (PER) ep = ((k == lp.L - 1 ? e_last / a : fcopysign(0.0, a)) - ep) / den;
+        } else {
+            cp = c;
+            if (PER) ep = k == lp.L - 1 ? e_last : (k == 0 ? e_first : 0.0);
+        }
+        FC[IDX(i, j)] = cp;
+        FY[IDX(i, j)] = y;
+        if (PER) f.tq[IDX(i, j)] = ep;
+    }
+    if (PER)
+        for (int k = lp.L - 2; k >= 0; k--) {
+            int i, j;
+            line_cell<DIR>(g, l, k, i, j);
+            ep = f.tq[IDX(i, j)] - FC[IDX(i, j)] * ep;
+            f.tq[IDX(i, j)] = ep;
+        }
+}
+// both directions in one launch: blocks [0, nbx) factor x, the rest y
+template <typename T, bool PERY>
+__global__ void __launch_bounds__(32) k_thomas_fac(Grid g, Fields<T> f, LinePart px, LinePart py, int nbx) {
+    if (!*f.m9_dirty) return;
+    if ((int)blockIdx.x < nbx) thomas_fac_body<T, 0, false>(g, f, px, blockIdx.x * 32 + threadIdx.x);
+    else thomas_fac_body<T, 1, PERY>(g, f, py, (blockIdx.x - nbx) * 32 + threadIdx.x);
+}
+
+// d/a (or d) and 1/a (or 0) of every row, as k_thomas_rows
+template <typename T, int DIR, bool PER>
+__global__ void __launch_bounds__(256) k_thomas_rhs(Grid g, Fields<T> f, LinePart lp, int clear_dirty) {
+    if (clear_dirty && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *f.m9_dirty = 0;
+    const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = g.jb + blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > g.ie || j > g.je) return;
+    const size_t q = IDX(i, j);
+    const int k = DIR == 0 ? i - g.ib : j - g.jb;
+    // tri_coef's a and d; tmp2 > 0 here (the launcher's condition)
+    const double mdf = g.min_depth_frc, g1 = g.gamma1;
+    const double dep = tmax((double)ro(f.Depth + q), mdf);
+    const double depl = tmax((double)ro(f.Depth + (DIR == 0 ? IDX(i - 1, j) : IDX(i, j - 1))), mdf);
+    const double m9 = ro(f.MASK9 + q) ? 1.0 : 0.0;
+    const double tmp4 = DIR == 0 ? ro(f.rhs_x + q) : ro(f.rhs_y + q);
+    const double k1 = g.tK1[DIR], k2 = g.tK2[DIR], k3 = g.tK3[DIR], k4 = g.tK4[DIR];
+    const double gm = g1 * m9;
+    const double tmp1 = gm * (k1 * dep * dep + k2 * depl * dep);
+    const double tmp2 = 1.0 + gm * (k3 * dep * dep - k4 * dep * dep);
+    const double r2 = __drcp_rn(tmp2);
+    const bool ok = div_rcp_ok(tmp2);
+    double a = ok ? div_rcp(tmp1, tmp2, r2) : tmp1 / tmp2, d = ok ? div_rcp(tmp4, tmp2, r2) : tmp4 / tmp2;
+    if (PER && (k == 0 || k == lp.L - 1)) {
+        double a2, c2, sc;
+        thomas_row<T, DIR, PER>(g, f, lp, i, j, a2, c2, sc);
+        if (k > 0) a = a / sc;
+        d = d / sc;
+    }
+    double ra = 0.0;
+    if (k > 0 && a != 0.0) {
+        ra = __drcp_rn(a);
+        d = div_rcp_ok(a) ? div_rcp(d, a, ra) : d / a;
+    }
+    f.tc[q] = ra;
+    f.ty[q] = d;
+}
+
 template <typename T, int DIR, bool PER>
 __global__ void __launch_bounds__(32) k_thomas_lines(Grid g, Fields<T> f, LinePart lp) {
     constexpr int U = 8;  // rows per block of loads
@@ -1765,6 +1897,153 @@ __global__ void __launch_bounds__(32) k_thomas_lines(Grid g, Fields<T> f, LinePa
         for (int k = 0; k < L; k++) {
             const size_t q = base + (size_t)k * step;
             out[q] = (T)(f.ty[q] + beta * f.tq[q]);
+        }
+    }
+}
+
+// The solves with the kept factors: one warp walks 32 lines.  A line's chain
+// is d'(k) = (d/a - d'(k-1)) / den: rows are worked in blocks of eight without
+// a branch, with the next block's loads in flight, and a block that holds a
+// row that is not eliminated, or a numerator outside div_rcp's range, is
+// worked again row by row.  For periodic lines the second solution is kept
+// (tq) and every warp of the block adds it at the end.
+// Measured with the launches beside it (us, before -> after): 701 x 937 x 650
+// -> 326, y 1326 -> 360; 250 x 500, periodic y, x 232 -> 120, y 1262 -> 219.
+// What bounds it is the chain: four dependent FP64 operations a row forward
+// and two back.
+constexpr int THS_WARPS = 8;  // warps of a block of periodic lines
+template <typename T, int DIR, bool PER>
+__global__ void __launch_bounds__(PER ? 32 * THS_WARPS : 32) k_thomas_solve(Grid g, Fields<T> f, LinePart lp) {
+    constexpr int U = 8;
+    const int l = blockIdx.x * 32 + threadIdx.x, L = lp.L;
+    const bool on = l < lp.nlines;
+    const int base = (int)(DIR == 0 ? IDX(g.ib, g.jb + (on ? l : 0)) : IDX(g.ib + (on ? l : 0), g.jb));
+    const int step = DIR == 0 ? 1 : g.pitch;
+    T *const out = (DIR == 0 ? f.U : f.V) + base;
+    double *const dp_ = f.ty + base;
+    if (on && threadIdx.y == 0) {
+        const double *const ra_ = f.tc + base, *const fc_ = tf_c<T, DIR>(f) + base, *const fy_ = tf_y<T, DIR>(f) + base;
+        double cp = 0.0, dp = 0.0;
+        // one row as k_thomas_lines
+        auto row = [&](double ra, double da, double fc, double fy) {
+            double d = da;
+            if (ra != 0.0) {
+                const double den = ra - cp;
+                d = fy != 0.0 ? div_rcp(da - dp, den, fy) : (da - dp) / den;
+            }
+            cp = fc;
+            dp = d;
+        };
+        const int nb = L / U;
+        double ra[U], da[U], fc[U], fy[U];
+        auto load = [&](double *a, double *b, double *c, double *d, int k0) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int q = (k0 + u) * step;
+                a[u] = ra_[q];
+                b[u] = dp_[q];
+                c[u] = fc_[q];
+                d[u] = fy_[q];
+            }
+        };
+        if (nb > 0) load(ra, da, fc, fy, 0);
+        for (int b = 0; b < nb; b++) {
+            double nra[U], nda[U], nfc[U], nfy[U];
+            load(nra, nda, nfc, nfy, b + 1 < nb ? (b + 1) * U : b * U);
+            double dv[U], c0 = cp, d0 = dp;
+            unsigned bad = 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const double den = ra[u] - c0, t = da[u] - d0, y = fy[u];
+                const double q = __dmul_rn(t, y);
+                dv[u] = d0 = __fma_rn(__fma_rn(-q, den, t), y, q);
+                c0 = fc[u];
+                // exponents of t and y (both high words); a zero t divides
+                // right when y < 0
+                const int th = __double2hiint(t), yh = __double2hiint(y);
+                const unsigned te = (unsigned)th & 0x7fffffffu;
+                const bool zero = (te | (unsigned)__double2loint(t)) == 0 && yh < 0;
+                if ((yh << 1) == 0 || (te - ((1023u - 500u) << 20) >= (1000u << 20) && !zero)) bad = 1;
+            }
+            if (bad) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    row(ra[u], da[u], fc[u], fy[u]);
+                    dv[u] = dp;
+                }
+            } else {
+                cp = c0;
+                dp = d0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                dp_[(b * U + u) * step] = dv[u];
+                ra[u] = nra[u];
+                da[u] = nda[u];
+                fc[u] = nfc[u];
+                fy[u] = nfy[u];
+            }
+        }
+        for (int k = nb * U; k < L; k++) {
+            const int q = k * step;
+            row(ra_[q], dp_[q], fc_[q], fy_[q]);
+            dp_[q] = dp;
+        }
+        // back substitution: the first solution into ty (periodic), else
+        // straight into U / V
+        double z = dp;
+        auto put = [&](int k, double v) {
+            if (PER) dp_[k * step] = v;
+            else out[k * step] = (T)v;
+        };
+        put(L - 1, z);
+        int k = L - 2;
+        double d1[U], c1[U];
+        auto back = [&](double *d, double *c, int k0) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int q = max(k0 - u, 0) * step;
+                d[u] = dp_[q];
+                c[u] = fc_[q];
+            }
+        };
+        back(d1, c1, k);
+        for (; k >= U - 1; k -= U) {
+            double d2[U], c2[U];
+            back(d2, c2, k - U);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                z = d1[u] - c1[u] * z;
+                put(k - u, z);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                d1[u] = d2[u];
+                c1[u] = c2[u];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (k - u >= 0) {
+                z = d1[u] - c1[u] * z;
+                put(k - u, z);
+            }
+    }
+    if (PER) {
+        __shared__ double beta_[32];
+        if (on && threadIdx.y == 0) {
+            double a_beg, c_end;
+            thomas_ends<T, DIR, PER>(g, f, lp, l, a_beg, c_end);
+            const double *z2 = f.tq + base;
+            const int e = (L - 1) * step;
+            beta_[threadIdx.x] = (c_end * dp_[0] - a_beg * dp_[e]) / (1.0 - (c_end * z2[0] - a_beg * z2[e]));
+        }
+        __syncthreads();
+        if (on) {
+            const double beta = beta_[threadIdx.x];
+            const double *z2 = f.tq + base;
+#pragma unroll 4
+            for (int k = threadIdx.y; k < L; k += THS_WARPS) out[k * step] = (T)(__ldcg(dp_ + k * step) + beta * ro(z2 + k * step));
         }
     }
 }
@@ -3186,8 +3465,8 @@ __device__ __forceinline__ int block_scan_1024(int x, int *wsum) {
 //    pass by level t = i + 2j: the cells a candidate reads new values of
 //    lie on levels t-1, t-3, t-2, t-1, the cells it reads old values of on
 //    levels above t.  The candidates are sorted by level (a histogram, its
-//    prefix sum and a scatter, into the line solver's tq and tp planes,
-//    which are free between the stage's line solve and the next) and the
+//    prefix sum and a scatter, into the line solver's tp plane, which is
+//    free between the stage's line solve and the next) and the
 //    non-empty levels are worked in order, one barrier each.  Starting
 //    from any pass's state (a subset of the sweep's result) this gives the
 //    sweep's result, in time bounded by the candidates and the levels
@@ -3219,9 +3498,10 @@ __global__ void __launch_bounds__(1024) k_break_b(Grid g, Fields<T> f) {
         // levels of the candidate range Ibeg-1..Iend+1 x Jbeg-1..Jend+1
         const int i0 = g.ib - 1, j0 = g.jb - 1;
         const int nlev = (g.ie + 1 - i0) + 2 * (g.je + 1 - j0) + 1;
-        volatile int *off = reinterpret_cast<volatile int *>(f.tq);
-        int *off_a = reinterpret_cast<int *>(f.tq);
+        // a plane of doubles holds two planes of ints
         int *sorted = reinterpret_cast<int *>(f.tp);
+        int *off_a = sorted + (size_t)g.pitch * (size_t)(g.Nloc + 1);
+        volatile int *off = off_a;
         auto level = [&](int code) { return (code % g.pitch - i0) + 2 * (code / g.pitch - j0); };
         for (int t = threadIdx.x; t < nlev; t += 1024) off[t] = 0;
         __syncthreads();
@@ -3984,7 +4264,9 @@ template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
     } else {
         const int nx = (g.ie + 32) / 32;
         int strip = fy;
-        while (strip > 4 && nx * ((g.Nglob + strip) / strip) < 152 * 16) strip /= 2;
+        // (FP64 fills its pipe with fewer warps, and a strip's start costs it more)
+        const int enough = 152 * (sizeof(T) == sizeof(double) ? 4 : 16);
+        while (strip > 4 && nx * ((g.Nglob + strip) / strip) < enough) strip /= 2;
         k_flux_y<T><<<dim3(nx, (g.Nglob + 4 * strip) / (4 * strip)), b, 0, c->stream>>>(g, c->F<T>(), strip);
     }
     note(c);
@@ -4054,6 +4336,19 @@ static void launch_linesolve(fw_ctx *c, const LinePart &lp, bool clear_dirty) {
     note(c);
 }
 
+// FP64 solves keep the factors where MASK9 stays (viscosity breaking: without
+// it the wet/dry front moves MASK9, and factoring at every change would cost
+// more than it saves) and tmp2 cannot vanish
+static bool thomas_kept(const fw_ctx *c) {
+    return c->p.precision == FW_PREC_FP64 && c->g.visc_breaking && c->g.gamma1 >= 0.0 &&
+           -c->g.b1 - 2.0 * c->g.b2 >= 0.0;
+}
+template <typename T> static void launch_thomas_fac(fw_ctx *c) {
+    const int nbx = (c->px.nlines + 31) / 32, nby = (c->py.nlines + 31) / 32;
+    if (c->g.periodic) k_thomas_fac<T, true><<<nbx + nby, 32, 0, c->stream>>>(c->g, c->F<T>(), c->px, c->py, nbx);
+    else k_thomas_fac<T, false><<<nbx + nby, 32, 0, c->stream>>>(c->g, c->F<T>(), c->px, c->py, nbx);
+}
+
 template <typename T, int DIR, bool PER>
 static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clear_dirty = false) {
     const Grid &g = c->g;
@@ -4093,6 +4388,16 @@ static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clea
         return false;
     }
     if constexpr (sizeof(T) == sizeof(double)) {
+        if (thomas_kept(c)) {
+            if (fac) {
+                launch_thomas_fac<T>(c);
+                note(c);
+            }
+            k_thomas_rhs<T, DIR, PER><<<grid2(g.Mglob, g.Nglob, B2D), B2D, 0, c->stream>>>(g, c->F<T>(), lp, clear_dirty ? 1 : 0);
+            k_thomas_solve<T, DIR, PER><<<(lp.nlines + 31) / 32, dim3(32, PER ? THS_WARPS : 1), 0, c->stream>>>(g, c->F<T>(), lp);
+            note(c, 2);
+            return clear_dirty;
+        }
         k_thomas_rows<T, DIR, PER><<<grid2(g.Mglob, g.Nglob, B2D), B2D, 0, c->stream>>>(g, c->F<T>(), lp);
         k_thomas_lines<T, DIR, PER><<<(lp.nlines + 31) / 32, 32, 0, c->stream>>>(g, c->F<T>(), lp);
         note(c, 2);
@@ -4151,9 +4456,11 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
                 note(c);
             }
         } else {
-            launch_tri<T, 0, false>(c, c->px);
-            if (g.periodic) launch_tri<T, 1, true>(c, c->py);
-            else launch_tri<T, 1, false>(c, c->py);
+            // (kept FP64 factors: brought up to date before the x solve, which
+            // clears the change flag)
+            launch_tri<T, 0, false>(c, c->px, true, true);
+            if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
+            else launch_tri<T, 1, false>(c, c->py, false);
         }
     }
     if (!with_post) return;

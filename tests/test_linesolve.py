@@ -76,3 +76,45 @@ def test_checkpoint_of_the_earlier_factor_layout_is_factored_again(fw, size, tmp
         assert np.array_equal(a.get(n), b.get(n)), n
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("periodic", [False, True])
+@pytest.mark.parametrize("how", ["set", "set_f32", "set_fields", "mask9"])
+def test_fp64_factors_follow_a_new_depth(fw, how, periodic):
+    """The FP64 solves keep their factors while Depth, MASK9 and MASK stand:
+    a run that solved before one of them was set gives the bits of one that
+    did not."""
+    M, N = 45, 70
+    p, depth, st = _case(M, N, periodic)
+    rng = np.random.default_rng(2)
+    got = []
+    for early in (True, False):
+        s = fw.Solver(fw.with_defaults(p), precision="FP64")
+        s.init(depth, *st)
+        s.begin_step()
+        names = ("U", "V", "Eta", "Ubar", "Vbar", "H", "HU", "HV", "P", "Q")
+        keep = {n: s.get(n) for n in names}
+        if early:
+            s.cal_dispersion()
+            s.fluxes()
+            s.estimate_huv(1)
+            for n in names:
+                s.set(n, keep[n])
+        new = np.asfortranarray((s.get("Depth") * 1.25).astype(np.float32).astype(np.float64))
+        if how == "set":
+            s.set("Depth", new)
+        elif how == "set_f32":
+            s.set_f32("Depth", new.astype(np.float32))
+        elif how == "set_fields":
+            s.set_fields({"Depth": new, "Eta": keep["Eta"]})
+        else:
+            m = s.get("MASK9")
+            m[10:20, 15:30] = 0
+            s.set("MASK9", m)
+        s.cal_dispersion()
+        s.fluxes()
+        s.estimate_huv(1)
+        got.append([s.get(n) for n in ("U", "V", "Eta")])
+        s.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
