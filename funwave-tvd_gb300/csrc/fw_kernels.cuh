@@ -114,6 +114,37 @@ __device__ __forceinline__ double div_rcp(double a, double b, double y) {
     return __fma_rn(__fma_rn(-q, b, a), y, q);
 }
 
+// whether a b lies in div_rcp's range
+__device__ __forceinline__ bool div_rcp_ok(double b) {
+    const unsigned long long m = dmag(b);
+    return m >= ((1023ull - 300) << 52) && m <= ((1023ull + 300) << 52);
+}
+// a / b for any b; y = RN(1/b)
+__device__ __forceinline__ double div_any(double a, double b, double y) {
+    const bool ok = div_rcp_ok(b);  // of b alone: once for all quotients by it
+    const unsigned long long m = dmag(a);
+    if (m - ((1023ull - 500) << 52) >= (ok ? 1000ull << 52 : 0)) {
+        if (m == 0 && ok) return dfrom(dbits(a) ^ (dbits(b) & D_SIGN));
+        return a / b;
+    }
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+// x / b for a constant b of the run whose reciprocal y is at hand: FP64 by
+// div_any, which rounds as the division; the mixed path multiplies
+__device__ __forceinline__ double over(double x, double b, double y) { return div_any(x, b, y); }
+__device__ __forceinline__ float over(float x, float, float y) { return x * y; }
+// the larger of x and a positive b (b for a NaN, as tmax), on the bits in
+// FP64: doubles order like their bits against a positive one
+__device__ __forceinline__ double max_pos(double x, double b) {
+    const long long m = __double_as_longlong(x);
+    return m > __double_as_longlong(b) && m <= (long long)D_INF ? x : b;
+}
+__device__ __forceinline__ float max_pos(float x, float b) { return x > b ? x : b; }
+// a - 2 b: the product is exact, so FP64's fused operation rounds as the two
+__device__ __forceinline__ double sub2(double a, double b) { return __fma_rn(-2.0, b, a); }
+__device__ __forceinline__ float sub2(float a, float b) { return a - 2.0f * b; }
+
 // ---------------------------------------------------------------------------
 // exchange source of a ghost cell (PHI_COLL, serial branches)
 // ---------------------------------------------------------------------------
@@ -143,7 +174,8 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f) {
     // ETAT from the previous stage's face fluxes (dispersion.F:103-119)
     if (i <= g.Mloc - 2 && j <= g.Nloc - 2) {
         if constexpr (sizeof(T) == sizeof(double))
-            f.ETAT[id] = -(ro(f.P + (IDX(i + 1, j))) - ro(f.P + (id))) / DX - (ro(f.Q + (IDX(i, j + 1))) - ro(f.Q + (id))) / DY;
+            f.ETAT[id] = over(-(ro(f.P + (IDX(i + 1, j))) - ro(f.P + (id))), DX, (T)g.rdx) -
+                         over(ro(f.Q + (IDX(i, j + 1))) - ro(f.Q + (id)), DY, (T)g.rdy);
         else
             f.ETAT[id] = -(ro(f.P + (IDX(i + 1, j))) - ro(f.P + (id))) * GC(rdx) - (ro(f.Q + (IDX(i, j + 1))) - ro(f.Q + (id))) * GC(rdy);
     }
@@ -169,19 +201,20 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f) {
     const bool wall = (si == g.ib) || (si == g.ie) || (sj == g.jb) || (sj == g.je);
 #define LU(a, b) ro(f.U + (IDX(si + (a), sj + (b))))
 #define LV(a, b) ro(f.V + (IDX(si + (a), sj + (b))))
-#define LDU(a, b) (tmax(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LU(a, b))
-#define LDV(a, b) (tmax(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LV(a, b))
+#define LDU(a, b) (max_pos(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LU(a, b))
+#define LDV(a, b) (max_pos(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LV(a, b))
     // FP64: the reference's divisions; mixed: reciprocal constants
     constexpr bool EXACT = sizeof(T) == sizeof(double);
     const T rdx2 = (T)g.f_rdx2, rdy2 = (T)g.f_rdy2, rdxy4 = (T)g.f_rdxy4;
-#define DXX(F) (EXACT ? (((F(1, 0) - (T)2 * F(0, 0) + F(-1, 0)) / DX / DX) * m9) \
+#define QX(x) div_any((double)(x), g.DX, g.rdx)
+#define QY(x) div_any((double)(x), g.DY, g.rdy)
+#define DXX(F) (EXACT ? (T)(QX(QX(sub2(F(1, 0), F(0, 0)) + F(-1, 0))) * m9) \
                       : ((F(1, 0) - (T)2 * F(0, 0) + F(-1, 0)) * rdx2 * m9))
-#define DYY(F) (EXACT ? (((F(0, 1) - (T)2 * F(0, 0) + F(0, -1)) / DY / DY) * m9) \
+#define DYY(F) (EXACT ? (T)(QY(QY(sub2(F(0, 1), F(0, 0)) + F(0, -1))) * m9) \
                       : ((F(0, 1) - (T)2 * F(0, 0) + F(0, -1)) * rdy2 * m9))
 #define DXY(F)                                                                                      \
     (wall ? (T)0                                                                                    \
-          : (EXACT ? ((((F(1, 1) - F(1, -1)) / (T)2 / DY) - ((F(-1, 1) - F(-1, -1)) / (T)2 / DY)) / \
-                      (T)2 / DX) * m9                                                               \
+          : (EXACT ? (T)(QX((QY((F(1, 1) - F(1, -1)) / (T)2) - QY((F(-1, 1) - F(-1, -1)) / (T)2)) / (T)2) * m9) \
                    : (((F(1, 1) - F(1, -1)) - (F(-1, 1) - F(-1, -1))) * rdxy4 * m9)))
     const T Uxx = DXX(LU), Vyy = DYY(LV), Uxy = DXY(LU), Vxy = DXY(LV);
     const T DUxx = DXX(LDU), DVyy = DYY(LDV), DUxy = DXY(LDU), DVxy = DXY(LDV);
@@ -215,8 +248,8 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f) {
     if (exch || (g.show_breaking && !gx && !gy)) {
         const T dex = ro(f.Eta + (IDX(si + 1, sj))) - ro(f.Eta + (IDX(si - 1, sj)));
         const T dey = ro(f.Eta + (IDX(si, sj + 1))) - ro(f.Eta + (IDX(si, sj - 1)));
-        const T ex = EXACT ? dex / DX / (T)2 * m9 : dex * (T)g.f_hdx * m9;
-        const T ey = EXACT ? dey / DY / (T)2 * m9 : dey * (T)g.f_hdy * m9;
+        const T ex = EXACT ? (T)(QX(dex) / 2.0 * m9) : dex * (T)g.f_hdx * m9;
+        const T ey = EXACT ? (T)(QY(dey) / 2.0 * m9) : dey * (T)g.f_hdy * m9;
         if (!stale) {
             if (exch && g.periodic && gx && !gy) {
                 // the periodic copy (bc.F:735-740) runs before the x mirror:
@@ -240,17 +273,88 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f) {
 // CAL_DISPERSION, part 2 (dispersion.F:293-503): U4, V4 on every cell;
 // U1p, V1p and U1pp+U2+U3, V1pp+V2+V3 on the interior.
 // ---------------------------------------------------------------------------
+// In FP64 the pipe is the bound (81 % busy): constant divisors divide through
+// their reciprocals, the time derivatives are taken once per cell of a tile
+// and the constants come evaluated (701 x 937: 1412 -> 726 us; k_disp_a the
+// same way 438 -> 252, k_update 555 -> 372).
+// the combinations of Beta_1 and Beta_2 that k_disp_b multiplies by, evaluated
+// in double in the reference's order (the FP64 mode's; the host's operations
+// round as the device's)
+struct DispK {
+    double c1, c2, c3, c4, c5, c6, c7, c8, c9, c10, c11, c12, c13;
+};
+static DispK disp_k(const Grid &g) {
+    const double B1 = g.Beta_1, B2 = g.Beta_2;
+    // one operation to a statement: nothing to contract
+    auto mul = [](double a, double b) { volatile double r = a * b; return (double)r; };
+    DispK k;
+    k.c8 = mul(B1, B1);
+    k.c13 = mul(mul(0.5, B1), B1);
+    volatile double t = 1.0 / 3.0 - B1;
+    k.c1 = t + k.c13;
+    k.c2 = B1 - 0.5;
+    t = 1.0 / 6.0 - B1;
+    k.c3 = t + k.c8;
+    k.c4 = mul(mul(0.5, B1), B1) - 1.0 / 6.0;
+    const double m = 1.0 - B1;
+    k.c5 = mul(mul(0.5, m), m);
+    k.c6 = B1 - 1.0;
+    k.c7 = mul(B1, m);
+    k.c9 = mul(m, m);
+    k.c10 = k.c8 - 1.0;
+    k.c11 = mul(0.5, k.c10);
+    k.c12 = mul(B2, B2);
+    return k;
+}
+// shared memory of k_disp_b: the FP64 tile's four planes
+template <typename T> static size_t disp_b_smem(dim3 b) {
+    return sizeof(T) == sizeof(double) ? (size_t)4 * (b.x + 2) * (b.y + 2) * sizeof(double) : 0;
+}
+
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_disp_b(Grid g, Fields<T> f) {
+__global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_disp_b(Grid g, Fields<T> f, DispK dk) {
+    constexpr bool EXACT = sizeof(T) == sizeof(double);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
+    const T mdf = GC(min_depth_frc), DT = DTV;
+    extern __shared__ double dsm[];
+    // FP64: the time derivatives of the tile's cells and of the ring around
+    // it, and their products with the depth, once per cell
+    const int tw = blockDim.x + 2, tc = tw * (blockDim.y + 2);
+    const int tq = (threadIdx.x + 1) + (threadIdx.y + 1) * tw;
+    if constexpr (EXACT) {
+        if (g.has_g2) {
+            const double rdt = __drcp_rn((double)DT);
+            for (int q = threadIdx.x + threadIdx.y * blockDim.x; q < tc; q += blockDim.x * blockDim.y) {
+                const int a = (int)(blockIdx.x * blockDim.x) - 1 + q % tw, c = (int)(blockIdx.y * blockDim.y) - 1 + q / tw;
+                if (a < 0 || a >= g.Mloc || c < 0 || c >= g.Nloc) continue;
+                const size_t id = IDX(a, c);
+                const double dep = max_pos((double)f.Depth[id], (double)mdf);
+                const double ut = div_any((double)(f.U[id] - f.U0[id]), (double)DT, rdt);
+                const double vt = div_any((double)(f.V[id] - f.V0[id]), (double)DT, rdt);
+                dsm[q] = ut;
+                dsm[tc + q] = vt;
+                dsm[2 * tc + q] = dep * ut;
+                dsm[3 * tc + q] = dep * vt;
+            }
+            __syncthreads();
+        }
+    }
     if (i >= g.Mloc || j >= g.Nloc) return;
     const size_t id = IDX(i, j);
-    const T DX = GC(DX), DY = GC(DY), mdf = GC(min_depth_frc);
+    const T DX = GC(DX), DY = GC(DY);
     const T B1 = GC(Beta_1), B2 = GC(Beta_2), g2 = GC(gamma2), b2 = GC(b2);
     const T one = (T)1, two = (T)2, half = (T)0.5;
     const T D = f.Depth[id], reta = f.Eta[id], m9 = m2r<T>(f.MASK9[id]);
-    constexpr bool EXACT = sizeof(T) == sizeof(double);
+    // the combinations of Beta_1 and Beta_2: FP64 reads them (each would cost
+    // every thread FP64 operations), the mixed path computes them
+#define DK(name, expr) (EXACT ? (T)dk.name : (T)(expr))
+    const T c1 = DK(c1, one / (T)3 - B1 + half * B1 * B1), c2 = DK(c2, B1 - one / two);
+    const T c3 = DK(c3, one / (T)6 - B1 + B1 * B1), c4 = DK(c4, one / two * B1 * B1 - one / (T)6);
+    const T c5 = DK(c5, half * (one - B1) * (one - B1)), c6 = DK(c6, B1 - one), c7 = DK(c7, B1 * (one - B1));
+    const T c8 = DK(c8, B1 * B1), c9 = DK(c9, (one - B1) * (one - B1)), c10 = DK(c10, B1 * B1 - one);
+    const T c11 = DK(c11, half * (B1 * B1 - one)), c12 = DK(c12, B2 * B2), c13 = DK(c13, half * B1 * B1);
+#undef DK
     T a, b, c, e;
     if constexpr (EXACT) {
         a = f.Uxx[id] + f.Vxy[id];
@@ -263,12 +367,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
         c = f.C[id];
         e = f.E[id];
     }
-    T u4 = (one / (T)3 - B1 + half * B1 * B1) * D * D * a + (B1 - one / two) * D * b;
-    T v4 = (one / (T)3 - B1 + half * B1 * B1) * D * D * c + (B1 - one / two) * D * e;
+    T u4 = c1 * D * D * a + c2 * D * b;
+    T v4 = c1 * D * D * c + c2 * D * e;
     if (g.has_g2) {
-        const T ken1 = (one / (T)6 - B1 + B1 * B1) * D * reta * B2 +
-                       (one / two * B1 * B1 - one / (T)6) * reta * reta * B2 * B2;
-        const T ken2 = (B1 - one / two) * reta * B2;
+        const T ken1 = c3 * D * reta * B2 +
+                       c4 * reta * reta * B2 * B2;
+        const T ken2 = c2 * reta * B2;
         u4 = u4 + g2 * m9 * (ken1 * a + ken2 * b);
         v4 = v4 + g2 * m9 * (ken1 * c + ken2 * e);
     }
@@ -276,11 +380,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
     f.V4[id] = v4;
     if (i < g.ib || i > g.ie || j < g.jb || j > g.je) return;
 
-    f.U1p[id] = half * (one - B1) * (one - B1) * D * D * a + (B1 - one) * D * b;
-    f.V1p[id] = half * (one - B1) * (one - B1) * D * D * c + (B1 - one) * D * e;
+    f.U1p[id] = c5 * D * D * a + c6 * D * b;
+    f.V1p[id] = c5 * D * D * c + c6 * D * e;
     if (!g.has_g2) return;
 
-    const T DT = DTV;
     const T rDT = (T)f.fsc[FS_RDT];
     const T hdx = (T)g.f_hdx, hdy = (T)g.f_hdy;
     const T rdx2 = (T)g.f_rdx2, rdy2 = (T)g.f_rdy2, rdxy4 = (T)g.f_rdxy4;
@@ -291,15 +394,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
     if constexpr (EXACT) {
         // (F1(I+1)+F2(I+1)-F1(I-1)-F2(I-1))/2/DX, evaluated left to right
 #define DIFF(F1, F2, a1, b1, a2, b2, H) \
-    ((AT(F1, a1, b1) + AT(F2, a1, b1) - AT(F1, a2, b2) - AT(F2, a2, b2)) / two / H)
-        UxxVxy_x = DIFF(Uxx, Vxy, 1, 0, -1, 0, DX);
-        UxxVxy_y = DIFF(Uxx, Vxy, 0, 1, 0, -1, DY);
-        UxyVyy_x = DIFF(Uxy, Vyy, 1, 0, -1, 0, DX);
-        UxyVyy_y = DIFF(Uxy, Vyy, 0, 1, 0, -1, DY);
-        HUxxHVxy_x = DIFF(DUxx, DVxy, 1, 0, -1, 0, DX);
-        HUxxHVxy_y = DIFF(DUxx, DVxy, 0, 1, 0, -1, DY);
-        HUxyHVyy_x = DIFF(DUxy, DVyy, 1, 0, -1, 0, DX);
-        HUxyHVyy_y = DIFF(DUxy, DVyy, 0, 1, 0, -1, DY);
+    H((AT(F1, a1, b1) + AT(F2, a1, b1) - AT(F1, a2, b2) - AT(F2, a2, b2)) / two)
+        UxxVxy_x = DIFF(Uxx, Vxy, 1, 0, -1, 0, QX);
+        UxxVxy_y = DIFF(Uxx, Vxy, 0, 1, 0, -1, QY);
+        UxyVyy_x = DIFF(Uxy, Vyy, 1, 0, -1, 0, QX);
+        UxyVyy_y = DIFF(Uxy, Vyy, 0, 1, 0, -1, QY);
+        HUxxHVxy_x = DIFF(DUxx, DVxy, 1, 0, -1, 0, QX);
+        HUxxHVxy_y = DIFF(DUxx, DVxy, 0, 1, 0, -1, QY);
+        HUxyHVyy_x = DIFF(DUxy, DVyy, 1, 0, -1, 0, QX);
+        HUxyHVyy_y = DIFF(DUxy, DVyy, 0, 1, 0, -1, QY);
 #undef DIFF
     } else {
         const T hx = (T)g.f_hdx, hy = (T)g.f_hdy;
@@ -313,12 +416,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
         HUxyHVyy_y = (AT(E, 0, 1) - AT(E, 0, -1)) * hy;
     }
     const T rh = D;
-    const T rhx = EXACT ? (AT(Depth, 1, 0) - AT(Depth, -1, 0)) / two / DX : (AT(Depth, 1, 0) - AT(Depth, -1, 0)) * hdx;
-    const T rhy = EXACT ? (AT(Depth, 0, 1) - AT(Depth, 0, -1)) / two / DY : (AT(Depth, 0, 1) - AT(Depth, 0, -1)) * hdy;
+    const T rhx = EXACT ? (T)QX((AT(Depth, 1, 0) - AT(Depth, -1, 0)) / two) : (AT(Depth, 1, 0) - AT(Depth, -1, 0)) * hdx;
+    const T rhy = EXACT ? (T)QY((AT(Depth, 0, 1) - AT(Depth, 0, -1)) / two) : (AT(Depth, 0, 1) - AT(Depth, 0, -1)) * hdy;
     const T ETAx = f.ETAx[id], ETAy = f.ETAy[id], ETAT = f.ETAT[id];
     // first derivatives of U, V, DU, DV (derivatives.F:123-162)
-#define FD1X(F) (EXACT ? ((F(1, 0) - F(-1, 0)) / DX / two) * m9 : ((F(1, 0) - F(-1, 0)) * hdx) * m9)
-#define FD1Y(F) (EXACT ? ((F(0, 1) - F(0, -1)) / DY / two) * m9 : ((F(0, 1) - F(0, -1)) * hdy) * m9)
+#define FD1X(F) (EXACT ? (T)((QX(F(1, 0) - F(-1, 0)) / 2.0) * m9) : ((F(1, 0) - F(-1, 0)) * hdx) * m9)
+#define FD1Y(F) (EXACT ? (T)((QY(F(0, 1) - F(0, -1)) / 2.0) * m9) : ((F(0, 1) - F(0, -1)) * hdy) * m9)
 #define LU_(a_, b_) AT(U, a_, b_)
 #define LV_(a_, b_) AT(V, a_, b_)
     const T Ux = FD1X(LU_);
@@ -327,25 +430,26 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
     const T Vy = FD1Y(LV_);
 #undef LU_
 #undef LV_
-#define DUP(a_, b_) (tmax(AT(Depth, a_, b_), mdf) * AT(U, a_, b_))
-#define DVP(a_, b_) (tmax(AT(Depth, a_, b_), mdf) * AT(V, a_, b_))
+#define DUP(a_, b_) (max_pos(AT(Depth, a_, b_), mdf) * AT(U, a_, b_))
+#define DVP(a_, b_) (max_pos(AT(Depth, a_, b_), mdf) * AT(V, a_, b_))
     const T DUx = FD1X(DUP);
     const T DVy = FD1Y(DVP);
     // time derivatives Ut=(U-U0)/DT (dispersion.F:133-141) and their
     // derivatives; the cross derivatives are zero on the wall rows
-#define UT(a_, b_) (EXACT ? ((AT(U, a_, b_) - AT(U0, a_, b_)) / DT) : ((AT(U, a_, b_) - AT(U0, a_, b_)) * rDT))
-#define VT(a_, b_) (EXACT ? ((AT(V, a_, b_) - AT(V0, a_, b_)) / DT) : ((AT(V, a_, b_) - AT(V0, a_, b_)) * rDT))
-#define DUT(a_, b_) (tmax(AT(Depth, a_, b_), mdf) * UT(a_, b_))
-#define DVT(a_, b_) (tmax(AT(Depth, a_, b_), mdf) * VT(a_, b_))
+#define TSM(k, a_, b_) (T)dsm[(k) * tc + tq + (a_) + (b_) * tw]
+#define UT(a_, b_) (EXACT ? TSM(0, a_, b_) : ((AT(U, a_, b_) - AT(U0, a_, b_)) * rDT))
+#define VT(a_, b_) (EXACT ? TSM(1, a_, b_) : ((AT(V, a_, b_) - AT(V0, a_, b_)) * rDT))
+#define DUT(a_, b_) (EXACT ? TSM(2, a_, b_) : (tmax(AT(Depth, a_, b_), mdf) * UT(a_, b_)))
+#define DVT(a_, b_) (EXACT ? TSM(3, a_, b_) : (tmax(AT(Depth, a_, b_), mdf) * VT(a_, b_)))
 #define D1X(F) FD1X(F)
 #define D1Y(F) FD1Y(F)
-#define D2X(F) (EXACT ? (((F(1, 0) - two * F(0, 0) + F(-1, 0)) / DX / DX) * m9) \
+#define D2X(F) (EXACT ? (T)(QX(QX(sub2(F(1, 0), F(0, 0)) + F(-1, 0))) * m9) \
                       : ((F(1, 0) - two * F(0, 0) + F(-1, 0)) * rdx2 * m9))
-#define D2Y(F) (EXACT ? (((F(0, 1) - two * F(0, 0) + F(0, -1)) / DY / DY) * m9) \
+#define D2Y(F) (EXACT ? (T)(QY(QY(sub2(F(0, 1), F(0, 0)) + F(0, -1))) * m9) \
                       : ((F(0, 1) - two * F(0, 0) + F(0, -1)) * rdy2 * m9))
 #define D2XY(F)                                                                                          \
     (wall ? (T)0                                                                                         \
-          : (EXACT ? ((((F(1, 1) - F(1, -1)) / two / DY) - ((F(-1, 1) - F(-1, -1)) / two / DY)) / two / DX) * m9 \
+          : (EXACT ? (T)(QX((QY((F(1, 1) - F(1, -1)) / two) - QY((F(-1, 1) - F(-1, -1)) / two)) / two) * m9) \
                    : (((F(1, 1) - F(1, -1)) - (F(-1, 1) - F(-1, -1))) * rdxy4 * m9)))
     const T Utx = D1X(UT), Vty = D1Y(VT);
     const T Utxx = D2X(UT), Vtyy = D2Y(VT);
@@ -362,6 +466,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
 #undef VT
 #undef DUT
 #undef DVT
+#undef TSM
 #undef DUP
 #undef DVP
 #undef FD1X
@@ -372,41 +477,44 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 1) k_dis
              ETAx * B2 * (DUtx + DVty) - reta * B2 * (DUtxx + DVtxy);
     T V1pp = -reta * B2 * ETAy * B2 * (Utx + Vty) - half * reta * reta * B2 * B2 * (Utxy + Vtyy) -
              ETAy * B2 * (DUtx + DVty) - reta * B2 * (DUtxy + DVtyy);
-    T ken1 = B1 * (one - B1) * rh * ETAT * B2 - B1 * B1 * reta * B2 * ETAT * B2;
-    T ken2 = B1 * (one - B1) * rh * reta * B2 - half * B1 * B1 * reta * reta * B2 * B2;
+    T ken1 = c7 * rh * ETAT * B2 - c8 * reta * B2 * ETAT * B2;
+    T ken2 = c7 * rh * reta * B2 - c13 * reta * reta * B2 * B2;
     T ken3 = B1 * ETAT * B2;
     T ken4 = B1 * reta * B2;
     U1pp = U1pp - ken1 * UxxVxy - ken2 * (Utxx + Vtxy) + ken3 * HUxxHVxy + ken4 * (DUtxx + DVtxy);
     V1pp = V1pp - ken1 * UxyVyy - ken2 * (Utxy + Vtyy) + ken3 * HUxyHVyy + ken4 * (DUtxy + DVtyy);
 
-    ken1 = (B1 - one) * (rhx + ETAx) * B2;
-    ken2 = (B1 - one) * (rh + reta) * B2;
-    ken3 = ((one - B1) * (one - B1) * rh * rhx * B2 * B2 - B1 * (one - B1) * (rhx * reta * B2 + rh * ETAx * B2) +
-            (B1 * B1 - one) * reta * ETAx * B2 * B2);
-    ken4 = (half * (one - B1) * (one - B1) * rh * rh * B2 * B2 - B1 * (one - B1) * rh * reta * B2 +
-            half * (B1 * B1 - one) * reta * reta * B2 * B2);
-    const T ken5 = ((one - B1) * (one - B1) * rh * rhy * B2 * B2 -
-                    B1 * (one - B1) * (rhy * reta * B2 + rh * ETAy * B2) + (B1 * B1 - one) * reta * ETAy * B2 * B2);
+    ken1 = c6 * (rhx + ETAx) * B2;
+    ken2 = c6 * (rh + reta) * B2;
+    ken3 = (c9 * rh * rhx * B2 * B2 - c7 * (rhx * reta * B2 + rh * ETAx * B2) +
+            c10 * reta * ETAx * B2 * B2);
+    ken4 = (c5 * rh * rh * B2 * B2 - c7 * rh * reta * B2 +
+            c11 * reta * reta * B2 * B2);
+    const T ken5 = (c9 * rh * rhy * B2 * B2 -
+                    c7 * (rhy * reta * B2 + rh * ETAy * B2) + c10 * reta * ETAy * B2 * B2);
     const T U2 = ken1 * (Uc * HUxxHVxy + Vc * HUxyHVyy) +
                  ken2 * (Ux * HUxxHVxy + Uc * HUxxHVxy_x + Vx * HUxyHVyy + Vc * HUxyHVyy_x) +
                  ken3 * (Uc * UxxVxy + Vc * UxyVyy) + ken4 * (Ux * UxxVxy + Uc * UxxVxy_x + Vx * UxyVyy + Vc * UxyVyy_x) +
-                 B2 * B2 * (DUx + DVy + reta * B2 * (Ux + Vy)) * (HUxxHVxy + ETAx * B2 * (Ux + Vy) + reta * B2 * UxxVxy);
-    ken1 = (B1 - one) * (rhy + ETAy) * B2;
+                 c12 * (DUx + DVy + reta * B2 * (Ux + Vy)) * (HUxxHVxy + ETAx * B2 * (Ux + Vy) + reta * B2 * UxxVxy);
+    ken1 = c6 * (rhy + ETAy) * B2;
     const T V2 = ken1 * (Uc * HUxxHVxy + Vc * HUxyHVyy) +
                  ken2 * (Uy * HUxxHVxy + Uc * HUxxHVxy_y + Vy * HUxyHVyy + Vc * HUxyHVyy_y) +
                  ken5 * (Uc * UxxVxy + Vc * UxyVyy) + ken4 * (Uy * UxxVxy + Uc * UxxVxy_y + Vy * UxyVyy + Vc * UxyVyy_y) +
-                 B2 * B2 * (DUx + DVy + reta * B2 * (Ux + Vy)) * (HUxyHVyy + ETAy * B2 * (Ux + Vy) + reta * B2 * UxyVyy);
+                 c12 * (DUx + DVy + reta * B2 * (Ux + Vy)) * (HUxyHVyy + ETAy * B2 * (Ux + Vy) + reta * B2 * UxyVyy);
     const T omega_0 = Vx - Uy;
     const T omega_1 = (b2 * rhx + B1 * ETAx) * B2 * (HUxyHVyy + (b2 * rh + B1 * reta) * B2 * UxyVyy) -
                       (b2 * rhy + B1 * ETAy) * B2 * (HUxxHVxy + (b2 * rh + B1 * reta) * B2 * UxxVxy);
-    ken1 = ((B1 - one / two) * (reta + rh) * B2);
-    ken2 = (one / (T)3 - B1 + half * B1 * B1) * rh * rh * B2 * B2 + (one / (T)6 - B1 + B1 * B1) * rh * reta * B2 +
-           (one / two * B1 * B1 - one / (T)6) * reta * reta * B2 * B2;
+    ken1 = (c2 * (reta + rh) * B2);
+    ken2 = c1 * rh * rh * B2 * B2 + c3 * rh * reta * B2 +
+           c4 * reta * reta * B2 * B2;
     const T U3 = -Vc * omega_1 - omega_0 * (ken1 * HUxyHVyy + ken2 * UxyVyy);
     const T V3 = Uc * omega_1 + omega_0 * (ken1 * HUxxHVxy + ken2 * UxxVxy);
     f.Udisp[id] = U1pp + U2 + U3;
     f.Vdisp[id] = V1pp + V2 + V3;
 }
+
+#undef QX
+#undef QY
 
 // ---------------------------------------------------------------------------
 // FLUXES (fluxes.F:52-117): 4th-order MUSCL-TVD (CONSTRUCT_HO_X/Y
@@ -694,8 +802,8 @@ __device__ __forceinline__ void face_flux(const Grid &g, const T *Lv, const T *R
 // a face is computed (without that, 189 us at 2048 x 2048: 20 warps to an SM
 // do not hide the loads).  The tiles that shared Din through shared memory
 // took 790 instructions per face; this takes 400.  2048 x 2048 float: 121 ->
-// 66 us (the bound: instruction issue); 701 x 937 double: 1493 -> 980 us, of
-// which the FP64 pipe is the bound.
+// 66 us (the bound: instruction issue); 701 x 937 double: 1493 -> 680 us (the
+// FP64 pipe).
 template <typename T>
 __global__ void __launch_bounds__(128) k_flux_y(Grid g, Fields<T> f, int strip) {
     const int i = blockIdx.x * 32 + threadIdx.x;
@@ -1101,8 +1209,8 @@ __device__ __forceinline__ void source_terms_b(const Grid &g, const Fields<T> &f
     const T DX = GC(DX), DY = GC(DY), mdf = GC(min_depth_frc);
     const T rdx = GC(rdx), rdy = GC(rdy);
     // x/DX: the reference's division in FP64, a reciprocal in the mixed path
-#define OX(x) (EXACT ? (x) / DX : (x) * rdx)
-#define OY(x) (EXACT ? (x) / DY : (x) * rdy)
+#define OX(x) over((x), DX, rdx)
+#define OY(x) over((x), DY, rdy)
     const T g1 = GC(gamma1), g2 = GC(gamma2);
     const size_t id = IDX(i, j);
     const size_t ie_ = IDX(i + 1, j), iw = IDX(i - 1, j), in_ = IDX(i, j + 1), is = IDX(i, j - 1);
@@ -1140,10 +1248,13 @@ __device__ __forceinline__ void source_terms_b(const Grid &g, const Fields<T> &f
         const T HUc = ro(f.HU + (id)), HVc = ro(f.HV + (id));
         T bx, by;
         if constexpr (EXACT) {
-            bx = (T)0.5 / DX * (nxp * (T)1 / DX * (ro(f.HU + (ie_)) - HUc) - nxm * (T)1 / DX * (HUc - ro(f.HU + (iw)))) +
-                 (T)0.5 / DY * (nyp * (T)1 / DY * (ro(f.HU + (in_)) - HUc) - nym * (T)1 / DY * (HUc - ro(f.HU + (is))));
-            by = (T)0.5 / DX * (nxp * (T)1 / DX * (ro(f.HV + (ie_)) - HVc) - nxm * (T)1 / DX * (HVc - ro(f.HV + (iw)))) +
-                 (T)0.5 / DY * (nyp * (T)1 / DY * (ro(f.HV + (in_)) - HVc) - nym * (T)1 / DY * (HVc - ro(f.HV + (is))));
+            // 0.5 / DX = half of RN(1/DX)
+            const T hx = (T)0.5 * rdx, hy = (T)0.5 * rdy;
+            const T qxp = OX(nxp), qxm = OX(nxm), qyp = OY(nyp), qym = OY(nym);
+            bx = hx * (qxp * (ro(f.HU + (ie_)) - HUc) - qxm * (HUc - ro(f.HU + (iw)))) +
+                 hy * (qyp * (ro(f.HU + (in_)) - HUc) - qym * (HUc - ro(f.HU + (is))));
+            by = hx * (qxp * (ro(f.HV + (ie_)) - HVc) - qxm * (HVc - ro(f.HV + (iw)))) +
+                 hy * (qyp * (ro(f.HV + (in_)) - HVc) - qym * (HVc - ro(f.HV + (is))));
         } else {
             const T cx = (T)g.f_cx, cy = (T)g.f_cy;
             bx = cx * (nxp * (ro(f.HU + (ie_)) - HUc) - nxm * (HUc - ro(f.HU + (iw)))) +
@@ -1224,7 +1335,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_upd
 
     const size_t ie_ = IDX(i + 1, j), in_ = IDX(i, j + 1);
     constexpr bool EXACT = sizeof(T) == sizeof(double);
-    const T cdx = EXACT ? (T)1 / DX : GC(rdx), cdy = EXACT ? (T)1 / DY : GC(rdy);
+    const T cdx = GC(rdx), cdy = GC(rdy);
     T R1 = -cdx * (ro(f.P + (ie_)) * (T)1 + ro(f.P + (id)) * (T)-1) - cdy * (ro(f.Q + (in_)) * (T)1 + ro(f.Q + (id)) * (T)-1);
     if (g.wavemaker != FW_WK_NONE) {
         const T xmk = i2r<T>(i - g.ib) * DX, ymk = i2r<T>(j - g.jb) * DY;
@@ -1269,8 +1380,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_upd
         const double Hm = tmax((double)H, mdf);
         // the cross derivatives CAL_DISPERSION left at the start of the stage
         const double Vxy = ro(f.Vxy + (id)), DVxy = ro(f.DVxy + (id)), Uxy = ro(f.Uxy + (id)), DUxy = ro(f.DUxy + (id));
-        f.rhs_x[id] = (double)ubar * mk / Hm + g1 * m9 * (-b1 / 2.0 * dep * dep * Vxy - b2 * dep * DVxy);
-        f.rhs_y[id] = (double)vbar * mk / Hm + g1 * m9 * (-b1 / 2.0 * dep * dep * Uxy - b2 * dep * DUxy);
+        const double rH = __drcp_rn(Hm);
+        f.rhs_x[id] = div_any((double)ubar * mk, Hm, rH) + g1 * m9 * (-b1 / 2.0 * dep * dep * Vxy - b2 * dep * DVxy);
+        f.rhs_y[id] = div_any((double)vbar * mk, Hm, rH) + g1 * m9 * (-b1 / 2.0 * dep * dep * Uxy - b2 * dep * DUxy);
     } else {
         // mixed: float arithmetic; the cross derivatives of the stage-start
         // U, V are recomputed here
@@ -1645,10 +1757,6 @@ __global__ void __launch_bounds__(256) k_thomas_rows(Grid g, Fields<T> f, LinePa
 // The planes are those that only the mixed mode's dispersion terms use.
 template <typename T, int DIR> __device__ __forceinline__ double *tf_c(const Fields<T> &f) { return (double *)(DIR == 0 ? f.A : f.C); }
 template <typename T, int DIR> __device__ __forceinline__ double *tf_y(const Fields<T> &f) { return (double *)(DIR == 0 ? f.B : f.E); }
-__device__ __forceinline__ bool div_rcp_ok(double b) {
-    const unsigned long long m = dmag(b);
-    return m >= ((1023ull - 300) << 52) && m <= ((1023ull + 300) << 52);
-}
 
 // a, c, 1 + c_end or 1 + a_beg (the scale of a periodic line's end rows, else
 // 1) and tmp2 of row k
@@ -4221,7 +4329,7 @@ template <typename T> void launch_dispersion(fw_ctx *c) {
     const Grid &g = c->g;
     k_disp_a<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_A)), c->blk(TK_DISP_A), 0, c->stream>>>(g, c->F<T>());
     note(c);
-    k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), 0, c->stream>>>(g, c->F<T>());
+    k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, c->F<T>(), disp_k(g));
     note(c);
 }
 
@@ -4245,6 +4353,25 @@ template <typename T> bool flux_tma_attrs() {
     return ok;
 }
 
+// faces of a y strip: the busiest SM works ceil(blocks / 152) blocks of four
+// strips, each with the work of about 2.3 faces before its first; in float
+// a face's latency is about that of 3.5 blocks' issue, so fewer blocks than
+// that on an SM gain nothing (701 x 937 FP64: 16 faces 1028 us with a third
+// of the SMs idle at the end, 19 faces 680 us)
+static int flux_strip(int nx, int faces, int most, bool fp64) {
+    int best = 4;
+    double least = 1e30;
+    for (int st = 4; st <= most; st++) {
+        const int blocks = nx * ((faces + 4 * st - 1) / (4 * st));
+        const double cost = (st + 2.3) * std::max(fp64 ? 1.0 : 3.5, (double)((blocks + 151) / 152));
+        if (cost < least) {
+            least = cost;
+            best = st;
+        }
+    }
+    return best;
+}
+
 template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
     const int fy = c->tune[TUNE_FLUX + DIR];
     if (c->tune[TUNE_FLUX_TMA + DIR] && c->fmaps_ok) {
@@ -4254,19 +4381,14 @@ template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
         note(c);
         return;
     }
-    // the tuned height is what a block of four warps covers along y; halved
-    // while the grid has fewer warps than the SMs take
+    // the tuned height sets the rows of an x block and bounds the strips of y
     const Grid &g = c->g;
     const dim3 b(32, 4);
     if (DIR == 0) {
         const int rows = std::max(1, fy / 8), nx = (g.ie + FLUX_XW) / FLUX_XW;
         k_flux_x<T><<<dim3(nx, (g.Nglob + 4 * rows - 1) / (4 * rows)), b, 0, c->stream>>>(g, c->F<T>(), rows);
     } else {
-        const int nx = (g.ie + 32) / 32;
-        int strip = fy;
-        // (FP64 fills its pipe with fewer warps, and a strip's start costs it more)
-        const int enough = 152 * (sizeof(T) == sizeof(double) ? 4 : 16);
-        while (strip > 4 && nx * ((g.Nglob + strip) / strip) < enough) strip /= 2;
+        const int nx = (g.ie + 32) / 32, strip = flux_strip(nx, g.Nglob + 1, sizeof(T) == sizeof(double) ? 2 * fy : fy, sizeof(T) == sizeof(double));
         k_flux_y<T><<<dim3(nx, (g.Nglob + 4 * strip) / (4 * strip)), b, 0, c->stream>>>(g, c->F<T>(), strip);
     }
     note(c);
@@ -4661,7 +4783,7 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     const dim3 gc = grid2(g.Mloc, g.Nloc, B2D);
     auto is = [&](const char *n) { return std::strcmp(name, n) == 0; };
     if (is("disp_a")) k_disp_a<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_A)), c->blk(TK_DISP_A), 0, c->stream>>>(g, f);
-    else if (is("disp_b")) k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), 0, c->stream>>>(g, f);
+    else if (is("disp_b")) k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, f, disp_k(g));
     else if (is("flux_x")) { launch_flux<T, 0>(c); return 0; }
     else if (is("flux_y")) { launch_flux<T, 1>(c); return 0; }
     else if (is("update")) k_update<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_UPDATE)), c->blk(TK_UPDATE), 0, c->stream>>>(g, f, (T)0.75, (T)0.25);
