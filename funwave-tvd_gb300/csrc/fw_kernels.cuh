@@ -3956,6 +3956,173 @@ __global__ void __launch_bounds__(256) k_begin(Grid g, Fields<T> f) {
     block_min_to_global(v, f.dtmin_bits);
 }
 
+// EXCHANGE in one pass, for grids of at least 3 x 3: the ghost fill (k_ghost),
+// then U,V,HU,HV *= MASK and SPONGE_DAMPING (k_maskmul), or at the begin of a
+// step k_eta0_ring, the fill and k_begin.  The thread of an interior cell
+// writes its own cell and the ghost cells that take their values from it (at
+// most three along each axis and their corner), so that no thread reads what
+// another writes.  With PERIODIC the ghost corners take the x ghost's value
+// from before its fill (bc.F:735-740), which the same thread reads first.
+// Blocks from row nby on fill P's and Q's ghosts (PHI_COLL_VARIABLE_LENGTH).
+// The fill as a launch of its own took 7-10 us (a chain of eight loads and
+// stores on a few thousand threads), four times a step: 20 steps of 250 x 500
+// 4181 -> 3879 us.
+template <typename T> struct ExCell {
+    T eta, u, v, hu, hv, age, nu;
+    uint8_t m;
+};
+template <typename T> __device__ __forceinline__ void ghost_pq(const Grid &g, const Fields<T> &f, int u) {
+    const int nPX = 6 * g.Nglob, nPY = 6 * (g.Mloc + 1);
+    int i, j;
+    if (u < nPX + nPY) {
+        const int ie1 = g.ie + 1;
+        if (u < nPX) {
+            const int col = u % 6;
+            i = col < 3 ? col : ie1 + 1 + (col - 3);
+            j = g.jb + u / 6;
+        } else {
+            u -= nPX;
+            const int row = u / (g.Mloc + 1);
+            i = u % (g.Mloc + 1);
+            j = row < 3 ? row : g.je + 1 + (row - 3);
+        }
+        const int si = i < g.ib ? 2 * g.ib - 1 - i : (i > ie1 ? 2 * ie1 + 1 - i : i);
+        f.P[IDX(i, j)] = f.P[IDX(si, mirror_y(g, j))];
+        return;
+    }
+    u -= nPX + nPY;
+    const int nQX = 6 * (g.Nglob + 1), nQY = 6 * g.Mloc;
+    if (u < nQX + nQY) {
+        const int je1 = g.je + 1;
+        if (u < nQX) {
+            const int col = u % 6;
+            i = col < 3 ? col : g.ie + 1 + (col - 3);
+            j = g.jb + u / 6;
+        } else {
+            u -= nQX;
+            const int row = u / g.Mloc;
+            i = u % g.Mloc;
+            j = row < 3 ? row : je1 + 1 + (row - 3);
+        }
+        const int sj = j < g.jb ? 2 * g.jb - 1 - j : (j > je1 ? 2 * je1 + 1 - j : j);
+        f.Q[IDX(i, j)] = f.Q[IDX(mirror_x(g, i), sj)];
+    }
+}
+// one cell as the fill leaves it, masked and damped; own: the interior cell
+// itself (its MASK, AGE and nu stay).  Returns the cell's CFL value (BEGIN).
+template <typename T, bool BEGIN>
+__device__ __forceinline__ T ex_put(const Grid &g, const Fields<T> &f, int id, const ExCell<T> &c, bool own, int sponge,
+                                    int with_age) {
+    const T m = m2r<T>(c.m);
+    T u = c.u * m, v = c.v * m, eta = c.eta, r = (T)1.0e30;
+    if (BEGIN) {
+        const T h = f.H[id], ub = f.Ubar[id], vb = f.Vbar[id], e0 = own ? c.eta : f.Eta[id];
+        f.Eta0[id] = e0;
+        f.Ubar0[id] = ub;
+        f.Vbar0[id] = vb;
+        f.U0[id] = u;
+        f.V0[id] = v;
+        r = dt_val(g, h, u, v);
+    } else if (sponge) {
+        const T s = f.SPONGE[id];
+        if (s != (T)1) {  // 1 outside the sponges: nothing to divide
+            if (c.m > 0) eta = eta / s;
+            u = u / s;
+            v = v / s;
+        }
+    }
+    f.U[id] = u;
+    f.V[id] = v;
+    f.HU[id] = c.hu * m;
+    f.HV[id] = c.hv * m;
+    if (!own || (!BEGIN && sponge)) f.Eta[id] = eta;
+    if (!own) {
+        f.MASK[id] = c.m;
+        if (with_age) {
+            f.AGE[id] = c.age;
+            f.nu[id] = c.nu;
+        }
+    }
+    return r;
+}
+template <typename T, bool BEGIN>
+__global__ void __launch_bounds__(256) k_exchange(Grid g, Fields<T> f, int sponge, int with_age, int nby) {
+    if ((int)blockIdx.y >= nby) {
+        const int nt = blockDim.x * blockDim.y;
+        ghost_pq(g, f, ((int)(blockIdx.y - nby) * (int)gridDim.x + (int)blockIdx.x) * nt + threadIdx.x + threadIdx.y * blockDim.x);
+        return;
+    }
+    const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = g.jb + blockIdx.y * blockDim.y + threadIdx.y;
+    T dt = (T)1.0e30;
+    if (i <= g.ie && j <= g.je) {
+        const int id = i + j * g.pitch;
+        ExCell<T> c;
+        c.m = f.MASK[id];
+        c.u = f.U[id];
+        c.v = f.V[id];
+        c.hu = f.HU[id];
+        c.hv = f.HV[id];
+        c.eta = f.Eta[id];
+        c.age = c.nu = (T)0;
+        const bool xl = i < g.ib + 3, xr = i > g.ie - 3, yl = j < g.jb + 3, yr = j > g.je - 3;
+        const bool edge = xl || xr || yl || yr;
+        if (edge && with_age) {
+            c.age = f.AGE[id];
+            c.nu = f.nu[id];
+        }
+        dt = ex_put<T, BEGIN>(g, f, id, c, true, sponge, with_age);
+        if (edge) {
+            // the ghost rows and columns that take their values from this cell
+            const int gx[2] = {xl ? 2 * g.ib - 1 - i : -1, xr ? 2 * g.ie + 1 - i : -1};
+            const int gy[2] = {yl ? (g.periodic ? j + g.je - 2 : 2 * g.jb - 1 - j) : -1,
+                               yr ? (g.periodic ? j - (g.je - 2) : 2 * g.je + 1 - j) : -1};
+            const T sy = g.periodic ? (T)1 : (T)-1;
+            auto signs = [&](T su, T sv) {
+                ExCell<T> d = c;
+                d.u = su * c.u;
+                d.hu = su * c.hu;
+                d.v = sv * c.v;
+                d.hv = sv * c.hv;
+                return d;
+            };
+#pragma unroll
+            for (int a = 0; a < 2; a++) {
+                if (gx[a] < 0) continue;
+                const int gid = gx[a] + j * g.pitch;
+                if (g.periodic && (yl || yr)) {
+                    ExCell<T> o;
+                    o.m = f.MASK[gid];
+                    o.u = f.U[gid];
+                    o.v = f.V[gid];
+                    o.hu = f.HU[gid];
+                    o.hv = f.HV[gid];
+                    o.eta = f.Eta[gid];
+                    o.age = with_age ? f.AGE[gid] : (T)0;
+                    o.nu = with_age ? f.nu[gid] : (T)0;
+#pragma unroll
+                    for (int b = 0; b < 2; b++)
+                        if (gy[b] >= 0)
+                            dt = tminr(dt, ex_put<T, BEGIN>(g, f, gx[a] + gy[b] * g.pitch, o, false, sponge, with_age));
+                }
+                dt = tminr(dt, ex_put<T, BEGIN>(g, f, gid, signs((T)-1, (T)1), false, sponge, with_age));
+                if (!g.periodic) {
+#pragma unroll
+                    for (int b = 0; b < 2; b++)
+                        if (gy[b] >= 0)
+                            dt = tminr(dt, ex_put<T, BEGIN>(g, f, gx[a] + gy[b] * g.pitch, signs((T)-1, sy), false, sponge,
+                                                           with_age));
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+                if (gy[b] >= 0)
+                    dt = tminr(dt, ex_put<T, BEGIN>(g, f, i + gy[b] * g.pitch, signs((T)1, sy), false, sponge, with_age));
+        }
+    }
+    if (BEGIN) block_min_to_global(dt, f.dtmin_bits);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) k_dt_only(Grid g, Fields<T> f) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -4281,8 +4448,25 @@ template <typename T> void launch_ghost(fw_ctx *c, bool full) {
     note(c);
 }
 
+// EXCHANGE in one launch; false for grids too small for it
+template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, bool sponge, dim3 b) {
+    const Grid &g = c->g;
+    if (g.Mglob < 3 || g.Nglob < 3) return false;
+    const bool age = g.visc_breaking != 0;
+    dim3 gr = grid2(g.Mglob, g.Nglob, b);
+    const int nby = (int)gr.y;
+    if (age) {  // blocks for P's and Q's ghosts
+        const int n = 6 * g.Nglob + 6 * (g.Mloc + 1) + 6 * (g.Nglob + 1) + 6 * g.Mloc, per = (int)(b.x * b.y * gr.x);
+        gr.y += (n + per - 1) / per;
+    }
+    k_exchange<T, BEGIN><<<gr, b, 0, c->stream>>>(g, c->F<T>(), sponge ? 1 : 0, age ? 1 : 0, nby);
+    note(c);
+    return true;
+}
+
 template <typename T> void launch_exchange(fw_ctx *c, bool with_sponge) {
     const Grid &g = c->g;
+    if (launch_exchange_one<T, false>(c, with_sponge, c->blk(TK_MASKMUL))) return;
     launch_ghost<T>(c, g.visc_breaking != 0);
     k_maskmul<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_MASKMUL)), c->blk(TK_MASKMUL), 0, c->stream>>>(g, c->F<T>(), with_sponge ? 1 : 0);
     note(c);
@@ -4316,6 +4500,10 @@ template <typename T> void launch_estimate_dt(fw_ctx *c) {
 
 template <typename T> void launch_begin_step(fw_ctx *c) {
     const Grid &g = c->g;
+    if (launch_exchange_one<T, true>(c, false, B2D)) {
+        launch_dt_final(c);
+        return;
+    }
     const int nring = 6 * g.Mloc + 6 * g.Nglob;
     k_eta0_ring<T><<<(nring + 255) / 256, 256, 0, c->stream>>>(g, c->F<T>());
     note(c);
@@ -4801,6 +4989,8 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     else if (is("mask")) k_mask<T><<<grid2(g.Mloc + 1, g.Nloc + 1, B2D), B2D, 0, c->stream>>>(g, f);
     else if (is("break_a")) k_break_a<T><<<gc, B2D, 0, c->stream>>>(g, f);
     else if (is("ghost")) { launch_ghost<T>(c, g.visc_breaking != 0); return 0; }
+    else if (is("maskmul") && launch_exchange_one<T, false>(c, g.direct_sponge, c->blk(TK_MASKMUL))) return 0;
+    else if (is("begin") && launch_exchange_one<T, true>(c, false, B2D)) return 0;
     else if (is("maskmul")) k_maskmul<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_MASKMUL)), c->blk(TK_MASKMUL), 0, c->stream>>>(g, f, g.direct_sponge);
     else if (is("begin")) k_begin<T><<<gc, B2D, 0, c->stream>>>(g, f);
     else return -1;
