@@ -3366,21 +3366,25 @@ __device__ __forceinline__ bool in_wk_zone(const Grid &g, int i, int j) {
     return fabs_(xmk - GC(xc_wk)) < GC(width_wk) && fabs_(ymk - GC(yc_wk)) < GC(ywidth_wk) / (T)2;
 }
 template <typename T>
-__device__ __forceinline__ T nu_value(const Grid &g, const Fields<T> &f, size_t id, const BrkLocal<T> &b, T age,
-                                      bool zone) {
+__device__ __forceinline__ T nu_of(const Grid &g, const BrkLocal<T> &b, T age, bool zone, T depth, T eta) {
     const T mdf = GC(min_depth_frc);
     if (zone) {
         if (b.et > tmin(b.tmp2, GC(wavemaker_cbrk) * b.tmp3)) {
-            const T cap1 = (T)1 * (tmax(ro(f.Depth + (id)), mdf) + ro(f.Eta + (id)));
+            const T cap1 = (T)1 * (tmax(depth, mdf) + eta);
             return cap1 * GC(wavemaker_cbrk) * b.tmp3 + GC(nu_bkg);
         }
         return (T)0 + GC(nu_bkg);
     }
     if (age > (T)0 && age < GC(T_brk) && b.et > b.tmp2) {
-        const T cap1 = (T)1 * (tmax(ro(f.Depth + (id)), mdf) + ro(f.Eta + (id)));
+        const T cap1 = (T)1 * (tmax(depth, mdf) + eta);
         return cap1 * b.tmp2 + GC(nu_bkg);
     }
     return (T)0 + GC(nu_bkg);
+}
+template <typename T>
+__device__ __forceinline__ T nu_value(const Grid &g, const Fields<T> &f, size_t id, const BrkLocal<T> &b, T age,
+                                      bool zone) {
+    return nu_of(g, b, age, zone, ro(f.Depth + (id)), ro(f.Eta + (id)));
 }
 
 // roller flux and undertow of a breaking cell (breaker.F:316-339):
@@ -3448,24 +3452,71 @@ __global__ void __launch_bounds__(256) k_break_a(Grid g, Fields<T> f) {
 // starts (U, V from the line solves; Eta, H from ESTIMATE_HUV; the MASK of
 // the start of the stage; AGE of the previous stage) and writes disjoint
 // arrays, so one thread can do all three.  Launched over (Mloc+1) x (Nloc+1).
+// A cell of the interior that is wet, with wet cells to its west and south
+// and viscosity breaking on (MASK9 = 1), needs one value of each input: they
+// are loaded together before the first use (the parts one after the other,
+// each loading behind the stores of the one before: 88 us at 2048 x 2048, now
+// 60, 2.6 times the floor of its 57 B per cell; the wait for those loads is
+// what is left).  The others take the parts one by one.
 template <typename T>
 __global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.Mloc || j > g.Nloc) return;
+    const bool in = i >= g.ib && i <= g.ie && j >= g.jb && j <= g.je;
+    if (in && g.visc_breaking && g.dispersion) {
+        const int id = i + j * g.pitch;
+        const int m = ro(f.MASK + id), mw = ro(f.MASK + (id - 1)), ms = ro(f.MASK + (id - g.pitch)),
+                  st = ro(f.MASK_STRUC + id), m9 = f.MASK9[id];
+        const T h = ro(f.H + id), u = f.U[id], v = f.V[id], age = ro(f.AGE + id), eta = ro(f.Eta + id), dep = ro(f.Depth + id);
+        BrkLocal<T> b;
+        b.et = ro(f.ETAT + id);
+        const T mdf = GC(min_depth_frc);
+        if (m >= 1 && mw >= 1 && ms >= 1) {
+            // GET_Eta_U_V_HU_HV tail (post_cell)
+            const T Hm = tmax(h, mdf);
+            f.HU[id] = Hm * u;
+            f.HV[id] = Hm * v;
+            const T Utotal = fsqrt(u * u + v * v);
+            const T Fr = fsqrt((T)GRAV * Hm);
+            // (a ratio of at most 1 does not exceed a cap of at least 1)
+            if (!(Utotal <= Fr && GC(froude_cap) >= (T)1) && Utotal / Fr > GC(froude_cap)) {
+                const T th = fatan2(v, u);
+                const T un = GC(froude_cap) * Fr * fcos(th);
+                const T vn = GC(froude_cap) * Fr * fsin(th);
+                f.U[id] = un;
+                f.V[id] = vn;
+                f.HU[id] = un * Hm;
+                f.HV[id] = vn * Hm;
+            }
+            // BREAKING (break_cell)
+            b.tmp3 = h == h ? Fr : h;  // sqrt(g max(mdf, h)), NaN where h is
+            b.tmp1 = GC(cbrk1) * b.tmp3;
+            b.tmp2 = GC(cbrk2) * b.tmp3;
+            const T DT = DTV;
+            T an = age;
+            bool cand = false;
+            if (b.et >= b.tmp1 && (age == (T)0 || age > GC(T_brk))) an = DT;
+            else if (age > (T)0) an = age + DT;
+            else if (b.et >= b.tmp2) cand = true;
+            f.AGEn[id] = an;
+            const bool zone = in_wk_zone<T>(g, i, j);
+            if (cand) {
+                const int slot = atomicAdd(f.ncand, 1);
+                f.cand[slot] = id;
+            }
+            if (zone || !cand) f.nu[id] = nu_of(g, b, an, zone, dep, eta);
+            if (g.track_roller && !zone && !cand && breaking_now(g, b, an)) roller_cell(g, f, id, b.et);
+            // UPDATE_MASK (mask_cell; wet cells beside it: no depth reset)
+            f.MASKn[id] = (uint8_t)(st == 1 && wet_test(eta, dep, f.DepthD + id) < 0 ? 0 : m);
+            if (m9 != 1) {
+                *f.m9_dirty = 1;  // the tridiagonal matrices change
+                f.MASK9[id] = 1;
+            }
+            return;
+        }
+    }
     if (i < g.Mloc && j < g.Nloc) {
-        // the breaking and mask parts' inputs, read after the post part's stores
-        const size_t id = IDX(i, j);
-        prefetch_l1(f.ETAT + id);
-        prefetch_l1(f.AGE + id);
-        prefetch_l1(f.Eta + id);
-        prefetch_l1(f.Depth + id);
-        prefetch_l1(f.MASK_STRUC + id);
-        // the post part's inputs, which it reads after a branch on MASK
-        prefetch_l1(f.MASK + id);
-        prefetch_l1(f.H + id);
-        prefetch_l1(f.U + id);
-        prefetch_l1(f.V + id);
         post_cell(g, f, i, j);
         break_cell(g, f, i, j);
     }
@@ -3963,7 +4014,8 @@ __global__ void __launch_bounds__(256) k_begin(Grid g, Fields<T> f) {
 // most three along each axis and their corner), so that no thread reads what
 // another writes.  With PERIODIC the ghost corners take the x ghost's value
 // from before its fill (bc.F:735-740), which the same thread reads first.
-// Blocks from row nby on fill P's and Q's ghosts (PHI_COLL_VARIABLE_LENGTH).
+// The rows of blocks before the last nby fill P's and Q's ghosts
+// (PHI_COLL_VARIABLE_LENGTH).
 // The fill as a launch of its own took 7-10 us (a chain of eight loads and
 // stores on a few thousand threads), four times a step: 20 steps of 250 x 500
 // 4181 -> 3879 us.
@@ -4013,23 +4065,29 @@ template <typename T> __device__ __forceinline__ void ghost_pq(const Grid &g, co
 template <typename T, bool BEGIN>
 __device__ __forceinline__ T ex_put(const Grid &g, const Fields<T> &f, int id, const ExCell<T> &c, bool own, int sponge,
                                     int with_age) {
+    // every load before the first use of a loaded value
+    T h = (T)0, ub = (T)0, vb = (T)0, e0 = c.eta, s = (T)1;
+    if (BEGIN) {
+        h = f.H[id];
+        ub = f.Ubar[id];
+        vb = f.Vbar[id];
+        if (!own) e0 = f.Eta[id];
+    } else if (sponge) {
+        s = f.SPONGE[id];
+    }
     const T m = m2r<T>(c.m);
     T u = c.u * m, v = c.v * m, eta = c.eta, r = (T)1.0e30;
     if (BEGIN) {
-        const T h = f.H[id], ub = f.Ubar[id], vb = f.Vbar[id], e0 = own ? c.eta : f.Eta[id];
         f.Eta0[id] = e0;
         f.Ubar0[id] = ub;
         f.Vbar0[id] = vb;
         f.U0[id] = u;
         f.V0[id] = v;
         r = dt_val(g, h, u, v);
-    } else if (sponge) {
-        const T s = f.SPONGE[id];
-        if (s != (T)1) {  // 1 outside the sponges: nothing to divide
-            if (c.m > 0) eta = eta / s;
-            u = u / s;
-            v = v / s;
-        }
+    } else if (s != (T)1) {  // 1 outside the sponges: nothing to divide
+        if (c.m > 0) eta = eta / s;
+        u = u / s;
+        v = v / s;
     }
     f.U[id] = u;
     f.V[id] = v;
@@ -4045,17 +4103,24 @@ __device__ __forceinline__ T ex_put(const Grid &g, const Fields<T> &f, int id, c
     }
     return r;
 }
+// (seven blocks to an SM, 36 registers: 41 -> 35 us at 2048 x 2048; the begin's
+// twelve streams want the registers: 62 us, 68 with seven)
 template <typename T, bool BEGIN>
-__global__ void __launch_bounds__(256) k_exchange(Grid g, Fields<T> f, int sponge, int with_age, int nby) {
-    if ((int)blockIdx.y >= nby) {
+__global__ void __launch_bounds__(256, !BEGIN && sizeof(T) == sizeof(float) ? 7 : 1) k_exchange(Grid g, Fields<T> f, int sponge, int with_age, int nby) {
+    const int npq = (int)gridDim.y - nby;
+    int by = (int)blockIdx.y - npq;
+    if (by < 0) {
         const int nt = blockDim.x * blockDim.y;
-        ghost_pq(g, f, ((int)(blockIdx.y - nby) * (int)gridDim.x + (int)blockIdx.x) * nt + threadIdx.x + threadIdx.y * blockDim.x);
+        ghost_pq(g, f, ((int)blockIdx.y * (int)gridDim.x + (int)blockIdx.x) * nt + threadIdx.x + threadIdx.y * blockDim.x);
         return;
     }
-    const int i = g.ib + blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = g.jb + blockIdx.y * blockDim.y + threadIdx.y;
+    // the rows with ghost images, which take longest, first: 0, last, 1, 2, ..
+    if (by > 0) by = by == 1 ? nby - 1 : by - 1;
+    // columns from 0: whole 128-byte lines to a warp
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = g.jb + by * blockDim.y + threadIdx.y;
     T dt = (T)1.0e30;
-    if (i <= g.ie && j <= g.je) {
+    if (i >= g.ib && i <= g.ie && j <= g.je) {
         const int id = i + j * g.pitch;
         ExCell<T> c;
         c.m = f.MASK[id];
@@ -4453,7 +4518,7 @@ template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, boo
     const Grid &g = c->g;
     if (g.Mglob < 3 || g.Nglob < 3) return false;
     const bool age = g.visc_breaking != 0;
-    dim3 gr = grid2(g.Mglob, g.Nglob, b);
+    dim3 gr = grid2(g.ie + 1, g.Nglob, b);
     const int nby = (int)gr.y;
     if (age) {  // blocks for P's and Q's ghosts
         const int n = 6 * g.Nglob + 6 * (g.Mloc + 1) + 6 * (g.Nglob + 1) + 6 * g.Mloc, per = (int)(b.x * b.y * gr.x);
