@@ -163,6 +163,21 @@ __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint3
         : "memory");
 }
 
+// The same by one lane of a warp that runs through it together: `me` is true
+// on that lane.  With the operands the same on every lane they stay in
+// uniform registers; issued from a branch that one lane takes, every operand
+// of every MMA is first moved there (about 100 cycles an MMA against 43: the
+// forward pass at 1 x 1024 x 1024 takes 156 us against 197).
+__device__ __forceinline__ void tc_mma_by(uint32_t me, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n.reg .pred p, q;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "setp.ne.b32 q, %5, 0;\n"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accum), "r"(me)
+        : "memory");
+}
+
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -177,10 +192,11 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// two floats as BF16 (round to nearest even) in one conversion
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    const uint32_t l = __bfloat16_as_ushort(__float2bfloat16(lo));
-    const uint32_t h = __bfloat16_as_ushort(__float2bfloat16(hi));
-    return l | (h << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
 __device__ __forceinline__ float lo_bf(uint32_t w) { return __uint_as_float(w << 16); }
@@ -206,7 +222,12 @@ __device__ __forceinline__ float hi_bf(uint32_t w) { return __uint_as_float(w & 
 // packed weight image (9 x CINC x N x 8 BF16).  EPI_RELU_BF16: y = BF16
 // relu(acc + bias), padded with 4 chunks; EPI_LINEAR_F32: y = FP32 acc +
 // bias, [pix][NOUTF] unpadded; EPI_MASK_BF16: y = BF16 acc where act > 0
-// else 0, padded with 4 chunks (act: padded, 4 chunks).  status: set to
+// else 0, padded with 4 chunks (act: padded, 4 chunks).
+// Bound by the MMA issue (18 per 128-pixel row of a 32 -> 32 layer, about 70
+// us of the 156 of a forward pass at 1 x 1024 x 1024) and by the bulk copies
+// (20 us a layer at the memory's rate).  Measured beside 3 stages of 4 rows,
+// the same pass: 4 stages 156 us, tiles of 2, 6 and 8 rows 165, 154 and 156,
+// the rows' MMAs interleaved 192.  status: set to
 // 1 (an input or accumulator wait expired) or 2 (an MMA wait expired); every
 // role then stops.
 __device__ __forceinline__ bool mbar_wait_or_abort(uint32_t bar, uint32_t parity, volatile uint32_t *flag,
@@ -249,7 +270,8 @@ __global__ void __launch_bounds__(320, 1) k_conv_tc(const bf16 *__restrict__ x, 
     auto acce_bar = [&](int a) { return bar + 8u * (2 * NSTAGE + 2 + a); };
     const uint32_t tptr = bar + 8u * (2 * NSTAGE + 4);
     volatile uint32_t *flag = reinterpret_cast<volatile uint32_t *>(smem + (tptr + 4u - xs0));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (the shuffle tells the compiler that the roles' branches are warp-uniform)
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const ActGeom gin{B, H, W, CINC}, gout{B, H, W, 4};
     const int tiles_x = (W + TPX - 1) / TPX, tiles_y = (H + TROWS - 1) / TROWS;
     const int ntiles = tiles_x * tiles_y * B;
@@ -288,6 +310,7 @@ __global__ void __launch_bounds__(320, 1) k_conv_tc(const bf16 *__restrict__ x, 
     tc_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tptr) : "memory");
+    tmem = __shfl_sync(0xffffffffu, tmem, 0);
 
     // the last tile issued to each input stage (producer lane) and the last
     // tile whose MMAs were committed (MMA lane): what a block that aborts
@@ -328,43 +351,44 @@ __global__ void __launch_bounds__(320, 1) k_conv_tc(const bf16 *__restrict__ x, 
                 if (k == st) last[k] = i;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16<TPX, N>();
-            for (int i = 0; i < ntl; i++) {
-                const int st = i % NSTAGE, a = i & 1;
-                if (!mbar_wait_or_abort(full_bar(st), (uint32_t)((i / NSTAGE) & 1), flag, wait_limit)) {
-                    if (*flag == 0u) fail(1);
-                    break;
-                }
-                if (i >= 2 && !mbar_wait_or_abort(acce_bar(a), (uint32_t)(((i >> 1) - 1) & 1), flag, wait_limit)) {
-                    if (*flag == 0u) fail(1);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t xs = xs0 + st * L::X_BYTES, acc = tmem + (uint32_t)(a * L::TMEM_COLS);
-                // the start address is the descriptors' low field (16-byte
-                // units), so each MMA's descriptors are these two plus a
-                // compile-time offset (all shared addresses stay below 256 KB,
-                // so the field does not overflow)
-                const uint64_t a_base = sdesc(xs, ROWB, 128), b_base = sdesc(ws, N * 16, 128);
+        constexpr uint32_t idesc = idesc_bf16<TPX, N>();
+        const uint32_t me = lane == 0;
+        for (int i = 0; i < ntl; i++) {
+            const int st = i % NSTAGE, a = i & 1;
+            // every lane waits; the warp goes on together or stops together
+            bool ok = mbar_wait_or_abort(full_bar(st), (uint32_t)((i / NSTAGE) & 1), flag, wait_limit);
+            if (ok && i >= 2) ok = mbar_wait_or_abort(acce_bar(a), (uint32_t)(((i >> 1) - 1) & 1), flag, wait_limit);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (me && *flag == 0u) fail(1);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t xs = xs0 + st * L::X_BYTES, acc = tmem + (uint32_t)(a * L::TMEM_COLS);
+            // the start address is the descriptors' low field (16-byte
+            // units), so each MMA's descriptors are these two plus a
+            // compile-time offset (all shared addresses stay below 256 KB,
+            // so the field does not overflow)
+            const uint64_t a_base = sdesc(xs, ROWB, 128), b_base = sdesc(ws, N * 16, 128);
 #pragma unroll 1
-                for (int r = 0; r < TROWS; r++) {
-                    const uint64_t a_row = a_base + (uint64_t)((r * CINC * ROWB) >> 4);
+            for (int r = 0; r < TROWS; r++) {
+                const uint64_t a_row = a_base + (uint64_t)((r * CINC * ROWB) >> 4);
 #pragma unroll
-                    for (int t = 0; t < 9; t++) {
-                        const int ky = t / 3, kx = t % 3;  // staged row and pixel offsets of the tap
+                for (int t = 0; t < 9; t++) {
+                    const int ky = t / 3, kx = t % 3;  // staged row and pixel offsets of the tap
 #pragma unroll
-                        for (int h = 0; h < CINC / 2; h++) {
-                            const uint32_t a_off = (uint32_t)(((ky * CINC + 2 * h) * ROWB + kx * 16) >> 4);
-                            const uint32_t b_off = (uint32_t)(((t * CINC + 2 * h) * N * 16) >> 4);
-                            tc_mma(acc + r * N, a_row + a_off, b_base + b_off, idesc, (t | h) != 0 ? 1u : 0u);
-                        }
+                    for (int h = 0; h < CINC / 2; h++) {
+                        const uint32_t a_off = (uint32_t)(((ky * CINC + 2 * h) * ROWB + kx * 16) >> 4);
+                        const uint32_t b_off = (uint32_t)(((t * CINC + 2 * h) * N * 16) >> 4);
+                        tc_mma_by(me, acc + r * N, a_row + a_off, b_base + b_off, idesc, (t | h) != 0 ? 1u : 0u);
                     }
                 }
+            }
+            if (me) {
                 tc_commit(empty_bar(st));
                 tc_commit(accf_bar(a));
-                committed = i;
             }
+            __syncwarp();
+            committed = i;
         }
     } else {
         const int q = warp & 3;  // TMEM lane quadrant of this warp
