@@ -57,13 +57,34 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return l | (h << 16);
 }
 
-__global__ void k_wgrad_reduce(const float *part, int nblocks, int E, float *gw, float *gb, int nw) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E) return;
+// The partials' sums, in the order of the CTAs.  A block takes 32 elements:
+// its 256 threads bring 256 partials of each to shared memory at a time, and
+// one warp adds them up, so that a sum waits for memory once per 256 partials
+// (a thread that read its 304 partials one after the other: 22 us).  ci_used,
+// ci_all: gradients of weights of input channels from ci_used on (padding of
+// ci_all) are zero.
+constexpr int WR_ROWS = 256;
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nblocks, int E, float *gw,
+                                                      float *gb, int nw, int ci_used, int ci_all) {
+    __shared__ float sh[WR_ROWS][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
     float s = 0.0f;
-    for (int b = 0; b < nblocks; b++) s += part[(size_t)b * E + e];
-    if (e < nw) gw[e] = s;
-    else gb[e - nw] = s;
+    for (int b0 = 0; b0 < nblocks; b0 += WR_ROWS) {
+        const int nb = min(WR_ROWS, nblocks - b0);
+        if (e < E) {
+#pragma unroll 8
+            for (int b = warp; b < nb; b += 8) sh[b][lane] = part[(size_t)(b0 + b) * E + e];
+        }
+        __syncthreads();
+        if (warp == 0 && e < E) {
+#pragma unroll 8
+            for (int b = 0; b < nb; b++) s += sh[b][lane];
+        }
+        __syncthreads();
+    }
+    if (warp != 0 || e >= E) return;
+    if (e >= nw) gb[e - nw] = s;
+    else gw[e] = (e / HID) % ci_all >= ci_used && ci_used < ci_all ? 0.0f : s;
 }
 
 // inputs: FP32 [npix][5] -> the padded BF16 input of 2 chunks (channels
@@ -120,26 +141,21 @@ __global__ void k_adam(float *w, const float *g, float *m, float *v, long long n
     w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-// zero the gradients of the padding input channels 5..7 of layer 0
-__global__ void k_zero_pad_grad(float *gw0) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 9 * CIN0 * HID) return;
-    const int ci = (e / HID) % CIN0;
-    if (ci >= NIN) gw0[e] = 0.0f;
-}
-
-// the network's input from a context's interior cells (x = I fastest)
+// the network's input from a context's interior cells (x = I fastest): the
+// padded BF16 input of 2 chunks that k_pack_input writes
 template <typename T>
-__global__ void k_corr_input(fw::Grid g, fw::Fields<T> f, float *in) {
+__global__ void k_corr_input(fw::Grid g, fw::Fields<T> f, bf16 *x) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mglob || j >= g.Nglob) return;
     const size_t id = (size_t)(i + g.ib) + (size_t)(j + g.jb) * g.pitch;
-    const long long p = (long long)i + (long long)j * g.Mglob;
-    in[p * NIN + 0] = (float)f.Eta[id];
-    in[p * NIN + 1] = (float)f.U[id];
-    in[p * NIN + 2] = (float)f.V[id];
-    in[p * NIN + 3] = (float)(f.Depth[id] / (T)FW_NET_DEPTH_SCALE);
-    in[p * NIN + 4] = f.MASK[id] ? 1.0f : 0.0f;
+    const float eta = (float)f.Eta[id], u = (float)f.U[id], v = (float)f.V[id];
+    const float dep = (float)(f.Depth[id] / (T)FW_NET_DEPTH_SCALE);
+    const float m = f.MASK[id] ? 1.0f : 0.0f;
+    const fwtc::ActGeom a{1, g.Nglob, g.Mglob, XC0 / 8};
+    uint4 *xq = reinterpret_cast<uint4 *>(x);
+    const long long o = fwtc::act_idx(a, 0, j, 0, i);
+    xq[o] = make_uint4(pack_bf16(eta, u), pack_bf16(v, dep), pack_bf16(m, 0.0f), 0u);
+    xq[o + g.Mglob + 2] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // The correction acts on the interior cells whose neighbourhood of
@@ -161,31 +177,57 @@ __device__ __forceinline__ bool wet_band(const fw::Grid &g, const fw::Fields<T> 
 // |correction|, [3] the largest amount by which a corrected total depth
 // would fall below MinDepth (bits of non-negative doubles); [4] the
 // decision of k_corr_apply (1 applied, 0 the plain step kept)
+// A block walks tiles of 32 x 8 cells and ends with one atomic per sum (one
+// per warp and tile: 136 us of same-address atomics at 1024 x 1024).
 template <typename T>
-__global__ void k_corr_sums(fw::Grid g, fw::Fields<T> f, const float *out, double *sums, float min_depth,
-                            int band) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    float se = 0.0f, sc = 0.0f, mx = 0.0f, dry = 0.0f;
-    if (i < g.Mglob && j < g.Nglob) {
-        const size_t id = (size_t)(i + g.ib) + (size_t)(j + g.jb) * g.pitch;
-        const long long p = (long long)i + (long long)j * g.Mglob;
-        if (wet_band(g, f, id, band)) {
-            const float inv = (float)(1.0 / FW_NET_OUT_SCALE);
-            se = out[p * NOUT] * inv;
-            sc = 1.0f;
-            mx = fmaxf(fabsf(out[p * NOUT]), fmaxf(fabsf(out[p * NOUT + 1]), fabsf(out[p * NOUT + 2]))) * inv;
-            dry = fmaxf(0.0f, min_depth - ((float)f.H[id] + se));
+__global__ void __launch_bounds__(256) k_corr_sums(fw::Grid g, fw::Fields<T> f, const float *out, double *sums,
+                                                   float min_depth, int band) {
+    const int tx = (g.Mglob + 31) / 32, ntiles = tx * ((g.Nglob + 7) / 8);
+    double de = 0.0;
+    int n = 0;
+    float mx = 0.0f, dry = 0.0f;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int i = (t % tx) * 32 + threadIdx.x, j = (t / tx) * 8 + threadIdx.y;
+        float se = 0.0f;
+        if (i < g.Mglob && j < g.Nglob) {
+            const size_t id = (size_t)(i + g.ib) + (size_t)(j + g.jb) * g.pitch;
+            const long long p = (long long)i + (long long)j * g.Mglob;
+            if (wet_band(g, f, id, band)) {
+                const float inv = (float)(1.0 / FW_NET_OUT_SCALE);
+                se = out[p * NOUT] * inv;
+                n++;
+                mx = fmaxf(mx, fmaxf(fabsf(out[p * NOUT]), fmaxf(fabsf(out[p * NOUT + 1]), fabsf(out[p * NOUT + 2]))) * inv);
+                dry = fmaxf(dry, fmaxf(0.0f, min_depth - ((float)f.H[id] + se)));
+            }
         }
+        // a warp's row in float, the rows in double
+        for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+        if (threadIdx.x == 0) de += (double)se;
     }
     for (int o = 16; o > 0; o >>= 1) {
-        se += __shfl_xor_sync(0xffffffffu, se, o);
-        sc += __shfl_xor_sync(0xffffffffu, sc, o);
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         dry = fmaxf(dry, __shfl_xor_sync(0xffffffffu, dry, o));
     }
-    if (((threadIdx.x + threadIdx.y * blockDim.x) & 31) == 0) {
-        atomicAdd(&sums[0], (double)se);
-        atomicAdd(&sums[1], (double)sc);
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    __shared__ double she[8];
+    __shared__ float shm[8], shd[8];
+    __shared__ int shn[8];
+    if (threadIdx.x == 0) {
+        she[threadIdx.y] = de;
+        shm[threadIdx.y] = mx;
+        shd[threadIdx.y] = dry;
+        shn[threadIdx.y] = n;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int k = 1; k < 8; k++) {
+            de += she[k];
+            mx = fmaxf(mx, shm[k]);
+            dry = fmaxf(dry, shd[k]);
+            n += shn[k];
+        }
+        atomicAdd(&sums[0], de);
+        atomicAdd(&sums[1], (double)n);
         atomicMax((unsigned long long *)&sums[2], (unsigned long long)__double_as_longlong((double)mx));
         atomicMax((unsigned long long *)&sums[3], (unsigned long long)__double_as_longlong((double)dry));
     }
@@ -207,26 +249,38 @@ __device__ __forceinline__ bool corr_ok(const double *sums, double max_corr) {
 template <typename T>
 __global__ void k_corr_apply(fw::Grid g, fw::Fields<T> f, const float *out, double *sums, double max_corr,
                              int band) {
-    const bool ok = corr_ok(sums, max_corr);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) sums[4] = ok ? 1.0 : 0.0;
-    if (!ok) return;
+    // the decision and the mean once per block (each thread's own division took
+    // most of the FP64 pipe's time: 68 us at 1024 x 1024)
+    __shared__ double mean_s;
+    __shared__ int ok_s;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        const bool ok = corr_ok(sums, max_corr);
+        mean_s = sums[1] > 0.0 ? sums[0] / sums[1] : 0.0;
+        ok_s = ok;
+        if (blockIdx.x == 0 && blockIdx.y == 0) sums[4] = ok ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    if (!ok_s) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mglob || j >= g.Nglob) return;
     const size_t id = (size_t)(i + g.ib) + (size_t)(j + g.jb) * g.pitch;
     if (!wet_band(g, f, id, band)) return;
     const long long p = (long long)i + (long long)j * g.Mglob;
     const double inv = 1.0 / FW_NET_OUT_SCALE;
-    const double mean = sums[1] > 0.0 ? sums[0] / sums[1] : 0.0;
+    const double mean = mean_s;
     const T de = (T)(out[p * NOUT] * inv - mean), du = (T)(out[p * NOUT + 1] * inv), dv = (T)(out[p * NOUT + 2] * inv);
-    f.Eta[id] += de;
-    f.H[id] += de;
-    const T h = f.H[id] > (T)0 ? f.H[id] : (T)0;
-    f.U[id] += du;
-    f.V[id] += dv;
-    f.HU[id] += h * du;
-    f.HV[id] += h * dv;
-    f.Ubar[id] += h * du;
-    f.Vbar[id] += h * dv;
+    // every load before the first store
+    const T eta = f.Eta[id], hh = f.H[id], u = f.U[id], v = f.V[id], hu = f.HU[id], hv = f.HV[id], ub = f.Ubar[id],
+            vb = f.Vbar[id];
+    f.Eta[id] = eta + de;
+    const T h1 = hh + de, h = h1 > (T)0 ? h1 : (T)0;
+    f.H[id] = h1;
+    f.U[id] = u + du;
+    f.V[id] = v + dv;
+    f.HU[id] = hu + h * du;
+    f.HV[id] = hv + h * dv;
+    f.Ubar[id] = ub + h * du;
+    f.Vbar[id] = vb + h * dv;
 }
 
 unsigned long long splitmix(unsigned long long &s) {
@@ -265,7 +319,6 @@ struct fw_net {
     bf16 *gbuf[2] = {nullptr, nullptr};  // masked gradients of hidden activations (4 chunks)
     float *part = nullptr;
     double *loss = nullptr;
-    float *corr_in = nullptr;   // fw_correct's input tensor
     // the checks of the last fw_correct that reported its decision: mean
     // raw eta correction, cells corrected, max |correction|, MinDepth
     // violation, decision
@@ -297,10 +350,9 @@ void free_ws(fw_net *n) {
         if (b) cudaFree(b);
         b = nullptr;
     }
-    for (void *p : {(void *)n->out, (void *)n->corr_in, (void *)n->gout})
+    for (void *p : {(void *)n->out, (void *)n->gout})
         if (p) cudaFree(p);
     n->out = nullptr;
-    n->corr_in = nullptr;
     n->gout = nullptr;
     n->npix_cap = 0;
     n->cap16 = n->cap32 = 0;
@@ -322,7 +374,6 @@ int ensure_ws(fw_net *n, int B, int H, int W, cudaStream_t s) {
         ok = ok && cudaMalloc(&n->out, (size_t)np * NOUT * sizeof(float)) == cudaSuccess;
         ok = ok && cudaMalloc(&n->gout, c16) == cudaSuccess;
         for (int k = 0; k < 2 && ok; k++) ok = cudaMalloc(&n->gbuf[k], c32) == cudaSuccess;
-        ok = ok && cudaMalloc(&n->corr_in, (size_t)np * NIN * sizeof(float)) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
             free_ws(n);
@@ -450,10 +501,10 @@ void pack_images(fw_net *n, cudaStream_t s) {
     n->img_ver = n->wver;
 }
 
-int forward(fw_net *n, const float *in, long long npix, int B, int H, int W, cudaStream_t s) {
+// the network from its packed input (act[0])
+int forward_packed(fw_net *n, int B, int H, int W, cudaStream_t s) {
     using namespace fwtc;
     pack_images(n, s);
-    k_pack_input<<<nblk(npix, 256), 256, 0, s>>>(in, n->act[0], B, H, W);
     const bf16 *im = n->img;
     int rc = conv_tc<2, 32, EPI_RELU_BF16, 0>(n->act[0], im + n->img_off[0], n->w + n->boff[0], nullptr,
                                               n->act[1], B, H, W, n->status, n->wait_limit, s);
@@ -464,6 +515,11 @@ int forward(fw_net *n, const float *in, long long npix, int B, int H, int W, cud
         rc = conv_tc<4, 16, EPI_LINEAR_F32, NOUT>(n->act[3], im + n->img_off[3], n->w + n->boff[3], nullptr,
                                                   n->out, B, H, W, n->status, n->wait_limit, s);
     return rc;
+}
+
+int forward(fw_net *n, const float *in, long long npix, int B, int H, int W, cudaStream_t s) {
+    k_pack_input<<<nblk(npix, 256), 256, 0, s>>>(in, n->act[0], B, H, W);
+    return forward_packed(n, B, H, W, s);
 }
 
 // weight and bias gradients of layer l on the tensor cores
@@ -481,8 +537,8 @@ int wgrad(fw_net *n, int l, const bf16 *x, const bf16 *dy, int B, int H, int W, 
     const unsigned grid = (unsigned)std::min<long long>(std::min<long long>(ntiles, (long long)nsm * Lw::PER_SM), cap);
     fwtc::k_wgrad_tc<XCC, CCU, DYCC, CIN, COUT><<<grid, 192, Lw::BYTES, s>>>(x, dy, n->part, H, W, B, n->status,
                                                                             n->wait_limit);
-    k_wgrad_reduce<<<nblk(E, 256), 256, 0, s>>>(n->part, (int)grid, E, n->g + n->woff[l], n->g + n->boff[l],
-                                                 9 * CIN * COUT);
+    k_wgrad_reduce<<<nblk(E, 32), 256, 0, s>>>(n->part, (int)grid, E, n->g + n->woff[l], n->g + n->boff[l],
+                                                9 * CIN * COUT, l == 0 ? NIN : CIN, CIN);
     return FW_OK;
 }
 
@@ -504,9 +560,7 @@ int backward(fw_net *n, int B, int H, int W, cudaStream_t s) {
         std::swap(ga, gb);
     }
     if (rc == FW_OK) rc = wgrad<CIN0, HID, XC0 / 8, HID / 8>(n, 0, n->act[0], ga, B, H, W, s);
-    if (rc != FW_OK) return rc;
-    k_zero_pad_grad<<<nblk(9 * CIN0 * HID, 256), 256, 0, s>>>(n->g + n->woff[0]);
-    return FW_OK;
+    return rc;
 }
 
 }  // namespace
@@ -517,15 +571,16 @@ namespace {
 template <typename T> int correct_enqueue(fw_ctx *c, fw_net *n, double max_corr) {
     const fw::Grid &g = c->g;
     fw::Fields<T> &f = c->F<T>();
-    const long long npix = (long long)g.Mglob * g.Nglob;
     cudaStream_t s = c->stream;
     const dim3 b(32, 8), gr((g.Mglob + 31) / 32, (g.Nglob + 7) / 8);
-    k_corr_input<T><<<gr, b, 0, s>>>(g, f, n->corr_in);
-    int rc = forward(n, n->corr_in, npix, 1, g.Nglob, g.Mglob, s);
+    k_corr_input<T><<<gr, b, 0, s>>>(g, f, n->act[0]);
+    int rc = forward_packed(n, 1, g.Nglob, g.Mglob, s);
     if (rc != FW_OK) return rc;
     double *sums = n->loss;  // 5 doubles of scratch after the loss slot
     if (cudaMemsetAsync(sums, 0, 6 * sizeof(double), s) != cudaSuccess) return FW_ERR_CUDA;
-    k_corr_sums<T><<<gr, b, 0, s>>>(g, f, n->out, sums + 1, (float)c->p.min_depth, n->shore_band);
+    const int nsm = sm_count();
+    if (!nsm) return FW_ERR_CUDA;
+    k_corr_sums<T><<<std::min((int)(gr.x * gr.y), 4 * nsm), b, 0, s>>>(g, f, n->out, sums + 1, (float)c->p.min_depth, n->shore_band);
     k_corr_apply<T><<<gr, b, 0, s>>>(g, f, n->out, sums + 1, max_corr, n->shore_band);
     return cudaGetLastError() == cudaSuccess ? FW_OK : FW_ERR_CUDA;
 }
