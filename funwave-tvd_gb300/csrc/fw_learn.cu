@@ -46,7 +46,7 @@ constexpr int HID = 32;
 constexpr int NOUT = 3;
 constexpr int LCIN[NL] = {CIN0, HID, HID, HID};
 constexpr int LCOUT[NL] = {HID, HID, HID, NOUT};
-constexpr long long WG_PART = 304LL * (9 * 32 * 32 + 32);  // floats of the weight-gradient partials
+constexpr long long WG_PART = 304LL * (9 * 32 * 32 + 32);  // floats of a layer's weight-gradient partials
 
 typedef __nv_bfloat16 bf16;
 
@@ -57,34 +57,43 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return l | (h << 16);
 }
 
-// The partials' sums, in the order of the CTAs.  A block takes 32 elements:
-// its 256 threads bring 256 partials of each to shared memory at a time, and
-// one warp adds them up, so that a sum waits for memory once per 256 partials
-// (a thread that read its 304 partials one after the other: 22 us).  ci_used,
-// ci_all: gradients of weights of input channels from ci_used on (padding of
-// ci_all) are zero.
+// The partials' sums of every layer in one launch (blockIdx.y = layer), in
+// the order of the CTAs.  A block takes 32 elements: its 256 threads bring 256
+// partials of each to shared memory at a time, and one warp adds them up, so
+// that a sum waits for memory once per 256 partials (a thread that read its
+// 304 partials one after the other: 22 us a layer; the four layers now 15).
+struct WgradSums {
+    const float *part;         // [nblocks][E]
+    float *gw, *gb;            // the weights' and the biases' gradients
+    int nblocks, E, nw;        // partials; elements; the weights among them
+    int cout, cin, ci_used;    // gradients of input channels from ci_used on (padding) are zero
+};
+struct WgradSumsAll {
+    WgradSums l[NL];
+};
 constexpr int WR_ROWS = 256;
-__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nblocks, int E, float *gw,
-                                                      float *gb, int nw, int ci_used, int ci_all) {
+__global__ void __launch_bounds__(256) k_wgrad_reduce(WgradSumsAll all) {
+    const WgradSums a = all.l[blockIdx.y];
     __shared__ float sh[WR_ROWS][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
+    if ((int)blockIdx.x * 32 >= a.E) return;
     float s = 0.0f;
-    for (int b0 = 0; b0 < nblocks; b0 += WR_ROWS) {
-        const int nb = min(WR_ROWS, nblocks - b0);
-        if (e < E) {
+    for (int b0 = 0; b0 < a.nblocks; b0 += WR_ROWS) {
+        const int nb = min(WR_ROWS, a.nblocks - b0);
+        if (e < a.E) {
 #pragma unroll 8
-            for (int b = warp; b < nb; b += 8) sh[b][lane] = part[(size_t)(b0 + b) * E + e];
+            for (int b = warp; b < nb; b += 8) sh[b][lane] = a.part[(size_t)(b0 + b) * a.E + e];
         }
         __syncthreads();
-        if (warp == 0 && e < E) {
+        if (warp == 0 && e < a.E) {
 #pragma unroll 8
             for (int b = 0; b < nb; b++) s += sh[b][lane];
         }
         __syncthreads();
     }
-    if (warp != 0 || e >= E) return;
-    if (e >= nw) gb[e - nw] = s;
-    else gw[e] = (e / HID) % ci_all >= ci_used && ci_used < ci_all ? 0.0f : s;
+    if (warp != 0 || e >= a.E) return;
+    if (e >= a.nw) a.gb[e - a.nw] = s;
+    else a.gw[e] = (e / a.cout) % a.cin < a.ci_used ? s : 0.0f;
 }
 
 // inputs: FP32 [npix][5] -> the padded BF16 input of 2 chunks (channels
@@ -105,7 +114,7 @@ __global__ void k_pack_input(const float *in, bf16 *x, int B, int H, int W) {
 
 // masked mean squared error and its gradient w.r.t. the output, stored as
 // a padded BF16 activation of 2 chunks (channels 3..15 zero)
-__global__ void k_loss(const float *out, const float *target, const float *wmask, int B, int H, int W, float inv_n,
+__global__ void __launch_bounds__(256) k_loss(const float *out, const float *target, const float *wmask, int B, int H, int W, float inv_n,
                        bf16 *dy, double *loss) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long npix = (long long)B * H * W;
@@ -126,7 +135,15 @@ __global__ void k_loss(const float *out, const float *target, const float *wmask
         dq[o + W + 2] = make_uint4(0u, 0u, 0u, 0u);
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)(l * inv_n));
+    // one atomic per block: every warp's goes to the same address
+    __shared__ double sh[8];
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = (double)(l * inv_n);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = sh[0];
+        for (int k = 1; k < 8; k++) t += sh[k];
+        atomicAdd(loss, t);
+    }
 }
 
 __global__ void k_adam(float *w, const float *g, float *m, float *v, long long n, float lr, float b1, float b2,
@@ -492,12 +509,14 @@ bool shape_ok(int B, int H, int W) {
 
 void pack_images(fw_net *n, cudaStream_t s) {
     if (n->img_ver == n->wver) return;
+    fwtc::WimgAll<NL + 3> a;
+    size_t most = 0;
     for (int i = 0; i < NL + 3; i++) {
         const int l = i < NL ? i : i - NL + 1;  // images 4..6 are the data gradients of layers 1..3
-        const int tot = (int)img_elems(i);
-        fwtc::k_pack_wimg<<<nblk(tot, 256), 256, 0, s>>>(n->w + n->woff[l], LCIN[l], LCOUT[l], IMG_CINC[i], IMG_N[i],
-                                                         i >= NL ? 1 : 0, n->img + n->img_off[i]);
+        a.im[i] = {n->w + n->woff[l], n->img + n->img_off[i], LCIN[l], LCOUT[l], IMG_CINC[i], IMG_N[i], i >= NL ? 1 : 0};
+        most = std::max(most, img_elems(i));
     }
+    fwtc::k_pack_wimg<NL + 3><<<dim3(nblk((long long)most, 256), NL + 3), 256, 0, s>>>(a);
     n->img_ver = n->wver;
 }
 
@@ -523,22 +542,24 @@ int forward(fw_net *n, const float *in, long long npix, int B, int H, int W, cud
 }
 
 // weight and bias gradients of layer l on the tensor cores
-// (fwtc::k_wgrad_tc): one partial per CTA, then k_wgrad_reduce adds them
+// (fwtc::k_wgrad_tc): one partial per CTA, in the layer's part of the partial
+// buffer; r: what k_wgrad_reduce is to add
 template <int CIN, int COUT, int XCC, int DYCC>
-int wgrad(fw_net *n, int l, const bf16 *x, const bf16 *dy, int B, int H, int W, cudaStream_t s) {
+int wgrad(fw_net *n, int l, const bf16 *x, const bf16 *dy, int B, int H, int W, WgradSums &r,
+          cudaStream_t s) {
     constexpr int CCU = (CIN + 7) / 8, E = 9 * CIN * COUT + COUT;
     using Lw = fwtc::WLayout<CCU, DYCC>;
     if (!wgrad_attr<CIN, COUT, XCC, DYCC>()) return FW_ERR_CUDA;
     const int nsm = sm_count();
     if (!nsm) return FW_ERR_CUDA;
     const long long ntiles = (long long)((W + fwtc::WKT - 1) / fwtc::WKT) * H * B;
-    // the partial buffer holds WG_PART floats
+    // a layer's part of the partial buffer holds WG_PART floats
+    float *part = n->part + (size_t)l * WG_PART;
     const long long cap = WG_PART / E;
     const unsigned grid = (unsigned)std::min<long long>(std::min<long long>(ntiles, (long long)nsm * Lw::PER_SM), cap);
-    fwtc::k_wgrad_tc<XCC, CCU, DYCC, CIN, COUT><<<grid, 192, Lw::BYTES, s>>>(x, dy, n->part, H, W, B, n->status,
+    fwtc::k_wgrad_tc<XCC, CCU, DYCC, CIN, COUT><<<grid, 192, Lw::BYTES, s>>>(x, dy, part, H, W, B, n->status,
                                                                             n->wait_limit);
-    k_wgrad_reduce<<<nblk(E, 32), 256, 0, s>>>(n->part, (int)grid, E, n->g + n->woff[l], n->g + n->boff[l],
-                                                9 * CIN * COUT, l == 0 ? NIN : CIN, CIN);
+    r = {part, n->g + n->woff[l], n->g + n->boff[l], (int)grid, E, 9 * CIN * COUT, COUT, CIN, l == 0 ? NIN : CIN};
     return FW_OK;
 }
 
@@ -547,20 +568,25 @@ int backward(fw_net *n, int B, int H, int W, cudaStream_t s) {
     using namespace fwtc;
     const bf16 *im = n->img;
     bf16 *ga = n->gbuf[0], *gb = n->gbuf[1];
-    int rc = wgrad<HID, NOUT, HID / 8, GC3 / 8>(n, 3, n->act[3], n->gout, B, H, W, s);
+    WgradSumsAll r;
+    int rc = wgrad<HID, NOUT, HID / 8, GC3 / 8>(n, 3, n->act[3], n->gout, B, H, W, r.l[3], s);
     // gradient of act[3] (the output of layer 2), masked by its ReLU
     if (rc == FW_OK)
         rc = conv_tc<2, 32, EPI_MASK_BF16, 0>(n->gout, im + n->img_off[NL + 2], nullptr, n->act[3], ga, B, H, W,
                                               n->status, n->wait_limit, s);
     for (int l = 2; l >= 1 && rc == FW_OK; l--) {
-        rc = wgrad<HID, HID, HID / 8, HID / 8>(n, l, n->act[l], ga, B, H, W, s);
+        rc = wgrad<HID, HID, HID / 8, HID / 8>(n, l, n->act[l], ga, B, H, W, r.l[l], s);
         if (rc == FW_OK)
             rc = conv_tc<4, 32, EPI_MASK_BF16, 0>(ga, im + n->img_off[NL + l - 1], nullptr, n->act[l], gb, B, H, W,
                                                   n->status, n->wait_limit, s);
         std::swap(ga, gb);
     }
-    if (rc == FW_OK) rc = wgrad<CIN0, HID, XC0 / 8, HID / 8>(n, 0, n->act[0], ga, B, H, W, s);
-    return rc;
+    if (rc == FW_OK) rc = wgrad<CIN0, HID, XC0 / 8, HID / 8>(n, 0, n->act[0], ga, B, H, W, r.l[0], s);
+    if (rc != FW_OK) return rc;
+    int most = 0;
+    for (const WgradSums &w : r.l) most = std::max(most, w.E);
+    k_wgrad_reduce<<<dim3(nblk(most, 32), NL), 256, 0, s>>>(r);
+    return FW_OK;
 }
 
 }  // namespace
@@ -649,7 +675,7 @@ int fw_net_create(unsigned long long seed, fw_net **out) {
     }
     bool ok = cudaMalloc(&n->w, off * sizeof(float)) == cudaSuccess && cudaMalloc(&n->g, off * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&n->m, off * sizeof(float)) == cudaSuccess && cudaMalloc(&n->v, off * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&n->part, (size_t)WG_PART * sizeof(float)) == cudaSuccess &&
+              cudaMalloc(&n->part, (size_t)NL * WG_PART * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&n->loss, 8 * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&n->status, sizeof(int)) == cudaSuccess;
     size_t ioff = 0;

@@ -154,17 +154,8 @@ template <int M, int N> __host__ __device__ constexpr uint32_t idesc_bf16() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accum)
-        : "memory");
-}
-
-// The same by one lane of a warp that runs through it together: `me` is true
-// on that lane.  With the operands the same on every lane they stay in
+// Issued by one lane of a warp that runs through it together: `me` is true on
+// that lane.  With the operands the same on every lane they stay in
 // uniform registers; issued from a branch that one lane takes, every operand
 // of every MMA is first moved there (about 100 cycles an MMA against 43: the
 // forward pass at 1 x 1024 x 1024 takes 156 us against 197).
@@ -497,20 +488,32 @@ __global__ void __launch_bounds__(320, 1) k_conv_tc(const bf16 *__restrict__ x, 
 // co, tap t reads w[t][ci][co].  Backward data gradient (dgrad != 0): the
 // convolution runs over dy, so K = co, n = ci, and tap t reads the layer's
 // tap 8 - t (the mirrored offset).  Channels beyond cin / cout are zero.
-static __global__ void k_pack_wimg(const float *__restrict__ w, int cin, int cout, int cinc, int n_img, int dgrad,
-                            bf16 *__restrict__ img) {
+// All images in one launch (blockIdx.y = image; seven launches of 3 us one by
+// one).
+struct Wimg {
+    const float *w;
+    bf16 *img;
+    int cin, cout, cinc, n_img, dgrad;
+};
+template <int NI> struct WimgAll {
+    Wimg im[NI];
+};
+template <int NI> __global__ void k_pack_wimg(WimgAll<NI> a) {
+    const Wimg &g = a.im[blockIdx.y];
+    const int cin = g.cin, cout = g.cout, cinc = g.cinc, n_img = g.n_img;
+    const float *__restrict__ w = g.w;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = 9 * cinc * n_img * 8;
     if (e >= total) return;
     const int j = e % 8, n = (e / 8) % n_img, c = (e / (8 * n_img)) % cinc, t = e / (8 * n_img * cinc);
     const int k = c * 8 + j;
     float v = 0.0f;
-    if (!dgrad) {
+    if (!g.dgrad) {
         if (k < cin && n < cout) v = w[((size_t)t * cin + k) * cout + n];
     } else {
         if (n < cin && k < cout) v = w[((size_t)(8 - t) * cin + n) * cout + k];
     }
-    img[e] = __float2bfloat16(v);
+    g.img[e] = __float2bfloat16(v);
 }
 
 // ---------------------------------------------------------------------------
@@ -582,7 +585,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
     const uint32_t done_bar = bar + 8u * (2 * WNSTAGE);
     const uint32_t tptr = bar + 8u * (2 * WNSTAGE + 1);
     volatile uint32_t *flag = reinterpret_cast<volatile uint32_t *>(smem + (tptr + 4u - xs0));
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const ActGeom gx{B, H, W, XCC}, gd{B, H, W, DYCC};
     const int tiles_x = (W + WKT - 1) / WKT;
     const int ntiles = tiles_x * H * B;
@@ -631,6 +634,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
     tc_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tptr) : "memory");
+    tmem = __shfl_sync(0xffffffffu, tmem, 0);
 
     int last[WNSTAGE];
 #pragma unroll
@@ -673,13 +677,12 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
     } else if (warp == 1) {
         // MN-major A and B (instruction descriptor bits 15 and 16)
         constexpr uint32_t idesc = idesc_bf16<128, N>() | (1u << 15) | (1u << 16);
+        const uint32_t me = lane == 0;
         bool ok = true;
         for (int i = 0; i < ntl; i++) {
             const int st = i % WNSTAGE;
-            int landed = 1;
-            if (lane == 0) landed = mbar_wait_or_abort(full_bar(st), (uint32_t)((i / WNSTAGE) & 1), flag, wait_limit);
-            landed = __shfl_sync(0xffffffffu, landed, 0);
-            if (!landed) {
+            // every lane waits; the warp goes on together or stops together
+            if (!__all_sync(0xffffffffu, mbar_wait_or_abort(full_bar(st), (uint32_t)((i / WNSTAGE) & 1), flag, wait_limit))) {
                 if (lane == 0 && *flag == 0u) fail(1);
                 ok = false;
                 break;
@@ -691,9 +694,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
             if (valid < WKT) {
                 // past the grid row: dy pixels valid.. and x pixels valid+2..
                 // (staged pixel s is grid pixel x0 - 1 + s; pixel W is the
-                // zero border) are zeroed, once every lane has seen the copies
-                // land (the phase is complete, so the first poll succeeds)
-                mbar_wait(full_bar(st), (uint32_t)((i / WNSTAGE) & 1), 64);
+                // zero border) are zeroed
                 const int nz = WKT - valid;
                 for (int e = lane; e < (L::NQ + DYCC) * nz; e += 32) {
                     const int qq = e / nz, r = e % nz;
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             __syncwarp();
-            if (lane == 0) {
+            {
                 tc_fence_after();
                 const uint32_t xs = xs0 + st * L::STAGE;
                 // no swizzle: the stride between core matrices along M / N in
@@ -714,9 +715,9 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
                 for (int ks = 0; ks < WKT / 16; ks++)
 #pragma unroll
                     for (int kx = 0; kx < 3; kx++)
-                        tc_mma(tmem + (uint32_t)(kx * N), a_base + (uint64_t)((kx * 16 + ks * 256) >> 4),
+                        tc_mma_by(me, tmem + (uint32_t)(kx * N), a_base + (uint64_t)((kx * 16 + ks * 256) >> 4),
                                b_base + (uint64_t)((ks * 256) >> 4), idesc, (i | ks) != 0 ? 1u : 0u);
-                tc_commit(empty_bar(st));
+                if (me) tc_commit(empty_bar(st));
             }
             committed = i;
             __syncwarp();
@@ -742,7 +743,10 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
         }
         st = __shfl_sync(0xffffffffu, st, 0);
         tc_fence_after();
-        const int row = q * 32 + lane;
+        // the input stages are free once the accumulators are final (or were
+        // never filled); each warp takes 32 x (N + 1) floats of them
+        static_assert(4 * 32 * (N + 1) * 4 <= WNSTAGE * L::STAGE, "the epilogue's rows fit the stages");
+        float *sh = reinterpret_cast<float *>(smem) + q * 32 * (N + 1);
 #pragma unroll 1
         for (int kx = 0; kx < 3 && st != 2; kx++) {
             uint32_t v[N];
@@ -755,16 +759,20 @@ __global__ void __launch_bounds__(192) k_wgrad_tc(const bf16 *__restrict__ x, co
 #pragma unroll
                 for (int c = 0; c < N; c++) v[c] = 0u;
             }
-            const int plane = row / 8, ch = row % 8;
-            if (plane < L::NQ) {
+            // the warp's 32 rows through shared memory, so that its stores are
+            // of consecutive floats (a lane storing its own row touched 32
+            // lines per store: 27 us the kernel at 8 x 128 x 128, now 16)
+            __syncwarp();
+#pragma unroll
+            for (int co = 0; co < COUT; co++) sh[lane * (N + 1) + co] = __uint_as_float(v[co]);
+            __syncwarp();
+#pragma unroll 4
+            for (int e = lane; e < 32 * COUT; e += 32) {
+                const int rr = e / COUT, co = e % COUT, prow = q * 32 + rr;
+                const int plane = prow / 8, ch = prow % 8;
                 const int t = (plane / CCU) * 3 + kx, ci = (plane % CCU) * 8 + ch;
-                if (ci < CIN) {
-#pragma unroll
-                    for (int co = 0; co < COUT; co++) pp[(t * CIN + ci) * COUT + co] = __uint_as_float(v[co]);
-                }
-            } else if (plane == L::NQ && kx == 0 && ch == 0) {
-#pragma unroll
-                for (int co = 0; co < COUT; co++) pp[9 * CIN * COUT + co] = __uint_as_float(v[co]);
+                if (plane < L::NQ && ci < CIN) pp[(t * CIN + ci) * COUT + co] = sh[rr * (N + 1) + co];
+                if (plane == L::NQ && kx == 0 && ch == 0) pp[9 * CIN * COUT + co] = sh[rr * (N + 1) + co];
             }
         }
     }
