@@ -25,6 +25,7 @@
 #include <cstdint>
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <type_traits>
 
 #include "fw_internal.h"
@@ -160,12 +161,55 @@ __device__ __forceinline__ int period_y(const Grid &g, int j) {
 }
 
 // ---------------------------------------------------------------------------
+// Lines ahead: a kernel whose threads each read one cell of many planes has
+// too few of those reads in flight (its registers bound the blocks on an SM)
+// to cover the memory's latency.  Its threads therefore also bring to the L2,
+// one line each, the lines that the block `dist` places later reads; that
+// block's loads then wait for the L2 only.
+// Mixed 2048 x 2048: k_update 146 -> 128 us, k_disp_a 74 -> 62,
+// k_post_mask_break 68 -> 62, k_exchange 35 -> 34 and at a step's begin 94 ->
+// 90.  The distance matters little between one and four blocks per SM (with
+// twice the resident blocks the gain is gone); k_disp_b and the fluxes, bound
+// by their issue, gain nothing.
+// ---------------------------------------------------------------------------
+struct Ahead {
+    const void *p[28];
+    int n, dist;  // planes; blocks ahead (0: none)
+};
+// from min_cells cells on
+template <typename T>
+static Ahead ahead_of(const Grid &g, long long min_cells, int dist, std::initializer_list<const T *> planes) {
+    Ahead a{};
+    for (const T *q : planes) a.p[a.n++] = q;
+    a.dist = sizeof(T) == sizeof(float) && (long long)g.Mloc * g.Nloc >= min_cells ? dist : 0;
+    return a;
+}
+// blocks of blockDim.x x blockDim.y cells from column 0 and row j0 on; by: the
+// block's row
+template <typename T>
+__device__ __forceinline__ void prefetch_ahead(const Grid &g, const Ahead &a, unsigned by, int j0) {
+    if constexpr (sizeof(T) == sizeof(float)) {
+        if (a.dist == 0) return;
+        const unsigned b = blockIdx.x + by * gridDim.x + a.dist;
+        const unsigned by2 = b / gridDim.x, bx2 = b - by2 * gridDim.x;
+        const unsigned nx = (blockDim.x + 31) / 32, lines = nx * blockDim.y;  // of a plane
+        for (unsigned t = threadIdx.x + threadIdx.y * blockDim.x; t < a.n * lines; t += blockDim.x * blockDim.y) {
+            const unsigned q = t / lines, r = t - q * lines, y = r / nx, x = r - y * nx;
+            const int i = (int)(bx2 * blockDim.x + x * 32), j = j0 + (int)(by2 * blockDim.y + y);
+            if (i < g.Mloc && j < g.Nloc)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T *>(a.p[q]) + IDX(i, j)));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // CAL_DISPERSION, part 1 (dispersion.F:62-289): masked derivatives at the
 // exchange source of every cell, combined into the four sums the rest of
 // the unit uses, plus ETAx/ETAy (exchanged) and ETAT.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f) {
+__global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f, Ahead ah) {
+    prefetch_ahead<T>(g, ah, blockIdx.y, 0);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mloc || j >= g.Nloc) return;
@@ -1302,7 +1346,8 @@ __global__ void __launch_bounds__(256) k_sources(Grid g, Fields<T> f) {
 // (etauv_solver.F:247) and BreakSourceX/Y.
 // ---------------------------------------------------------------------------
 template <typename T, bool RAD = false>
-__global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_update(Grid g, Fields<T> f, T al, T be) {
+__global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_update(Grid g, Fields<T> f, T al, T be, Ahead ah) {
+    prefetch_ahead<T>(g, ah, blockIdx.y, 0);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mloc || j >= g.Nloc) return;
@@ -3459,7 +3504,8 @@ __global__ void __launch_bounds__(256) k_break_a(Grid g, Fields<T> f) {
 // 60, 2.6 times the floor of its 57 B per cell; the wait for those loads is
 // what is left).  The others take the parts one by one.
 template <typename T>
-__global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f) {
+__global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f, Ahead ah) {
+    prefetch_ahead<T>(g, ah, blockIdx.y, 0);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.Mloc || j > g.Nloc) return;
@@ -4106,7 +4152,7 @@ __device__ __forceinline__ T ex_put(const Grid &g, const Fields<T> &f, int id, c
 // (seven blocks to an SM, 36 registers: 41 -> 35 us at 2048 x 2048; the begin's
 // twelve streams want the registers: 62 us, 68 with seven)
 template <typename T, bool BEGIN>
-__global__ void __launch_bounds__(256, !BEGIN && sizeof(T) == sizeof(float) ? 7 : 1) k_exchange(Grid g, Fields<T> f, int sponge, int with_age, int nby) {
+__global__ void __launch_bounds__(256, !BEGIN && sizeof(T) == sizeof(float) ? 7 : 1) k_exchange(Grid g, Fields<T> f, int sponge, int with_age, int nby, Ahead ah) {
     const int npq = (int)gridDim.y - nby;
     int by = (int)blockIdx.y - npq;
     if (by < 0) {
@@ -4115,6 +4161,7 @@ __global__ void __launch_bounds__(256, !BEGIN && sizeof(T) == sizeof(float) ? 7 
         return;
     }
     // the rows with ghost images, which take longest, first: 0, last, 1, 2, ..
+    if (by >= 2) prefetch_ahead<T>(g, ah, by - 1, g.jb);
     if (by > 0) by = by == 1 ? nby - 1 : by - 1;
     // columns from 0: whole 128-byte lines to a warp
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -4513,6 +4560,38 @@ template <typename T> void launch_ghost(fw_ctx *c, bool full) {
     note(c);
 }
 
+// Grids from which on a kernel brings lines ahead: where its inputs no longer
+// come from the L2 anyway.  k_update, of 28 planes: 1024 x 1024 51.5 us with
+// and 51.3 without, 1000 x 1500 60.7 and 64.3.  k_disp_a and
+// k_post_mask_break: 1000 x 1500 24.7 and 24.5, 22.7 and 20.6; 1448 x 1448
+// 36.9 and 39.3, 35.0 and 35.1.  k_exchange: 1448 x 1448 14.5 and 12.4; 2048 x
+// 1500 20.7 and 20.5; 2048 x 2048 34.2 and 35.0.
+constexpr long long AHEAD_UPDATE = 1LL << 20, AHEAD_A_PMB = 2LL << 20, AHEAD_EXCHANGE = 3LL << 20;
+template <typename T> static void launch_disp_a(fw_ctx *c) {
+    const Grid &g = c->g;
+    const Fields<T> &f = c->F<T>();
+    const dim3 b = c->blk(TK_DISP_A);
+    k_disp_a<T><<<grid2(g.Mloc, g.Nloc, b), b, 0, c->stream>>>(
+        g, f, ahead_of<T>(g, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.Depth, f.Eta, f.P, f.Q}));
+}
+template <typename T, bool RAD> static void launch_update(fw_ctx *c, T al, T be) {
+    const Grid &g = c->g;
+    const Fields<T> &f = c->F<T>();
+    const dim3 b = c->blk(TK_UPDATE);
+    k_update<T, RAD><<<grid2(g.Mloc, g.Nloc, b), b, 0, c->stream>>>(
+        g, f, al, be,
+        ahead_of<T>(g, AHEAD_UPDATE, 2 * 152, {f.Eta0, f.Ubar0, f.Vbar0, f.Eta, f.Ubar, f.Vbar, f.P, f.Q, f.Fx, f.Fy, f.Gx, f.Gy,
+                                              f.Depth, f.H, f.U, f.V, f.U4, f.V4, f.Depthx, f.Depthy, f.Udisp, f.Vdisp, f.U1p,
+                                              f.V1p, f.Cd, f.HU, f.HV, f.nu}));
+}
+template <typename T> static void launch_pmb(fw_ctx *c) {
+    const Grid &g = c->g;
+    const Fields<T> &f = c->F<T>();
+    const dim3 b = c->blk(TK_PMB);
+    k_post_mask_break<T><<<grid2(g.Mloc + 1, g.Nloc + 1, b), b, 0, c->stream>>>(
+        g, f, ahead_of<T>(g, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.H, f.AGE, f.Eta, f.Depth, f.ETAT}));
+}
+
 // EXCHANGE in one launch; false for grids too small for it
 template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, bool sponge, dim3 b) {
     const Grid &g = c->g;
@@ -4524,7 +4603,10 @@ template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, boo
         const int n = 6 * g.Nglob + 6 * (g.Mloc + 1) + 6 * (g.Nglob + 1) + 6 * g.Mloc, per = (int)(b.x * b.y * gr.x);
         gr.y += (n + per - 1) / per;
     }
-    k_exchange<T, BEGIN><<<gr, b, 0, c->stream>>>(g, c->F<T>(), sponge ? 1 : 0, age ? 1 : 0, nby);
+    const Fields<T> &f = c->F<T>();
+    const Ahead ah = BEGIN ? ahead_of<T>(g, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta, f.H, f.Ubar, f.Vbar})
+                           : ahead_of<T>(g, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta});
+    k_exchange<T, BEGIN><<<gr, b, 0, c->stream>>>(g, f, sponge ? 1 : 0, age ? 1 : 0, nby, ah);
     note(c);
     return true;
 }
@@ -4580,7 +4662,7 @@ template <typename T> void launch_begin_step(fw_ctx *c) {
 
 template <typename T> void launch_dispersion(fw_ctx *c) {
     const Grid &g = c->g;
-    k_disp_a<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_A)), c->blk(TK_DISP_A), 0, c->stream>>>(g, c->F<T>());
+    launch_disp_a<T>(c);
     note(c);
     k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, c->F<T>(), disp_k(g));
     note(c);
@@ -4800,11 +4882,9 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
     // previous exchange in the ghost corners (bc.F:735-740), so the last
     // stage's corners hold the second stage's values
     if (istage >= 2 && g.track_rad)
-        k_update<T, true><<<grid2(g.Mloc, g.Nloc, c->blk(TK_UPDATE)), c->blk(TK_UPDATE), 0, c->stream>>>(
-            g, c->F<T>(), al, be);
+        launch_update<T, true>(c, al, be);
     else
-        k_update<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_UPDATE)), c->blk(TK_UPDATE), 0, c->stream>>>(g, c->F<T>(), al,
-                                                                                                     be);
+        launch_update<T, false>(c, al, be);
     note(c);
     if (g.dispersion) {
         if (sizeof(T) == sizeof(float) && c->factored) {
@@ -4936,7 +5016,7 @@ template <typename T> void launch_stage(fw_ctx *c, int istage) {
         // GET_Eta_U_V_HU_HV tail + UPDATE_MASK + BREAKING (parallel part)
         // in one kernel, then the breaking sweep's candidates
         launch_estimate_huv_opt<T>(c, istage, false);
-        k_post_mask_break<T><<<grid2(g.Mloc + 1, g.Nloc + 1, c->blk(TK_PMB)), c->blk(TK_PMB), 0, c->stream>>>(g, c->F<T>());
+        launch_pmb<T>(c);
         note(c);
         auto &F = c->F<T>();
         uint8_t *t = F.MASK;
@@ -5035,15 +5115,12 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     Fields<T> &f = c->F<T>();
     const dim3 gc = grid2(g.Mloc, g.Nloc, B2D);
     auto is = [&](const char *n) { return std::strcmp(name, n) == 0; };
-    if (is("disp_a")) k_disp_a<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_A)), c->blk(TK_DISP_A), 0, c->stream>>>(g, f);
+    if (is("disp_a")) launch_disp_a<T>(c);
     else if (is("disp_b")) k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, f, disp_k(g));
     else if (is("flux_x")) { launch_flux<T, 0>(c); return 0; }
     else if (is("flux_y")) { launch_flux<T, 1>(c); return 0; }
-    else if (is("update")) k_update<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_UPDATE)), c->blk(TK_UPDATE), 0, c->stream>>>(g, f, (T)0.75, (T)0.25);
-    else if (is("post_mask_break")) {
-        const dim3 b = c->blk(TK_PMB);
-        k_post_mask_break<T><<<grid2(g.Mloc + 1, g.Nloc + 1, b), b, 0, c->stream>>>(g, f);
-    }
+    else if (is("update")) launch_update<T, false>(c, (T)0.75, (T)0.25);
+    else if (is("post_mask_break")) launch_pmb<T>(c);
     else if (is("tri_x")) { launch_tri<T, 0, false>(c, c->px); return 0; }
     else if (is("tri_y")) {
         if (g.periodic) launch_tri<T, 1, true>(c, c->py);
