@@ -34,6 +34,11 @@
 namespace fw {
 
 #define IDX(i, j) ((size_t)(i) + (size_t)(j) * (size_t)g.pitch)
+// in 32 bits (fw_create keeps a plane below 2^31 cells): fewer instructions and
+// registers an address where a kernel reads one cell of many planes
+// (2048 x 2048: k_post_mask_break 62 -> 52 us, k_disp_a 60 -> 57); the stencils of k_disp_b and
+// k_update are faster with IDX (115 and 128 us, 131 and 132 with this)
+#define IDI(i, j) ((i) + (j) * g.pitch)
 
 // pi as the reference stores it: a default-REAL literal (mod_param.F:71)
 constexpr double PI_SP = (double)(float)3.141592653;
@@ -52,6 +57,13 @@ __device__ __forceinline__ void prefetch_l1(const void *p) {
 // path, which also frees the compiler to issue it before the kernel's
 // stores (the Fields pointers could otherwise alias them)
 template <typename X> __device__ __forceinline__ X ro(const X *p) { return __ldg(p); }
+// the same of element id; in the mixed path the offset in bytes has 32 bits too,
+// so that the address is a uniform base and one register (a float plane of 4
+// GiB would need an arena of more than 288 GiB)
+template <typename X> __device__ __forceinline__ X ro(const X *p, int id) {
+    if constexpr (sizeof(X) <= 4) return __ldg((const X *)((const char *)p + (unsigned)id * (unsigned)sizeof(X)));
+    else return __ldg(p + id);
+}
 
 __device__ __forceinline__ double fsqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float fsqrt(float x) { return sqrtf(x); }
@@ -166,38 +178,52 @@ __device__ __forceinline__ int period_y(const Grid &g, int j) {
 // to cover the memory's latency.  Its threads therefore also bring to the L2,
 // one line each, the lines that the block `dist` places later reads; that
 // block's loads then wait for the L2 only.
-// Mixed 2048 x 2048: k_update 146 -> 128 us, k_disp_a 74 -> 62,
-// k_post_mask_break 68 -> 62, k_exchange 35 -> 34 and at a step's begin 94 ->
-// 90.  The distance matters little between one and four blocks per SM (with
+// Mixed 2048 x 2048: k_update 146 -> 128 us, k_disp_a 74 -> 60,
+// k_post_mask_break 68 -> 62, k_exchange 35 -> 33 and at a step's begin 94 ->
+// 86.  The distance matters little between one and four blocks per SM (with
 // twice the resident blocks the gain is gone); k_disp_b and the fluxes, bound
 // by their issue, gain nothing.
 // ---------------------------------------------------------------------------
 struct Ahead {
     const void *p[28];
-    int n, dist;  // planes; blocks ahead (0: none)
+    int n;       // planes (0: none)
+    int dx, dy;  // the later block: columns and rows of blocks from this one
+    int lx, ll;  // log2 of a block's lines of a plane: in a row, in all
 };
-// from min_cells cells on
+// dist: blocks ahead in a grid of nbx columns of blocks b; from min_cells cells
+// on, and for blocks of a power of two of lines (the thread's line then needs
+// no division)
 template <typename T>
-static Ahead ahead_of(const Grid &g, long long min_cells, int dist, std::initializer_list<const T *> planes) {
+static Ahead ahead_of(const Grid &g, dim3 b, int nbx, long long min_cells, int dist, std::initializer_list<const T *> planes) {
     Ahead a{};
+    const unsigned nx = (b.x + 31) / 32, lines = nx * b.y;
+    if (sizeof(T) != sizeof(float) || (long long)g.Mloc * g.Nloc < min_cells || (nx & (nx - 1)) || (lines & (lines - 1)))
+        return a;
     for (const T *q : planes) a.p[a.n++] = q;
-    a.dist = sizeof(T) == sizeof(float) && (long long)g.Mloc * g.Nloc >= min_cells ? dist : 0;
+    a.dx = dist % nbx;
+    a.dy = dist / nbx;
+    while (1u << a.lx < nx) a.lx++;
+    while (1u << a.ll < lines) a.ll++;
     return a;
 }
 // blocks of blockDim.x x blockDim.y cells from column 0 and row j0 on; by: the
 // block's row
 template <typename T>
-__device__ __forceinline__ void prefetch_ahead(const Grid &g, const Ahead &a, unsigned by, int j0) {
+__device__ __forceinline__ void prefetch_ahead(const Grid &g, const Ahead &a, int by, int j0) {
     if constexpr (sizeof(T) == sizeof(float)) {
-        if (a.dist == 0) return;
-        const unsigned b = blockIdx.x + by * gridDim.x + a.dist;
-        const unsigned by2 = b / gridDim.x, bx2 = b - by2 * gridDim.x;
-        const unsigned nx = (blockDim.x + 31) / 32, lines = nx * blockDim.y;  // of a plane
-        for (unsigned t = threadIdx.x + threadIdx.y * blockDim.x; t < a.n * lines; t += blockDim.x * blockDim.y) {
-            const unsigned q = t / lines, r = t - q * lines, y = r / nx, x = r - y * nx;
-            const int i = (int)(bx2 * blockDim.x + x * 32), j = j0 + (int)(by2 * blockDim.y + y);
+        if (a.n == 0) return;
+        int bx = blockIdx.x + a.dx;
+        by += a.dy;
+        if (bx >= (int)gridDim.x) {
+            bx -= gridDim.x;
+            by++;
+        }
+        const int i0 = bx * blockDim.x;
+        j0 += by * blockDim.y;
+        for (int t = threadIdx.x + threadIdx.y * blockDim.x; t < a.n << a.ll; t += blockDim.x * blockDim.y) {
+            const int q = t >> a.ll, r = t & ((1 << a.ll) - 1), i = i0 + (r & ((1 << a.lx) - 1)) * 32, j = j0 + (r >> a.lx);
             if (i < g.Mloc && j < g.Nloc)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T *>(a.p[q]) + IDX(i, j)));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T *>(a.p[q]) + IDI(i, j)));
         }
     }
 }
@@ -214,14 +240,14 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f, Ahead ah) {
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mloc || j >= g.Nloc) return;
     const T DX = GC(DX), DY = GC(DY), mdf = GC(min_depth_frc);
-    const size_t id = IDX(i, j);
+    const int id = IDI(i, j);
     // ETAT from the previous stage's face fluxes (dispersion.F:103-119)
     if (i <= g.Mloc - 2 && j <= g.Nloc - 2) {
         if constexpr (sizeof(T) == sizeof(double))
-            f.ETAT[id] = over(-(ro(f.P + (IDX(i + 1, j))) - ro(f.P + (id))), DX, (T)g.rdx) -
-                         over(ro(f.Q + (IDX(i, j + 1))) - ro(f.Q + (id)), DY, (T)g.rdy);
+            f.ETAT[id] = over(-(ro(f.P + (IDI(i + 1, j))) - ro(f.P + (id))), DX, (T)g.rdx) -
+                         over(ro(f.Q + (IDI(i, j + 1))) - ro(f.Q + (id)), DY, (T)g.rdy);
         else
-            f.ETAT[id] = -(ro(f.P + (IDX(i + 1, j))) - ro(f.P + (id))) * GC(rdx) - (ro(f.Q + (IDX(i, j + 1))) - ro(f.Q + (id))) * GC(rdy);
+            f.ETAT[id] = -(ro(f.P + (IDI(i + 1, j))) - ro(f.P + (id))) * GC(rdx) - (ro(f.Q + (IDI(i, j + 1))) - ro(f.Q + (id))) * GC(rdy);
     }
 
     const bool gx = (i < g.ib) || (i > g.ie);
@@ -241,12 +267,12 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f, Ahead ah) {
     }
     const T sx2 = gx ? (T)-1 : (T)1;  // sign of VTYPE 2 fields in an x ghost
 
-    const T m9 = m2r<T>(ro(f.MASK9 + (IDX(si, sj))));
+    const T m9 = m2r<T>(ro(f.MASK9 + (IDI(si, sj))));
     const bool wall = (si == g.ib) || (si == g.ie) || (sj == g.jb) || (sj == g.je);
-#define LU(a, b) ro(f.U + (IDX(si + (a), sj + (b))))
-#define LV(a, b) ro(f.V + (IDX(si + (a), sj + (b))))
-#define LDU(a, b) (max_pos(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LU(a, b))
-#define LDV(a, b) (max_pos(ro(f.Depth + (IDX(si + (a), sj + (b)))), mdf) * LV(a, b))
+#define LU(a, b) ro(f.U + (IDI(si + (a), sj + (b))))
+#define LV(a, b) ro(f.V + (IDI(si + (a), sj + (b))))
+#define LDU(a, b) (max_pos(ro(f.Depth + (IDI(si + (a), sj + (b)))), mdf) * LU(a, b))
+#define LDV(a, b) (max_pos(ro(f.Depth + (IDI(si + (a), sj + (b)))), mdf) * LV(a, b))
     // FP64: the reference's divisions; mixed: reciprocal constants
     constexpr bool EXACT = sizeof(T) == sizeof(double);
     const T rdx2 = (T)g.f_rdx2, rdy2 = (T)g.f_rdy2, rdxy4 = (T)g.f_rdxy4;
@@ -290,8 +316,8 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f, Ahead ah) {
     // (bc.F:395-398); without Gamma2 the ghosts keep their old values
     const bool exch = g.has_g2 != 0;
     if (exch || (g.show_breaking && !gx && !gy)) {
-        const T dex = ro(f.Eta + (IDX(si + 1, sj))) - ro(f.Eta + (IDX(si - 1, sj)));
-        const T dey = ro(f.Eta + (IDX(si, sj + 1))) - ro(f.Eta + (IDX(si, sj - 1)));
+        const T dex = ro(f.Eta + (IDI(si + 1, sj))) - ro(f.Eta + (IDI(si - 1, sj)));
+        const T dey = ro(f.Eta + (IDI(si, sj + 1))) - ro(f.Eta + (IDI(si, sj - 1)));
         const T ex = EXACT ? (T)(QX(dex) / 2.0 * m9) : dex * (T)g.f_hdx * m9;
         const T ey = EXACT ? (T)(QY(dey) / 2.0 * m9) : dey * (T)g.f_hdy * m9;
         if (!stale) {
@@ -299,12 +325,12 @@ __global__ void __launch_bounds__(256) k_disp_a(Grid g, Fields<T> f, Ahead ah) {
                 // the periodic copy (bc.F:735-740) runs before the x mirror:
                 // a corner cell receives this x-ghost cell's previous value
                 if (j >= g.je - 2) {
-                    f.ETAx[IDX(i, j - (g.je - 2))] = f.ETAx[id];
-                    f.ETAy[IDX(i, j - (g.je - 2))] = f.ETAy[id];
+                    f.ETAx[IDI(i, j - (g.je - 2))] = f.ETAx[id];
+                    f.ETAy[IDI(i, j - (g.je - 2))] = f.ETAy[id];
                 }
                 if (j <= g.jb + 2) {
-                    f.ETAx[IDX(i, j + g.je - 2)] = f.ETAx[id];
-                    f.ETAy[IDX(i, j + g.je - 2)] = f.ETAy[id];
+                    f.ETAx[IDI(i, j + g.je - 2)] = f.ETAx[id];
+                    f.ETAy[IDI(i, j + g.je - 2)] = f.ETAy[id];
                 }
             }
             f.ETAx[id] = sx2 * ex;
@@ -3234,7 +3260,7 @@ __global__ void __launch_bounds__(LSF_T, 2) k_linesolve(Grid g, Fields<T> f, Lin
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ void post_cell(const Grid &g, const Fields<T> &f, int i, int j) {
-    const size_t id = IDX(i, j);
+    const int id = IDI(i, j);
     const T mdf = GC(min_depth_frc);
     const bool interior = !(i < g.ib || i > g.ie || j < g.jb || j > g.je);
     if (interior) {
@@ -3284,7 +3310,7 @@ __global__ void k_nodisp_copy(Grid g, Fields<T> f) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= g.Mloc || j >= g.Nloc) return;
-    const size_t id = IDX(i, j);
+    const int id = IDI(i, j);
     f.Ubar[id] = f.HU[id];
     f.Vbar[id] = f.HV[id];
 }
@@ -3325,7 +3351,7 @@ __device__ __forceinline__ bool in_mask_range(const Grid &g, int a, int b) {
 }
 template <typename T>
 __device__ __forceinline__ int new_mask(const Grid &g, const Fields<T> &f, int a, int b) {
-    const size_t q = IDX(a, b);
+    const size_t q = IDI(a, b);
     const int m = ro(f.MASK + (q));
     if (!in_mask_range<T>(g, a, b) || ro(f.MASK_STRUC + (q)) != 1) return m;
     // total-depth tests (masks.F:107, 129) of eta against Depth as given, in
@@ -3335,10 +3361,10 @@ __device__ __forceinline__ int new_mask(const Grid &g, const Fields<T> &f, int a
     if (m < 1) {
         int r = m;
         if (side > 0) r = 1;
-        if (ro(f.MASK + (IDX(a - 1, b))) == 1 && ro(f.Eta + (IDX(a - 1, b))) > eta) r = 1;
-        if (ro(f.MASK + (IDX(a + 1, b))) == 1 && ro(f.Eta + (IDX(a + 1, b))) > eta) r = 1;
-        if (ro(f.MASK + (IDX(a, b - 1))) == 1 && ro(f.Eta + (IDX(a, b - 1))) > eta) r = 1;
-        if (ro(f.MASK + (IDX(a, b + 1))) == 1 && ro(f.Eta + (IDX(a, b + 1))) > eta) r = 1;
+        if (ro(f.MASK + (IDI(a - 1, b))) == 1 && ro(f.Eta + (IDI(a - 1, b))) > eta) r = 1;
+        if (ro(f.MASK + (IDI(a + 1, b))) == 1 && ro(f.Eta + (IDI(a + 1, b))) > eta) r = 1;
+        if (ro(f.MASK + (IDI(a, b - 1))) == 1 && ro(f.Eta + (IDI(a, b - 1))) > eta) r = 1;
+        if (ro(f.MASK + (IDI(a, b + 1))) == 1 && ro(f.Eta + (IDI(a, b + 1))) > eta) r = 1;
         return r;
     }
     return (side < 0) ? 0 : m;
@@ -3351,18 +3377,18 @@ __device__ __forceinline__ void mask_cell(const Grid &g, const Fields<T> &f, int
     if (j < g.Nloc && j >= g.jb - 2 && j <= g.je + 2) {
         const bool rin = (i >= g.ib - 2 && i <= g.ie + 2);
         const bool lin = (i - 1 >= g.ib - 2 && i - 1 <= g.ie + 2);
-        if (rin && ro(f.MASK + (IDX(i, j))) < 1) f.Depthx[IDX(i, j)] = ro(f.Depth + (IDX(i - 1, j)));
-        else if (lin && ro(f.MASK + (IDX(i - 1, j))) < 1) f.Depthx[IDX(i, j)] = ro(f.Depth + (IDX(i, j)));
+        if (rin && ro(f.MASK + (IDI(i, j))) < 1) f.Depthx[IDI(i, j)] = ro(f.Depth + (IDI(i - 1, j)));
+        else if (lin && ro(f.MASK + (IDI(i - 1, j))) < 1) f.Depthx[IDI(i, j)] = ro(f.Depth + (IDI(i, j)));
     }
     // Depthy at y-face j of column i
     if (i < g.Mloc && i >= g.ib - 2 && i <= g.ie + 2) {
         const bool tin = (j >= g.jb - 2 && j <= g.je + 2);
         const bool bin = (j - 1 >= g.jb - 2 && j - 1 <= g.je + 2);
-        if (tin && ro(f.MASK + (IDX(i, j))) < 1) f.Depthy[IDX(i, j)] = ro(f.Depth + (IDX(i, j - 1)));
-        else if (bin && ro(f.MASK + (IDX(i, j - 1))) < 1) f.Depthy[IDX(i, j)] = ro(f.Depth + (IDX(i, j)));
+        if (tin && ro(f.MASK + (IDI(i, j))) < 1) f.Depthy[IDI(i, j)] = ro(f.Depth + (IDI(i, j - 1)));
+        else if (bin && ro(f.MASK + (IDI(i, j - 1))) < 1) f.Depthy[IDI(i, j)] = ro(f.Depth + (IDI(i, j)));
     }
     if (i >= g.Mloc || j >= g.Nloc) return;
-    const size_t id = IDX(i, j);
+    const int id = IDI(i, j);
     f.MASKn[id] = (uint8_t)new_mask(g, f, i, j);
     // MASK9 on Ibeg-1..Iend+1 x Jbeg-1..Jend+1; 0 elsewhere (never written
     // in the reference, whose temporary is fresh memory)
@@ -3397,7 +3423,7 @@ template <typename T> struct BrkLocal {
     T tmp1, tmp2, tmp3, et;
 };
 template <typename T>
-__device__ __forceinline__ BrkLocal<T> brk_local(const Grid &g, const Fields<T> &f, size_t id) {
+__device__ __forceinline__ BrkLocal<T> brk_local(const Grid &g, const Fields<T> &f, int id) {
     BrkLocal<T> b;
     b.tmp3 = fsqrt((T)GRAV * tmax(GC(min_depth_frc), ro(f.H + (id))));
     b.tmp1 = GC(cbrk1) * b.tmp3;
@@ -3427,7 +3453,7 @@ __device__ __forceinline__ T nu_of(const Grid &g, const BrkLocal<T> &b, T age, b
     return (T)0 + GC(nu_bkg);
 }
 template <typename T>
-__device__ __forceinline__ T nu_value(const Grid &g, const Fields<T> &f, size_t id, const BrkLocal<T> &b, T age,
+__device__ __forceinline__ T nu_value(const Grid &g, const Fields<T> &f, int id, const BrkLocal<T> &b, T age,
                                       bool zone) {
     return nu_of(g, b, age, zone, ro(f.Depth + (id)), ro(f.Eta + (id)));
 }
@@ -3439,7 +3465,7 @@ __device__ __forceinline__ T nu_value(const Grid &g, const Fields<T> &f, size_t 
 // a _SP one, so both enter FP64 as their float values.  ETAmean is zero
 // until a mean is computed.
 template <typename T>
-__device__ __forceinline__ void roller_cell(const Grid &g, const Fields<T> &f, size_t id, T et) {
+__device__ __forceinline__ void roller_cell(const Grid &g, const Fields<T> &f, int id, T et) {
     const T ex = ro(f.ETAx + (id)), ey = ro(f.ETAy + (id));
     const T tmp4 = tmax(fsqrt(ex * ex + ey * ey), (T)SMALL);
     const T ANGLE = fatan2(-ey, -ex) * (T)180 / (T)PI_SP;
@@ -3461,7 +3487,7 @@ template <typename T> __device__ __forceinline__ bool breaking_now(const Grid &g
 
 template <typename T>
 __device__ __forceinline__ void break_cell(const Grid &g, const Fields<T> &f, int i, int j) {
-    const size_t id = IDX(i, j);
+    const int id = IDI(i, j);
     const T age = ro(f.AGE + (id));
     if (i < g.ib - 1 || i > g.ie + 1 || j < g.jb - 1 || j > g.je + 1) {
         f.AGEn[id] = age;
@@ -3501,8 +3527,8 @@ __global__ void __launch_bounds__(256) k_break_a(Grid g, Fields<T> f) {
 // and viscosity breaking on (MASK9 = 1), needs one value of each input: they
 // are loaded together before the first use (the parts one after the other,
 // each loading behind the stores of the one before: 88 us at 2048 x 2048, now
-// 60, 2.6 times the floor of its 57 B per cell; the wait for those loads is
-// what is left).  The others take the parts one by one.
+// 52 with 32-bit offsets and lines ahead, 1.5 times the floor of its 57 B per
+// cell).  The others take the parts one by one.
 template <typename T>
 __global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f, Ahead ah) {
     prefetch_ahead<T>(g, ah, blockIdx.y, 0);
@@ -3512,11 +3538,11 @@ __global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f, Ah
     const bool in = i >= g.ib && i <= g.ie && j >= g.jb && j <= g.je;
     if (in && g.visc_breaking && g.dispersion) {
         const int id = i + j * g.pitch;
-        const int m = ro(f.MASK + id), mw = ro(f.MASK + (id - 1)), ms = ro(f.MASK + (id - g.pitch)),
-                  st = ro(f.MASK_STRUC + id), m9 = f.MASK9[id];
-        const T h = ro(f.H + id), u = f.U[id], v = f.V[id], age = ro(f.AGE + id), eta = ro(f.Eta + id), dep = ro(f.Depth + id);
+        const int m = ro(f.MASK, id), mw = ro(f.MASK, id - 1), ms = ro(f.MASK, id - g.pitch),
+                  st = ro(f.MASK_STRUC, id), m9 = f.MASK9[id];
+        const T h = ro(f.H, id), u = f.U[id], v = f.V[id], age = ro(f.AGE, id), eta = ro(f.Eta, id), dep = ro(f.Depth, id);
         BrkLocal<T> b;
-        b.et = ro(f.ETAT + id);
+        b.et = ro(f.ETAT, id);
         const T mdf = GC(min_depth_frc);
         if (m >= 1 && mw >= 1 && ms >= 1) {
             // GET_Eta_U_V_HU_HV tail (post_cell)
@@ -4571,16 +4597,18 @@ template <typename T> static void launch_disp_a(fw_ctx *c) {
     const Grid &g = c->g;
     const Fields<T> &f = c->F<T>();
     const dim3 b = c->blk(TK_DISP_A);
-    k_disp_a<T><<<grid2(g.Mloc, g.Nloc, b), b, 0, c->stream>>>(
-        g, f, ahead_of<T>(g, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.Depth, f.Eta, f.P, f.Q}));
+    const dim3 gr = grid2(g.Mloc, g.Nloc, b);
+    k_disp_a<T><<<gr, b, 0, c->stream>>>(
+        g, f, ahead_of<T>(g, b, gr.x, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.Depth, f.Eta, f.P, f.Q}));
 }
 template <typename T, bool RAD> static void launch_update(fw_ctx *c, T al, T be) {
     const Grid &g = c->g;
     const Fields<T> &f = c->F<T>();
     const dim3 b = c->blk(TK_UPDATE);
-    k_update<T, RAD><<<grid2(g.Mloc, g.Nloc, b), b, 0, c->stream>>>(
+    const dim3 gr = grid2(g.Mloc, g.Nloc, b);
+    k_update<T, RAD><<<gr, b, 0, c->stream>>>(
         g, f, al, be,
-        ahead_of<T>(g, AHEAD_UPDATE, 2 * 152, {f.Eta0, f.Ubar0, f.Vbar0, f.Eta, f.Ubar, f.Vbar, f.P, f.Q, f.Fx, f.Fy, f.Gx, f.Gy,
+        ahead_of<T>(g, b, gr.x, AHEAD_UPDATE, 2 * 152, {f.Eta0, f.Ubar0, f.Vbar0, f.Eta, f.Ubar, f.Vbar, f.P, f.Q, f.Fx, f.Fy, f.Gx, f.Gy,
                                               f.Depth, f.H, f.U, f.V, f.U4, f.V4, f.Depthx, f.Depthy, f.Udisp, f.Vdisp, f.U1p,
                                               f.V1p, f.Cd, f.HU, f.HV, f.nu}));
 }
@@ -4588,8 +4616,9 @@ template <typename T> static void launch_pmb(fw_ctx *c) {
     const Grid &g = c->g;
     const Fields<T> &f = c->F<T>();
     const dim3 b = c->blk(TK_PMB);
-    k_post_mask_break<T><<<grid2(g.Mloc + 1, g.Nloc + 1, b), b, 0, c->stream>>>(
-        g, f, ahead_of<T>(g, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.H, f.AGE, f.Eta, f.Depth, f.ETAT}));
+    const dim3 gr = grid2(g.Mloc + 1, g.Nloc + 1, b);
+    k_post_mask_break<T><<<gr, b, 0, c->stream>>>(
+        g, f, ahead_of<T>(g, b, gr.x, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.H, f.AGE, f.Eta, f.Depth, f.ETAT}));
 }
 
 // EXCHANGE in one launch; false for grids too small for it
@@ -4604,8 +4633,8 @@ template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, boo
         gr.y += (n + per - 1) / per;
     }
     const Fields<T> &f = c->F<T>();
-    const Ahead ah = BEGIN ? ahead_of<T>(g, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta, f.H, f.Ubar, f.Vbar})
-                           : ahead_of<T>(g, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta});
+    const Ahead ah = BEGIN ? ahead_of<T>(g, b, gr.x, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta, f.H, f.Ubar, f.Vbar})
+                           : ahead_of<T>(g, b, gr.x, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta});
     k_exchange<T, BEGIN><<<gr, b, 0, c->stream>>>(g, f, sponge ? 1 : 0, age ? 1 : 0, nby, ah);
     note(c);
     return true;
