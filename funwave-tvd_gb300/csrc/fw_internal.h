@@ -246,6 +246,10 @@ struct fw_ctx {
     int graph1_next = 0;
     void invalidate_graphs() { graph_ready = graph1_ok[0] = graph1_ok[1] = 0; }
     // asynchronous output (fw_output_begin / fw_output_wait): host-layout
+    // the second branch of a captured step's graph
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    bool one_branch = false;  // the capture under way takes one branch only
     // snapshots in out_buf, copied to the caller's buffers on out_stream
     void *out_buf = nullptr;
     size_t out_cap = 0;

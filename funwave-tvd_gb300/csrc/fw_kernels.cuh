@@ -4604,6 +4604,41 @@ static inline void note(fw_ctx *c, int n = 1) {
     if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
 }
 
+// A captured step's launches that do not depend on one another go on two
+// branches of its graph: the time step's end beside the first dispersion
+// kernel, the factorisation (an early exit while MASK9 stands) beside the
+// dispersion and the fluxes, the x fluxes beside the y fluxes and the x solve
+// beside the y solve (they read the same planes and write their own).  On a
+// small grid each of them leaves most of the GPU idle, on a large one the
+// second fills the first one's last wave (a step of 128 x 256 cells 174 -> 143
+// us, 250 x 500 194 -> 152, 2048 x 2048 2134 -> 2081; 250 x 500 in double 3186
+// -> 3063, 701 x 937 11.0 -> 10.8 ms).
+// Outside a capture (the entry points of single parts) everything stays on the
+// context's stream, in the order of the step.
+static bool branching(fw_ctx *c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return !c->one_branch && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive;
+}
+// what `to` runs from here on comes after what `from` has so far
+static void branch_after(fw_ctx *c, cudaStream_t to, cudaStream_t from, cudaEvent_t ev) {
+    cudaError_t e = cudaEventRecord(ev, from);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
+    if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
+}
+// the launches of f on the side branch (behind what the step has so far), or
+// in line
+template <typename F> static void on_side(fw_ctx *c, bool branch, F f) {
+    if (!branch) return f();
+    cudaStream_t main = c->stream;
+    branch_after(c, c->side, main, c->fork_ev);
+    c->stream = c->side;
+    f();
+    c->stream = main;
+}
+static void join_side(fw_ctx *c, bool branch) {
+    if (branch) branch_after(c, c->stream, c->side, c->join_ev);
+}
+
 template <typename T> void launch_ghost(fw_ctx *c, bool full) {
     const Grid &g = c->g;
     int n = 6 * g.Nglob + 6 * g.Mloc;
@@ -4703,7 +4738,7 @@ template <typename T> void launch_estimate_dt(fw_ctx *c) {
 template <typename T> void launch_begin_step(fw_ctx *c) {
     const Grid &g = c->g;
     if (launch_exchange_one<T, true>(c, false, B2D)) {
-        launch_dt_final(c);
+        on_side(c, branching(c), [&] { launch_dt_final(c); });  // joined by the first stage
         return;
     }
     const int nring = 6 * g.Mloc + 6 * g.Nglob;
@@ -4712,15 +4747,19 @@ template <typename T> void launch_begin_step(fw_ctx *c) {
     launch_ghost<T>(c, g.visc_breaking != 0);
     k_begin<T><<<grid2(g.Mloc, g.Nloc, B2D), B2D, 0, c->stream>>>(g, c->F<T>());
     note(c);
-    launch_dt_final(c);
+    on_side(c, branching(c), [&] { launch_dt_final(c); });
 }
 
-template <typename T> void launch_dispersion(fw_ctx *c) {
+template <typename T> static void launch_disp_b(fw_ctx *c) {
     const Grid &g = c->g;
+    const dim3 b = c->blk(TK_DISP_B);
+    k_disp_b<T><<<grid2(g.Mloc, g.Nloc, b), b, disp_b_smem<T>(b), c->stream>>>(g, c->F<T>(), disp_k(g));
+    note(c);
+}
+template <typename T> void launch_dispersion(fw_ctx *c) {
     launch_disp_a<T>(c);
     note(c);
-    k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, c->F<T>(), disp_k(g));
-    note(c);
+    launch_disp_b<T>(c);
 }
 
 // the TMA-staged flux kernel with the maps of the current MASK buffer (its
@@ -4784,10 +4823,13 @@ template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
     note(c);
 }
 
-template <typename T> void launch_fluxes(fw_ctx *c) {
+template <typename T> static void launch_fluxes_opt(fw_ctx *c, bool branch) {
+    if (branch) on_side(c, true, [&] { launch_flux<T, 1>(c); });
     launch_flux<T, 0>(c);
-    launch_flux<T, 1>(c);
+    if (!branch) launch_flux<T, 1>(c);
+    join_side(c, branch);
 }
+template <typename T> void launch_fluxes(fw_ctx *c) { launch_fluxes_opt<T>(c, false); }
 
 template <typename T> void launch_sources_debug(fw_ctx *c) {
     const Grid &g = c->g;
@@ -4926,9 +4968,37 @@ static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clea
     return false;
 }
 
+// the factors that the solves of both directions keep, brought up to date when
+// MASK9 has changed
+template <typename T> static bool kept_factors(const fw_ctx *c) {
+    return c->g.dispersion && (sizeof(T) == sizeof(float) ? c->factored != 0 : thomas_kept(c));
+}
+template <typename T> static void launch_factors(fw_ctx *c) {
+    const Grid &g = c->g;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        launch_thomas_fac<T>(c);
+        note(c);
+    } else {
+        const int nbx = (c->px.nlines * c->px.P + 127) / 128;
+        const int nby = (c->py.nlines * c->py.P + 127) / 128;
+        const int lbx = (c->px.nlines + 127) / 128, lby = (c->py.nlines + 127) / 128;
+        const int nm = std::min((lsf_line(c->px) ? c->px.nlines : 0) + (lsf_line(c->py) ? c->py.nlines : 0), PCR_BLOCKS);
+        const size_t sp = nm ? 12 * std::max(lsf_line(c->px) ? c->px.P : 0, lsf_line(c->py) ? c->py.P : 0) * sizeof(float) : 0;
+        if (g.periodic) {
+            k_fac_a_xy<T, true><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
+            k_fac_b_xy<T, true><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
+        } else {
+            k_fac_a_xy<T, false><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
+            k_fac_b_xy<T, false><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
+        }
+        note(c, 2);
+    }
+}
+
 // ESTIMATE_HUV; with_post = false leaves the GET_Eta_U_V_HU_HV tail (k_post)
-// to the fused kernel of the stage
-template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage, bool with_post) {
+// to the fused kernel of the stage; branch: a captured stage, whose side branch
+// has brought the factors up to date and is joined
+template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage, bool with_post, bool branch) {
     const Grid &g = c->g;
     static const double AL[3] = {0.0, 3.0 / 4.0, 1.0 / 3.0};
     static const double BE[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
@@ -4942,33 +5012,25 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
         launch_update<T, false>(c, al, be);
     note(c);
     if (g.dispersion) {
+        if (!branch && kept_factors<T>(c)) launch_factors<T>(c);
         if (sizeof(T) == sizeof(float) && c->factored) {
-            // factor both directions (when MASK9 changed) in one launch each,
-            // then solve; the x solve resets the change flag when it can
-            const int nbx = (c->px.nlines * c->px.P + 127) / 128;
-            const int nby = (c->py.nlines * c->py.P + 127) / 128;
-            const int lbx = (c->px.nlines + 127) / 128, lby = (c->py.nlines + 127) / 128;
-            const int nm = std::min((lsf_line(c->px) ? c->px.nlines : 0) + (lsf_line(c->py) ? c->py.nlines : 0), PCR_BLOCKS);
-            const size_t sp = nm ? 12 * std::max(lsf_line(c->px) ? c->px.P : 0, lsf_line(c->py) ? c->py.P : 0) * sizeof(float) : 0;
-            if (g.periodic) {
-                k_fac_a_xy<T, true><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
-                k_fac_b_xy<T, true><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
-            } else {
-                k_fac_a_xy<T, false><<<nbx + nby, 128, 0, c->stream>>>(g, c->F<T>(), c->px, c->py, nbx);
-                k_fac_b_xy<T, false><<<lbx + lby + nm, 128, sp, c->stream>>>(g, c->F<T>(), c->px, c->py, lbx, lby);
-            }
-            note(c, 2);
+            // the x solve resets the change flag when it can
+            const bool both = branch && lsf_line(c->px) && lsf_line(c->py);
+            auto y = [&] {
+                if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
+                else launch_tri<T, 1, false>(c, c->py, false);
+            };
+            if (both) on_side(c, true, y);
             const bool cleared = launch_tri<T, 0, false>(c, c->px, false, true);
-            if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
-            else launch_tri<T, 1, false>(c, c->py, false);
+            if (!both) y();
+            join_side(c, both);
             if (!cleared) {
                 k_fac_clear<<<1, 1, 0, c->stream>>>(c->F<T>().m9_dirty);
                 note(c);
             }
         } else {
-            // (kept FP64 factors: brought up to date before the x solve, which
-            // clears the change flag)
-            launch_tri<T, 0, false>(c, c->px, true, true);
+            // (the x solve clears the change flag of kept FP64 factors)
+            launch_tri<T, 0, false>(c, c->px, !kept_factors<T>(c), true);
             if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
             else launch_tri<T, 1, false>(c, c->py, false);
         }
@@ -4982,7 +5044,7 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
     }
 }
 
-template <typename T> void launch_estimate_huv(fw_ctx *c, int istage) { launch_estimate_huv_opt<T>(c, istage, true); }
+template <typename T> void launch_estimate_huv(fw_ctx *c, int istage) { launch_estimate_huv_opt<T>(c, istage, true, false); }
 
 template <typename T> void launch_update_mask(fw_ctx *c) {
     const Grid &g = c->g;
@@ -5065,12 +5127,34 @@ template <typename T> void launch_end_step(fw_ctx *c) {
 
 template <typename T> void launch_stage(fw_ctx *c, int istage) {
     const Grid &g = c->g;
-    if (g.dispersion) launch_dispersion<T>(c);
-    launch_fluxes<T>(c);
+    const bool branch = branching(c);
+    // the first stage joins the time step's end (on the side since the step
+    // began) before its first use
+    if (branch && kept_factors<T>(c)) {
+        if (istage == 1) {
+            const cudaError_t e = cudaEventRecord(c->join_ev, c->side);
+            if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
+        }
+        on_side(c, true, [&] { launch_factors<T>(c); });
+    }
+    if (g.dispersion) {
+        launch_disp_a<T>(c);
+        note(c);
+    }
+    if (branch && istage == 1) {
+        if (kept_factors<T>(c)) {
+            const cudaError_t e = cudaStreamWaitEvent(c->stream, c->join_ev, 0);
+            if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
+        } else {
+            join_side(c, true);
+        }
+    }
+    if (g.dispersion) launch_disp_b<T>(c);
+    launch_fluxes_opt<T>(c, branch);
     if (g.dispersion && g.show_breaking) {
         // GET_Eta_U_V_HU_HV tail + UPDATE_MASK + BREAKING (parallel part)
         // in one kernel, then the breaking sweep's candidates
-        launch_estimate_huv_opt<T>(c, istage, false);
+        launch_estimate_huv_opt<T>(c, istage, false, branch);
         launch_pmb<T>(c);
         note(c);
         auto &F = c->F<T>();
@@ -5083,7 +5167,7 @@ template <typename T> void launch_stage(fw_ctx *c, int istage) {
         F.AGE = F.AGEn;
         F.AGEn = a;
     } else {
-        launch_estimate_huv<T>(c, istage);
+        launch_estimate_huv_opt<T>(c, istage, true, branch);
         launch_update_mask<T>(c);
         launch_breaking<T>(c);
     }
@@ -5171,7 +5255,7 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     const dim3 gc = grid2(g.Mloc, g.Nloc, B2D);
     auto is = [&](const char *n) { return std::strcmp(name, n) == 0; };
     if (is("disp_a")) launch_disp_a<T>(c);
-    else if (is("disp_b")) k_disp_b<T><<<grid2(g.Mloc, g.Nloc, c->blk(TK_DISP_B)), c->blk(TK_DISP_B), disp_b_smem<T>(c->blk(TK_DISP_B)), c->stream>>>(g, f, disp_k(g));
+    else if (is("disp_b")) { launch_disp_b<T>(c); return 0; }
     else if (is("flux_x")) { launch_flux<T, 0>(c); return 0; }
     else if (is("flux_y")) { launch_flux<T, 1>(c); return 0; }
     else if (is("update")) launch_update<T, false>(c, (T)0.75, (T)0.25);
