@@ -1907,6 +1907,12 @@ __global__ void __launch_bounds__(32) k_thomas_fac(Grid g, Fields<T> f, LinePart
     else thomas_fac_body<T, 1, PERY>(g, f, py, (blockIdx.x - nbx) * 32 + threadIdx.x);
 }
 
+// the planes of 1/a and of d/a: each direction its own, so that both can be
+// solved at once (y: its right-hand side's place)
+template <typename T, int DIR> __device__ __forceinline__ double *tf_ra(const Fields<T> &f) { return DIR == 0 ? f.tc : f.tp; }
+template <typename T, int DIR> __device__ __forceinline__ double *tf_d(const Fields<T> &f) {
+    return DIR == 0 ? f.ty : reinterpret_cast<double *>(f.rhs_y);
+}
 // d/a (or d) and 1/a (or 0) of every row, as k_thomas_rows
 template <typename T, int DIR, bool PER>
 __global__ void __launch_bounds__(256) k_thomas_rhs(Grid g, Fields<T> f, LinePart lp, int clear_dirty) {
@@ -1921,7 +1927,7 @@ __global__ void __launch_bounds__(256) k_thomas_rhs(Grid g, Fields<T> f, LinePar
     const double dep = tmax((double)ro(f.Depth + q), mdf);
     const double depl = tmax((double)ro(f.Depth + (DIR == 0 ? IDX(i - 1, j) : IDX(i, j - 1))), mdf);
     const double m9 = ro(f.MASK9 + q) ? 1.0 : 0.0;
-    const double tmp4 = DIR == 0 ? ro(f.rhs_x + q) : ro(f.rhs_y + q);
+    const double tmp4 = DIR == 0 ? f.rhs_x[q] : f.rhs_y[q];
     const double k1 = g.tK1[DIR], k2 = g.tK2[DIR], k3 = g.tK3[DIR], k4 = g.tK4[DIR];
     const double gm = g1 * m9;
     const double tmp1 = gm * (k1 * dep * dep + k2 * depl * dep);
@@ -1940,8 +1946,8 @@ __global__ void __launch_bounds__(256) k_thomas_rhs(Grid g, Fields<T> f, LinePar
         ra = __drcp_rn(a);
         d = div_rcp_ok(a) ? div_rcp(d, a, ra) : d / a;
     }
-    f.tc[q] = ra;
-    f.ty[q] = d;
+    tf_ra<T, DIR>(f)[q] = ra;
+    tf_d<T, DIR>(f)[q] = d;
 }
 
 template <typename T, int DIR, bool PER>
@@ -2099,9 +2105,9 @@ __global__ void __launch_bounds__(PER ? 32 * THS_WARPS : 32) k_thomas_solve(Grid
     const int base = (int)(DIR == 0 ? IDX(g.ib, g.jb + (on ? l : 0)) : IDX(g.ib + (on ? l : 0), g.jb));
     const int step = DIR == 0 ? 1 : g.pitch;
     T *const out = (DIR == 0 ? f.U : f.V) + base;
-    double *const dp_ = f.ty + base;
+    double *const dp_ = tf_d<T, DIR>(f) + base;
     if (on && threadIdx.y == 0) {
-        const double *const ra_ = f.tc + base, *const fc_ = tf_c<T, DIR>(f) + base, *const fy_ = tf_y<T, DIR>(f) + base;
+        const double *const ra_ = tf_ra<T, DIR>(f) + base, *const fc_ = tf_c<T, DIR>(f) + base, *const fy_ = tf_y<T, DIR>(f) + base;
         double cp = 0.0, dp = 0.0;
         // one row as k_thomas_lines
         auto row = [&](double ra, double da, double fc, double fy) {
@@ -2168,7 +2174,7 @@ __global__ void __launch_bounds__(PER ? 32 * THS_WARPS : 32) k_thomas_solve(Grid
             row(ra_[q], dp_[q], fc_[q], fy_[q]);
             dp_[q] = dp;
         }
-        // back substitution: the first solution into ty (periodic), else
+        // back substitution: the first solution into d's place (periodic), else
         // straight into U / V
         double z = dp;
         auto put = [&](int k, double v) {
@@ -5013,13 +5019,13 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
     note(c);
     if (g.dispersion) {
         if (!branch && kept_factors<T>(c)) launch_factors<T>(c);
+        auto y = [&] {
+            if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
+            else launch_tri<T, 1, false>(c, c->py, false);
+        };
         if (sizeof(T) == sizeof(float) && c->factored) {
             // the x solve resets the change flag when it can
             const bool both = branch && lsf_line(c->px) && lsf_line(c->py);
-            auto y = [&] {
-                if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
-                else launch_tri<T, 1, false>(c, c->py, false);
-            };
             if (both) on_side(c, true, y);
             const bool cleared = launch_tri<T, 0, false>(c, c->px, false, true);
             if (!both) y();
@@ -5030,9 +5036,11 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
             }
         } else {
             // (the x solve clears the change flag of kept FP64 factors)
-            launch_tri<T, 0, false>(c, c->px, !kept_factors<T>(c), true);
-            if (g.periodic) launch_tri<T, 1, true>(c, c->py, false);
-            else launch_tri<T, 1, false>(c, c->py, false);
+            const bool kept = kept_factors<T>(c), both = branch && kept;
+            if (both) on_side(c, true, y);
+            launch_tri<T, 0, false>(c, c->px, !kept, true);
+            if (!both) y();
+            join_side(c, both);
         }
     }
     if (!with_post) return;
