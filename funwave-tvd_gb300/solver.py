@@ -484,7 +484,7 @@ class Solver:
         return ms.value
 
     # FW_TUNE_LEN of include/funwave_gpu.h: (bx, by) of disp_a, disp_b,
-    # update, post_mask_break, maskmul, then the x and y flux tile heights
+    # update, post_mask_break, maskmul, then the x and y flux heights
     TUNE_LEN = 14
     TUNE_NAMES = ("disp_a", "disp_b", "update", "post_mask_break", "maskmul")
 
@@ -496,8 +496,8 @@ class Solver:
         return self.tuning()
 
     def tuning(self):
-        """{kernel: (bx, by)} of the per-cell kernels plus "flux_x"/"flux_y"
-        tile heights."""
+        """{kernel: (bx, by)} of the per-cell kernels plus the "flux_x" and
+        "flux_y" heights."""
         t = (ctypes.c_int * self.TUNE_LEN)()
         self._check(self.L.fw_get_tuning(self.ctx, t), "fw_get_tuning")
         out = {n: (t[2 * k], t[2 * k + 1]) for k, n in enumerate(self.TUNE_NAMES)}
@@ -511,7 +511,7 @@ class Solver:
         for k, n in enumerate(self.TUNE_NAMES):
             t[2 * k], t[2 * k + 1] = tuning[n]
         t[10], t[11] = tuning["flux_x"], tuning["flux_y"]
-        # TMA staging of the flux tiles; 0 (each thread loads) when not given
+        # fluxes by TMA-staged tiles; 0 (by lines and strips) when not given
         t[12], t[13] = tuning.get("flux_x_tma", 0), tuning.get("flux_y_tma", 0)
         self._check(self.L.fw_set_tuning(self.ctx, t), "fw_set_tuning")
 
