@@ -329,9 +329,11 @@ template <typename T> void dispatch_stage(fw_ctx *c, int istage) { launch_stage<
 
 // one whole step on the stream (main.F:284-535 minus OUTPUT)
 template <typename T> void enqueue_step(fw_ctx *c) {
+    c->whole_step = true;
     launch_begin_step<T>(c);
     for (int s = 1; s <= 3; s++) launch_stage<T>(c, s);
     launch_end_step<T>(c);
+    c->whole_step = false;
 }
 
 int check_ready(fw_ctx *c) {
@@ -777,11 +779,11 @@ int fw_init(fw_ctx *c, const double *depth, const double *eta, const double *u, 
         const bool d = c->p.precision == FW_PREC_FP64;
         const size_t es = d ? sizeof(double) : sizeof(float);
         const size_t mf = c->p.nfreq, mt = c->p.ntheta;
-        const size_t nb = (size_t)bw * bh * mf * es;
+        const size_t nb = (size_t)bw * bh * mf * es, nwm = (size_t)bw * bh * es;  // (wm_band behind Cm)
         void *Cm = nullptr, *Sm = nullptr;
         double *tab = nullptr;
         const size_t ntab = 3 * mf * mt + mf;
-        if (cudaMalloc(&Cm, nb) != cudaSuccess || cudaMalloc(&Sm, nb) != cudaSuccess ||
+        if (cudaMalloc(&Cm, nb + nwm) != cudaSuccess || cudaMalloc(&Sm, nb) != cudaSuccess ||
             cudaMalloc(&tab, ntab * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
             if (Cm) cudaFree(Cm);
@@ -1533,7 +1535,8 @@ int fw_restore(fw_ctx *c, const char *path) {
     // band tables: (re)allocate to the saved size
     void *nb[2] = {nullptr, nullptr};
     if (h.band_bytes) {
-        if (cudaMalloc(&nb[0], h.band_bytes) != cudaSuccess || cudaMalloc(&nb[1], h.band_bytes) != cudaSuccess) {
+        // (wm_band behind Cm)
+        if (cudaMalloc(&nb[0], h.band_bytes + h.band_bytes / c->p.nfreq) != cudaSuccess || cudaMalloc(&nb[1], h.band_bytes) != cudaSuccess) {
             cudaGetLastError();
             if (nb[0]) cudaFree(nb[0]);
             return FW_ERR_OOM;

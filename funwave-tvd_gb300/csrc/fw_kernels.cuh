@@ -1268,6 +1268,22 @@ __device__ __forceinline__ T wavemaker_mass(const Grid &g, const Fields<T> &f, i
     return (T)0;
 }
 
+// The JON_2D mass depends on TIME, which stays through a step's three stages: a
+// whole step sums the band's frequencies once, beside the first stage's
+// dispersion, into the words behind Cm.  Summed in every stage's k_update, the
+// warps of the band kept the others waiting (k_update at 2048 x 2048 128 ->
+// 112 us, 1024 x 1024 50 -> 37).
+template <typename T> __host__ __device__ __forceinline__ T *wm_band(const Grid &g, const Fields<T> &f) {
+    return f.Cm + (size_t)g.nfreq * (size_t)(g.ihi - g.ilo + 1) * (size_t)(g.jhi - g.jlo + 1);
+}
+template <typename T> __global__ void __launch_bounds__(256) k_wm_band(Grid g, Fields<T> f) {
+    const int bw = g.ihi - g.ilo + 1, n = bw * (g.jhi - g.jlo + 1);
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= n) return;
+    const int j = b / bw, i = b - j * bw;
+    wm_band(g, f)[b] = wavemaker_mass(g, f, g.ilo + i, g.jlo + j, f.dsc[S_TIME]);
+}
+
 // SourceTerms at one cell; BX, BY get BreakSourceX/Y (sources.F:428-456),
 // zero without viscosity breaking
 template <typename T>
@@ -1369,9 +1385,10 @@ __global__ void __launch_bounds__(256) k_sources(Grid g, Fields<T> f) {
 // GET_Eta_U_V_HU_HV (etauv_solver.F:365-539).  RAD (the last two stages,
 // with the radiation sums on) also stores P_center, Q_center, U_davg, V_davg
 // with the stage's starting H (etauv_solver.F:94-101), Wsurf = R1
-// (etauv_solver.F:247) and BreakSourceX/Y.
+// (etauv_solver.F:247) and BreakSourceX/Y.  BAND: the wavemaker's mass comes from
+// k_wm_band.
 // ---------------------------------------------------------------------------
-template <typename T, bool RAD = false>
+template <typename T, bool RAD, bool BAND>
 __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_update(Grid g, Fields<T> f, T al, T be, Ahead ah) {
     prefetch_ahead<T>(g, ah, blockIdx.y, 0);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1399,8 +1416,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == sizeof(float) ? 4 : 3) k_upd
     }
     const T DX = GC(DX), DY = GC(DY);
     const T DT = DTV;
-    const double TIME = f.dsc[S_TIME];
-    const T wm = wavemaker_mass(g, f, i, j, TIME);
+    T wm = (T)0;
+    if constexpr (BAND) {
+        if (i >= g.ilo && i <= g.ihi && j >= g.jlo && j <= g.jhi)
+            wm = ro(wm_band(g, f) + (i - g.ilo) + (j - g.jlo) * (g.ihi - g.ilo + 1));
+    } else {
+        wm = wavemaker_mass(g, f, i, j, f.dsc[S_TIME]);
+    }
     T SX, SY, BX, BY;
     source_terms_b(g, f, i, j, wm, SX, SY, BX, BY);
 
@@ -4668,12 +4690,17 @@ template <typename T> static void launch_disp_a(fw_ctx *c) {
     k_disp_a<T><<<gr, b, 0, c->stream>>>(
         g, f, ahead_of<T>(g, b, gr.x, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.Depth, f.Eta, f.P, f.Q}));
 }
+// whether this step's launches leave the wavemaker's mass to k_wm_band
+template <typename T> static bool wm_in_band(fw_ctx *c) {
+    return c->whole_step && c->g.wavemaker == FW_WK_JON_2D && c->F<T>().Cm != nullptr;
+}
 template <typename T, bool RAD> static void launch_update(fw_ctx *c, T al, T be) {
     const Grid &g = c->g;
     const Fields<T> &f = c->F<T>();
     const dim3 b = c->blk(TK_UPDATE);
     const dim3 gr = grid2(g.Mloc, g.Nloc, b);
-    k_update<T, RAD><<<gr, b, 0, c->stream>>>(
+    auto kern = wm_in_band<T>(c) ? k_update<T, RAD, true> : k_update<T, RAD, false>;
+    kern<<<gr, b, 0, c->stream>>>(
         g, f, al, be,
         ahead_of<T>(g, b, gr.x, AHEAD_UPDATE, 2 * 152, {f.Eta0, f.Ubar0, f.Vbar0, f.Eta, f.Ubar, f.Vbar, f.P, f.Q, f.Fx, f.Fy, f.Gx, f.Gy,
                                               f.Depth, f.H, f.U, f.V, f.U4, f.V4, f.Depthx, f.Depthy, f.Udisp, f.Vdisp, f.U1p,
@@ -4743,8 +4770,23 @@ template <typename T> void launch_estimate_dt(fw_ctx *c) {
 
 template <typename T> void launch_begin_step(fw_ctx *c) {
     const Grid &g = c->g;
+    const bool branch = branching(c);
+    // the time step's end, which the first stage waits for before its first use
+    // (join_ev), and the wavemaker's mass
+    auto dt_final = [&] {
+        launch_dt_final(c);
+        if (branch) {
+            const cudaError_t e = cudaEventRecord(c->join_ev, c->stream);
+            if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
+        }
+        if (wm_in_band<T>(c)) {
+            const int n = (g.ihi - g.ilo + 1) * (g.jhi - g.jlo + 1);
+            k_wm_band<T><<<(n + 255) / 256, 256, 0, c->stream>>>(g, c->F<T>());
+            note(c);
+        }
+    };
     if (launch_exchange_one<T, true>(c, false, B2D)) {
-        on_side(c, branching(c), [&] { launch_dt_final(c); });  // joined by the first stage
+        on_side(c, branch, dt_final);
         return;
     }
     const int nring = 6 * g.Mloc + 6 * g.Nglob;
@@ -4753,7 +4795,7 @@ template <typename T> void launch_begin_step(fw_ctx *c) {
     launch_ghost<T>(c, g.visc_breaking != 0);
     k_begin<T><<<grid2(g.Mloc, g.Nloc, B2D), B2D, 0, c->stream>>>(g, c->F<T>());
     note(c);
-    on_side(c, branching(c), [&] { launch_dt_final(c); });
+    on_side(c, branch, dt_final);
 }
 
 template <typename T> static void launch_disp_b(fw_ctx *c) {
@@ -5136,26 +5178,14 @@ template <typename T> void launch_end_step(fw_ctx *c) {
 template <typename T> void launch_stage(fw_ctx *c, int istage) {
     const Grid &g = c->g;
     const bool branch = branching(c);
-    // the first stage joins the time step's end (on the side since the step
-    // began) before its first use
-    if (branch && kept_factors<T>(c)) {
-        if (istage == 1) {
-            const cudaError_t e = cudaEventRecord(c->join_ev, c->side);
-            if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
-        }
-        on_side(c, true, [&] { launch_factors<T>(c); });
-    }
+    if (branch && kept_factors<T>(c)) on_side(c, true, [&] { launch_factors<T>(c); });
     if (g.dispersion) {
         launch_disp_a<T>(c);
         note(c);
     }
     if (branch && istage == 1) {
-        if (kept_factors<T>(c)) {
-            const cudaError_t e = cudaStreamWaitEvent(c->stream, c->join_ev, 0);
-            if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
-        } else {
-            join_side(c, true);
-        }
+        const cudaError_t e = cudaStreamWaitEvent(c->stream, c->join_ev, 0);
+        if (e != cudaSuccess && !c->sticky_error) c->sticky_error = (int)e;
     }
     if (g.dispersion) launch_disp_b<T>(c);
     launch_fluxes_opt<T>(c, branch);

@@ -43,3 +43,30 @@ def test_branches_equal_one_stream(fw, size, precision, mode):
     for n, a in got[0].items():
         assert np.array_equal(a, got[1][n]), n
     assert np.isfinite(got[0]["Eta"]).all()
+
+
+@pytest.mark.parametrize("precision", ["MIXED", "FP64"])
+@pytest.mark.parametrize("shape", [(200, 24, 60.0), (331, 67, 90.0)])
+def test_wavemaker_band_equals_inline(fw, shape, precision):
+    """JON_2D: whole steps take the wavemaker's mass from a kernel of its own
+    over the band, single parts sum it in each cell."""
+    M, N, shore = shape
+    p, depth, phases, _ = fw.cases.barred_beach(M, N, 1.0, seed=3, wk_from_shore=shore)
+    p = fw.with_defaults(p)
+    got = []
+    for captured in (True, False):
+        s = fw.Solver(p, precision=precision)
+        s.init(depth, phases=phases)
+        if captured:
+            assert s.step(7) == 0
+        else:
+            for _ in range(7):
+                s.begin_step()
+                for k in (1, 2, 3):
+                    s.stage(k)
+                s.end_step()
+        got.append({n: s.get(n) for n in FIELDS})
+        s.close()
+    for n, a in got[0].items():
+        assert np.array_equal(a, got[1][n]), n
+    assert np.abs(got[0]["Eta"]).max() > 0
