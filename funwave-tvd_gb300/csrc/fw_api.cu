@@ -496,18 +496,38 @@ cudaError_t clear_arena(fw_ctx *c) {
     return e;
 }
 
-int read_status(fw_ctx *c, int *status) {
-    unsigned long long bits = 0;
-    cudaError_t e = cudaMemcpyAsync(&bits, etamax_ptr(c), sizeof(bits), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+// the step maximum on its way to the context's page-locked word, behind the
+// stream's work (a copy to pageable memory passes a staging buffer and holds
+// the host; 16 runs of an ensemble, whose copies now queue before the first
+// wait: 7.59 -> 7.45 ms for four steps)
+int queue_status(fw_ctx *c) {
+    return cuda_status(c, cudaMemcpyAsync(c->max_host, etamax_ptr(c), sizeof(*c->max_host), cudaMemcpyDeviceToHost, c->stream));
+}
+int take_status(fw_ctx *c, int *status) {
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_status(c, e);
     double mx;
-    std::memcpy(&mx, &bits, sizeof(mx));
+    std::memcpy(&mx, c->max_host, sizeof(mx));
     int st = FW_OK;
     if (!(mx == mx) || std::isinf(mx)) st = FW_ERR_NAN;
     else if (mx > c->EtaBlowVal) st = FW_ERR_BLOWUP;
     if (status) *status = st;
     return FW_OK;
+}
+int read_status(fw_ctx *c, int *status) {
+    const int rc = queue_status(c);
+    return rc == FW_OK ? take_status(c, status) : rc;
+}
+// the same for n contexts, whose copies are all queued before the first wait
+int read_statuses(fw_ctx *const *ctx, int n, int *status) {
+    int first = FW_OK;
+    std::vector<int> rcs(n);
+    for (int k = 0; k < n; k++) rcs[k] = queue_status(ctx[k]);
+    for (int k = 0; k < n; k++) {
+        const int rc = rcs[k] == FW_OK ? take_status(ctx[k], status ? &status[k] : nullptr) : rcs[k];
+        if (rc != FW_OK && first == FW_OK) first = rc;
+    }
+    return first;
 }
 
 }  // namespace
@@ -676,7 +696,8 @@ int fw_create(const fw_params *p, fw_ctx **out) {
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming) != cudaSuccess ||
+        cudaMallocHost(&c->max_host, sizeof(*c->max_host)) != cudaSuccess) {
         cudaGetLastError();
         fw_destroy(c);
         return FW_ERR_CUDA;
@@ -725,6 +746,7 @@ int fw_destroy(fw_ctx *c) {
     if (c->fork_ev) cudaEventDestroy(c->fork_ev);
     if (c->join_ev) cudaEventDestroy(c->join_ev);
     if (c->side) cudaStreamDestroy(c->side);
+    if (c->max_host) cudaFreeHost(c->max_host);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return FW_OK;
@@ -1153,12 +1175,7 @@ int fw_ensemble_step(fw_ctx *const *ctxs, int n, int nsteps, int *status) {
             if (rc != FW_OK) return rc;
         }
     }
-    int first = FW_OK;
-    for (int k = 0; k < n; k++) {
-        const int rc = read_status(ctxs[k], status ? &status[k] : nullptr);
-        if (rc != FW_OK && first == FW_OK) first = rc;
-    }
-    return first;
+    return read_statuses(ctxs, n, status);
 }
 
 }  // extern "C"
@@ -1302,12 +1319,7 @@ int fw_ensemble_run(fw_ensemble *e, int nsteps, int *status) {
             if (rc != FW_OK) return rc;
         }
     }
-    int first = FW_OK;
-    for (int k = 0; k < n; k++) {
-        const int rc = read_status(e->ctx[k], status ? &status[k] : nullptr);
-        if (rc != FW_OK && first == FW_OK) first = rc;
-    }
-    return first;
+    return read_statuses(e->ctx.data(), n, status);
 }
 
 int fw_ensemble_destroy(fw_ensemble *e) {

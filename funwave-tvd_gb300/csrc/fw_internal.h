@@ -251,6 +251,7 @@ struct fw_ctx {
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     bool one_branch = false;  // the capture under way takes one branch only
     bool whole_step = false;  // the launches under way are of one whole step
+    unsigned long long *max_host = nullptr;  // page-locked: the step maximum as the host reads it
     // snapshots in out_buf, copied to the caller's buffers on out_stream
     void *out_buf = nullptr;
     size_t out_cap = 0;
