@@ -145,12 +145,12 @@ template <typename T> int get_field(fw_ctx *c, const FieldRef &r, void *host) {
     return cuda_status(c, e);
 }
 
-// a field that the FP64 line solver's kept factors depend on was set: factor
-// again at the next solve (the mixed factors follow MASK9's own changes)
+// a field that the line solver's kept factors depend on was set: factor again
+// at the next solve (UPDATE_MASK marks its own changes of MASK9 only)
 int refactor_after(fw_ctx *c, const char *name) {
-    if (c->p.precision != FW_PREC_FP64) return FW_OK;
     if (std::strcmp(name, "Depth") && std::strcmp(name, "MASK9") && std::strcmp(name, "MASK")) return FW_OK;
-    return cuda_status(c, cudaMemsetAsync(c->fd.m9_dirty, 1, sizeof(int), c->stream));
+    int *dirty = c->p.precision == FW_PREC_FP64 ? c->fd.m9_dirty : c->ff.m9_dirty;
+    return cuda_status(c, cudaMemsetAsync(dirty, 1, sizeof(int), c->stream));
 }
 
 int put_named(fw_ctx *c, const char *name, const void *host) {
@@ -167,7 +167,7 @@ int put_named(fw_ctx *c, const char *name, const void *host) {
         FieldRef rd{c->ff.DepthD, 0, 0};
         rc = put_field<double>(c, rd, host);
     }
-    return rc;
+    return rc == FW_OK ? refactor_after(c, name) : rc;
 }
 
 void fill_float_constants(Grid &g) {
@@ -1898,7 +1898,11 @@ int fw_set_fields_f32(fw_ctx *c, int n, const char *const *names, const float *c
         return FW_OK;
     }
     HostPlanes hp;
-    if (host_planes(c, n, names, (const void *const *)host, true, hp)) return host_planes_run(c, n, hp, true);
+    if (host_planes(c, n, names, (const void *const *)host, true, hp)) {
+        int rc = host_planes_run(c, n, hp, true);
+        for (int k = 0; k < n && rc == FW_OK; k++) rc = refactor_after(c, names[k]);
+        return rc;
+    }
     std::vector<FieldRef> refs;
     std::vector<size_t> off;
     int rc = f32_planes(c, n, names, refs, off);
@@ -1919,6 +1923,7 @@ int fw_set_fields_f32(fw_ctx *c, int n, const char *const *names, const float *c
         // the double Depth of the total-depth tests, widened from the floats
         if (e == cudaSuccess && std::strcmp(names[k], "Depth") == 0)
             convert_in_f32(c, (const float *)(buf + off[k]), c->ff.DepthD, w, h);
+        if (e == cudaSuccess && (rc = refactor_after(c, names[k])) != FW_OK) return rc;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_status(c, e);

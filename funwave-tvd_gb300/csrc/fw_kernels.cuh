@@ -2257,8 +2257,9 @@ __global__ void __launch_bounds__(PER ? 32 * THS_WARPS : 32) k_thomas_solve(Grid
 
 // Mixed path: the tridiagonal matrices depend on Depth and MASK9 only, so
 // their partitioned factorisation is computed (in double) when MASK9 has
-// changed - never again once viscosity breaking has set MASK9 = 1 on the
-// ring - and stored rounded to float.  Each stage then solves in float and
+// changed or one of them was set - never again in a run with viscosity
+// breaking once that has set MASK9 = 1 on the ring - and stored rounded to
+// float.  Each stage then solves in float and
 // refines once: x0 = S(d), r = d - T x0 with a compensated (float-pair)
 // residual, x = x0 + S(r).  S is the partitioned substitution: per chunk of
 // m rows a forward/backward sweep, a reduced system of two rows per chunk,
