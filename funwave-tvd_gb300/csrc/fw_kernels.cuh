@@ -4617,6 +4617,7 @@ __global__ void __launch_bounds__(256) k_end(Grid g, Fields<T> f, int track_hmax
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+constexpr int GRID_Y_MAX = 65535;  // blocks of a launch along y
 static inline dim3 grid2(int nx, int ny, dim3 b) { return dim3((nx + b.x - 1) / b.x, (ny + b.y - 1) / b.y); }
 static const dim3 B2D(32, 8);
 // blocks of k_flux_tma: tiles of FX x FY faces over (Mglob+1) x Nglob x-faces
@@ -4863,7 +4864,9 @@ template <typename T, int DIR> static void launch_flux(fw_ctx *c) {
     const Grid &g = c->g;
     const dim3 b(32, 4);
     if (DIR == 0) {
-        const int rows = std::max(1, fy / 8), nx = (g.ie + FLUX_XW) / FLUX_XW;
+        // (more rows where the grid's blocks along y would pass the launch limit)
+        const int rows = std::max({1, fy / 8, (g.Nglob + 4 * GRID_Y_MAX - 1) / (4 * GRID_Y_MAX)});
+        const int nx = (g.ie + FLUX_XW) / FLUX_XW;
         k_flux_x<T><<<dim3(nx, (g.Nglob + 4 * rows - 1) / (4 * rows)), b, 0, c->stream>>>(g, c->F<T>(), rows);
     } else {
         const int nx = (g.ie + 32) / 32, strip = flux_strip(nx, g.Nglob + 1, sizeof(T) == sizeof(double) ? 2 * fy : fy, sizeof(T) == sizeof(double));
