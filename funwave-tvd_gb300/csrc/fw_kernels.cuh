@@ -4717,7 +4717,8 @@ template <typename T> static void launch_pmb(fw_ctx *c) {
         g, f, ahead_of<T>(g, b, gr.x, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.H, f.AGE, f.Eta, f.Depth, f.ETAT}));
 }
 
-// EXCHANGE in one launch; false for grids too small for it
+// EXCHANGE in one launch; false for grids too small for it, and for those
+// whose rows of blocks and P's and Q's on top of them pass the launch limit
 template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, bool sponge, dim3 b) {
     const Grid &g = c->g;
     if (g.Mglob < 3 || g.Nglob < 3) return false;
@@ -4728,6 +4729,7 @@ template <typename T, bool BEGIN> static bool launch_exchange_one(fw_ctx *c, boo
         const int n = 6 * g.Nglob + 6 * (g.Mloc + 1) + 6 * (g.Nglob + 1) + 6 * g.Mloc, per = (int)(b.x * b.y * gr.x);
         gr.y += (n + per - 1) / per;
     }
+    if (gr.y > GRID_Y_MAX) return false;
     const Fields<T> &f = c->F<T>();
     const Ahead ah = BEGIN ? ahead_of<T>(g, b, gr.x, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta, f.H, f.Ubar, f.Vbar})
                            : ahead_of<T>(g, b, gr.x, AHEAD_EXCHANGE, 4 * 152, {f.U, f.V, f.HU, f.HV, f.Eta});

@@ -12,7 +12,7 @@ from helpers import G, make_pair, maxrel
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [262200])
+@pytest.mark.parametrize("rows", [262200, 400000])
 def test_a_step_of_a_very_long_grid(fw, oracle_mod, rows):
     M = 4
     rng = np.random.default_rng(rows)
