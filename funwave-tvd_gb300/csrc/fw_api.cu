@@ -715,7 +715,8 @@ int fw_create(const fw_params *p, fw_ctx **out) {
     // the load-based kernels run
     c->fmaps_ok = (fp64 ? build_flux_maps<double>(c) : build_flux_maps<float>(c)) ? 1 : 0;
     cudaGetLastError();
-    cudaError_t e = clear_arena(c);
+    const bool attrs = fp64 ? fw::linesolve_attrs<double>() : fw::linesolve_attrs<float>();
+    cudaError_t e = attrs ? clear_arena(c) : cudaErrorUnknown;
     if (e != cudaSuccess) {
         cudaGetLastError();
         fw_destroy(c);

@@ -165,6 +165,7 @@ template <typename T>
 void launch_cm_sm(fw_ctx *c, int bw, int bh, int i0, int j0, const double *tab, T *Cm, T *Sm);
 template <typename T> int launch_by_name(fw_ctx *c, const char *name);
 template <typename T> bool flux_tma_attrs();  // shared-memory sizes of the TMA-staged flux kernels
+template <typename T> bool linesolve_attrs();  // and of the mixed line solves
 // staging buffer <-> field (double <-> float fields, int32 <-> uint8 masks)
 void convert_in(fw_ctx *c, const void *staging, int is_mask, void *field, int w, int h);
 void convert_out(fw_ctx *c, const void *field, int is_mask, void *staging, int w, int h);

@@ -4923,6 +4923,26 @@ static LsfShape lsf_shape(int dir, const Grid &g, const LinePart &lp) {
     return S;
 }
 
+// The line solves' limits of shared memory.  A limit belongs to the kernel in
+// this process, whatever context launches it: each is set once, when a context
+// is made, to the most that any line asks for (lsf_smem_floats over all line
+// lengths and counts: 62500 bytes, for x lines of 4096 rows; y 45312), and
+// never to one context's own need, which would fail the launches of others.
+constexpr size_t LSF_SMEM_MAX = 64 * 1024, LSX_SMEM_MAX = 200 * 1024;
+template <typename T, int DIR, bool PER> static bool linesolve_attr() {
+    return cudaFuncSetAttribute(k_linesolve<T, DIR, PER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)LSF_SMEM_MAX) == cudaSuccess &&
+           cudaFuncSetAttribute(k_linesolve<T, DIR, PER, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)LSF_SMEM_MAX) == cudaSuccess;
+}
+template <typename T> bool linesolve_attrs() {
+    if constexpr (sizeof(T) == sizeof(float))
+        return linesolve_attr<T, 0, false>() && linesolve_attr<T, 1, false>() && linesolve_attr<T, 1, true>() &&
+               cudaFuncSetAttribute(k_linesolve_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)LSX_SMEM_MAX) == cudaSuccess;
+    return true;
+}
+
 template <typename T, int DIR, bool PER>
 static void launch_linesolve(fw_ctx *c, const LinePart &lp, bool clear_dirty) {
     const LsfShape S = lsf_shape(DIR, c->g, lp);
@@ -4938,8 +4958,6 @@ static void launch_linesolve(fw_ctx *c, const LinePart &lp, bool clear_dirty) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = S.nc > 1 ? 1 : 0;
-    if (cfg.dynamicSmemBytes > 48 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
     cudaLaunchKernelEx(&cfg, kern, c->g, c->F<T>(), lp, S, clear_dirty ? 1 : 0);
     note(c);
 }
@@ -4975,8 +4993,7 @@ static bool launch_tri(fw_ctx *c, const LinePart &lp, bool fac = true, bool clea
         }
         // lines of more than 4096 rows
         const size_t smem = lsx_smem_floats(lp.L, lp.P) * sizeof(float);
-        if (DIR == 0 && !PER && lp.P <= 256 && smem <= 200 * 1024) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(k_linesolve_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (DIR == 0 && !PER && lp.P <= 256 && smem <= LSX_SMEM_MAX) {
             k_linesolve_x<T><<<lp.nlines, 256, smem, c->stream>>>(g, c->F<T>(), lp, clear_dirty ? 1 : 0);
             note(c);
             return clear_dirty;
@@ -5338,6 +5355,7 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     template void launch_stage<T>(fw_ctx *, int);     \
     template void launch_cm_sm<T>(fw_ctx *, int, int, int, int, const double *, T *, T *); \
     template int launch_by_name<T>(fw_ctx *, const char *);      \
-    template bool flux_tma_attrs<T>();
+    template bool flux_tma_attrs<T>();                           \
+    template bool linesolve_attrs<T>();
 
 }  // namespace fw
