@@ -4643,11 +4643,14 @@ static inline void note(fw_ctx *c, int n = 1) {
 // second fills the first one's last wave (a step of 128 x 256 cells 174 -> 143
 // us, 250 x 500 194 -> 152, 2048 x 2048 2134 -> 2081; 250 x 500 in double 3186
 // -> 3063, 701 x 937 11.0 -> 10.8 ms).
-// Outside a capture (the entry points of single parts) everything stays on the
-// context's stream, in the order of the step.
+// Everything else stays on the context's stream, in the order of the step: a
+// step outside a capture, and the entry points of single parts, any of which
+// a caller may capture alone; such a capture must end with nothing on another
+// stream and wait for nothing from outside it.
 static bool branching(fw_ctx *c) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    return !c->one_branch && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusActive;
+    return c->whole_step && !c->one_branch && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess &&
+           st == cudaStreamCaptureStatusActive;
 }
 // what `to` runs from here on comes after what `from` has so far
 static void branch_after(fw_ctx *c, cudaStream_t to, cudaStream_t from, cudaEvent_t ev) {
