@@ -1930,10 +1930,12 @@ __global__ void __launch_bounds__(32) k_thomas_fac(Grid g, Fields<T> f, LinePart
 }
 
 // the planes of 1/a and of d/a: each direction its own, so that both can be
-// solved at once (y: its right-hand side's place)
+// solved at once, and neither in its right-hand side's place, so that a solve
+// can be repeated.  (Vyy: read by k_disp_b alone, which has run by then, and
+// written anew before it runs again.)
 template <typename T, int DIR> __device__ __forceinline__ double *tf_ra(const Fields<T> &f) { return DIR == 0 ? f.tc : f.tp; }
 template <typename T, int DIR> __device__ __forceinline__ double *tf_d(const Fields<T> &f) {
-    return DIR == 0 ? f.ty : reinterpret_cast<double *>(f.rhs_y);
+    return DIR == 0 ? f.ty : reinterpret_cast<double *>(f.Vyy);
 }
 // d/a (or d) and 1/a (or 0) of every row, as k_thomas_rows
 template <typename T, int DIR, bool PER>
