@@ -303,7 +303,7 @@ template <typename T> size_t carve(fw_ctx *c, char *base, bool assign) {
     f.dtmin_bits = (unsigned long long *)take(sizeof(unsigned long long));
     f.etamax_bits = (unsigned long long *)take(sizeof(unsigned long long));
     f.ncand = (int *)take(sizeof(int));
-    f.cand = (int *)take((size_t)c->ncand_cap * sizeof(int));
+    f.cand = (int *)take((size_t)fw::cand_cap(g) * sizeof(int));
     const int nf = c->p.wavemaker == FW_WK_JON_2D ? (c->p.nfreq > 0 ? c->p.nfreq : 1) : 1;
     f.omega = (double *)take((size_t)nf * sizeof(double));
     f.wmcs = (double *)take((size_t)nf * 2 * sizeof(double));
@@ -687,7 +687,6 @@ int fw_create(const fw_params *p, fw_ctx **out) {
     c->py.red0 = (long long)c->px.nlines * 2 * c->px.P * 6;
     c->px.pcr0 = 0;
     c->py.pcr0 = fw::lsf_line(c->px) ? (long long)c->px.nlines * fw::pcr_words(c->px) : 0;
-    c->ncand_cap = (p->Mglob + 2) * (p->Nglob + 2);
     // the factored solve assumes tmp2 = 1 + Gamma1*MASK9*(-b1-2*b2)/h^2*dep^2
     // never vanishes, which holds for -b1-2*b2 >= 0 (Beta_ref in [-2, 0])
     c->factored = (p->precision == FW_PREC_MIXED) && (-g.b1 - 2.0 * g.b2 >= 0.0) ? 1 : 0;
@@ -2013,6 +2012,8 @@ int fw_time_kernel(fw_ctx *c, const char *name, int nrep, double *ms_per_launch)
     if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, a, b);
     cudaEventDestroy(a);
     cudaEventDestroy(b);
+    // the breaking candidates of the launches: their sweep does not follow
+    if (e == cudaSuccess) e = cudaMemsetAsync(fp64 ? c->fd.ncand : c->ff.ncand, 0, sizeof(int), c->stream);
     if (e != cudaSuccess) return cuda_status(c, e);
     *ms_per_launch = (double)ms / nrep;
     return finish(c);

@@ -192,6 +192,9 @@ __host__ __device__ __forceinline__ int pcr_words(const LinePart &lp) {
     const int n = 2 * lp.P;
     return (2 * pcr_steps(n) + 1) * ((n + 3) & ~3);
 }
+// places of the breaking sweep's candidate list: the cells that can be one
+// (Ibeg-1..Iend+1 x Jbeg-1..Jend+1)
+__host__ __device__ __forceinline__ int cand_cap(const Grid &g) { return (g.Mglob + 2) * (g.Nglob + 2); }
 // tensor maps of the flux kernels' TMA-staged tiles: U V HU HV Eta U4 V4 and
 // MASK, for one direction and tile height (the box shape is part of a map)
 // and one of the two MASK buffers
@@ -227,7 +230,6 @@ struct fw_ctx {
     void *arena = nullptr;       // one device allocation holds every field
     void *staging = nullptr;     // one host-layout plane for field transfers
     size_t arena_bytes = 0;
-    int ncand_cap = 0;
     long long launches = 0;
     int initialized = 0;
     int sticky_error = 0;        // first CUDA error seen by a launcher

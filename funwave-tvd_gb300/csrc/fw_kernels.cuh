@@ -3516,6 +3516,14 @@ template <typename T> __device__ __forceinline__ bool breaking_now(const Grid &g
     return age > (T)0 && age < GC(T_brk) && b.et > b.tmp2;
 }
 
+// A stage adds a cell at most once, and its sweep empties the list.  Launched
+// again without the sweep (fw_time_kernel, fw_autotune) cells come again; those
+// past the list's end are left out.
+template <typename T> __device__ __forceinline__ void add_cand(const Grid &g, const Fields<T> &f, int id) {
+    const unsigned slot = (unsigned)atomicAdd(f.ncand, 1);
+    if (slot < (unsigned)cand_cap(g)) f.cand[slot] = id;
+}
+
 template <typename T>
 __device__ __forceinline__ void break_cell(const Grid &g, const Fields<T> &f, int i, int j) {
     const int id = IDI(i, j);
@@ -3533,10 +3541,7 @@ __device__ __forceinline__ void break_cell(const Grid &g, const Fields<T> &f, in
     else if (b.et >= b.tmp2) cand = true;
     f.AGEn[id] = an;
     const bool zone = in_wk_zone<T>(g, i, j);
-    if (cand) {
-        const int slot = atomicAdd(f.ncand, 1);
-        f.cand[slot] = i + j * g.pitch;
-    }
+    if (cand) add_cand(g, f, id);
     if (zone || !cand) f.nu[id] = nu_value(g, f, id, b, an, zone);
     if (g.track_roller && !zone && !cand && breaking_now(g, b, an)) roller_cell(g, f, id, b.et);
 }
@@ -3604,10 +3609,7 @@ __global__ void __launch_bounds__(256) k_post_mask_break(Grid g, Fields<T> f, Ah
             else if (b.et >= b.tmp2) cand = true;
             f.AGEn[id] = an;
             const bool zone = in_wk_zone<T>(g, i, j);
-            if (cand) {
-                const int slot = atomicAdd(f.ncand, 1);
-                f.cand[slot] = id;
-            }
+            if (cand) add_cand(g, f, id);
             if (zone || !cand) f.nu[id] = nu_of(g, b, an, zone, dep, eta);
             if (g.track_roller && !zone && !cand && breaking_now(g, b, an)) roller_cell(g, f, id, b.et);
             // UPDATE_MASK (mask_cell; wet cells beside it: no depth reset)
@@ -3739,7 +3741,7 @@ __global__ void __launch_bounds__(1024) k_break_b(Grid g, Fields<T> f) {
     __shared__ int wsum[32];
     __shared__ int lev_beg[1024], lev_end[1024];
     __shared__ unsigned nonempty[32];
-    const int n = *f.ncand;
+    const int n = (int)min((unsigned)*f.ncand, (unsigned)cand_cap(g));
     const T DT = DTV;
     volatile T *N = f.AGEn;
     bool done = false;

@@ -27,3 +27,29 @@ def test_solving_again_gives_the_same(fw, name, field, precision, periodic):
     assert np.array_equal(s.get(field), a)
     assert np.abs(a).max() > 0
     s.close()
+
+
+@pytest.mark.parametrize("precision", ["MIXED", "FP64"])
+@pytest.mark.parametrize("name", ["post_mask_break", "break_a"])
+def test_breaking_candidates_do_not_pile_up(fw, name, precision):
+    """Every cell a candidate of the breaking sweep (0.35 sqrt(g H) <= ETAT <
+    0.65 sqrt(g H), AGE 0), launched 60 times without the sweep: the list
+    keeps to its place in memory, and the run goes on as after two launches."""
+    p, depth, phases, _ = fw.cases.barred_beach(200, 24, 1.0, seed=3, wk_from_shore=60.0)
+    depth = np.asfortranarray(np.full_like(depth, 1.0))
+    p = fw.with_defaults(p)
+    sea = fw.cases.random_state(*depth.shape, seed=6)
+    got = []
+    for reps in (1, 59):
+        s = fw.Solver(p, precision=precision)
+        s.init(depth, *sea, phases)
+        s.step(4)
+        s.set("ETAT", np.full(s.shape("ETAT"), 1.5))
+        s.set("AGE", np.zeros(s.shape("AGE")))
+        s.time_kernel(name, reps)
+        s.step(6)
+        got.append([s.get(n) for n in ("Eta", "U", "V", "AGE", "nu_break", "MASK")])
+        s.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+    assert np.abs(got[0][0]).max() > 0
