@@ -1201,7 +1201,7 @@ struct fw_ensemble {
     std::vector<cudaEvent_t> ready;  // one per run: its stream's earlier work
     cudaGraphExec_t exec = nullptr;
     std::vector<long long> states;   // swap_state of each run at capture
-    std::vector<std::array<int, FW_TUNE_LEN>> tunes;
+    std::vector<unsigned long long> epochs;  // and its epoch
 };
 
 namespace {
@@ -1209,8 +1209,7 @@ namespace {
 bool ens_stale(const fw_ensemble *e) {
     if (!e->exec) return true;
     for (size_t k = 0; k < e->ctx.size(); k++) {
-        if (e->states[k] != swap_state(e->ctx[k])) return true;
-        if (std::memcmp(e->tunes[k].data(), e->ctx[k]->tune, sizeof(e->ctx[k]->tune)) != 0) return true;
+        if (e->states[k] != swap_state(e->ctx[k]) || e->epochs[k] != e->ctx[k]->epoch) return true;
     }
     return false;
 }
@@ -1242,7 +1241,7 @@ int ens_build(fw_ensemble *e) {
         err = cudaGraphAddChildGraphNode(&node, parent, nullptr, 0, g);
         cudaGraphDestroy(g);
         e->states[k] = swap_state(c);
-        std::memcpy(e->tunes[k].data(), c->tune, sizeof(c->tune));
+        e->epochs[k] = c->epoch;
     }
     if (err == cudaSuccess) err = cudaGraphInstantiate(&e->exec, parent, 0);
     if (parent) cudaGraphDestroy(parent);
@@ -1269,7 +1268,7 @@ int fw_ensemble_create(fw_ctx *const *ctxs, int n, fw_ensemble **out) {
     if (!e) return FW_ERR_OOM;
     e->ctx.assign(ctxs, ctxs + n);
     e->states.assign(n, 0);
-    e->tunes.resize(n);
+    e->epochs.assign(n, 0);
     e->ready.assign(n, nullptr);
     bool ok = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&e->done, cudaEventDisableTiming) == cudaSuccess;

@@ -174,6 +174,7 @@ void convert_out_f32(fw_ctx *c, const double *field, float *staging, int w, int 
 
 }  // namespace fw
 
+#include <atomic>
 #include <cuda_runtime.h>
 
 // Host context behind the opaque C handle.
@@ -191,6 +192,11 @@ __host__ __device__ __forceinline__ int pcr_steps(int n) {
 __host__ __device__ __forceinline__ int pcr_words(const LinePart &lp) {
     const int n = 2 * lp.P;
     return (2 * pcr_steps(n) + 1) * ((n + 3) & ~3);
+}
+// values that no earlier call returned
+inline unsigned long long new_epoch() {
+    static std::atomic<unsigned long long> next{1};
+    return next++;
 }
 // places of the breaking sweep's candidate list: the cells that can be one
 // (Ibeg-1..Iend+1 x Jbeg-1..Jend+1)
@@ -247,14 +253,21 @@ struct fw_ctx {
     void *graph1_post[2][4] = {};
     int graph1_ok[2] = {0, 0};
     int graph1_next = 0;
-    void invalidate_graphs() { graph_ready = graph1_ok[0] = graph1_ok[1] = 0; }
-    // asynchronous output (fw_output_begin / fw_output_wait): host-layout
+    // what an ensemble's or a network's capture of this context's steps was
+    // made with: a new value whenever such a capture is out of date, and never
+    // the value of another context, at this address or another
+    unsigned long long epoch = fw::new_epoch();
+    void invalidate_graphs() {
+        graph_ready = graph1_ok[0] = graph1_ok[1] = 0;
+        epoch = fw::new_epoch();
+    }
     // the second branch of a captured step's graph
     cudaStream_t side = nullptr;
     cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
     bool one_branch = false;  // the capture under way takes one branch only
     bool whole_step = false;  // the launches under way are of one whole step
     unsigned long long *max_host = nullptr;  // page-locked: the step maximum as the host reads it
+    // asynchronous output (fw_output_begin / fw_output_wait): host-layout
     // snapshots in out_buf, copied to the caller's buffers on out_stream
     void *out_buf = nullptr;
     size_t out_cap = 0;

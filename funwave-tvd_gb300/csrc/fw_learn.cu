@@ -344,10 +344,13 @@ struct fw_net {
     // fw_correct_run's graph of two (step + correction) pairs and what it was
     // captured with
     cudaGraphExec_t cexec = nullptr;
-    fw_ctx *cctx = nullptr;
+    unsigned long long cepoch = 0;  // of the context
     long long cstate = 0;
-    int ctune[FW_TUNE_LEN] = {0};
     double cmax = 0.0;
+    void drop_graph() {
+        if (cexec) cudaGraphExecDestroy(cexec);
+        cexec = nullptr;
+    }
 };
 
 namespace {
@@ -701,22 +704,14 @@ int fw_net_create(unsigned long long seed, fw_net **out) {
 int fw_net_set_shore_band(fw_net *n, int cells) {
     if (!n || cells < 0 || cells > 3) return FW_ERR_BAD_PARAM;
     n->shore_band = cells;
-    // fw_correct_run's graph holds the old band
-    if (n->cexec) {
-        cudaGraphExecDestroy(n->cexec);
-        n->cexec = nullptr;
-    }
+    n->drop_graph();  // it holds the old band
     return FW_OK;
 }
 
 int fw_net_set_wait_limit(fw_net *n, unsigned polls) {
     if (!n) return FW_ERR_BAD_PARAM;
     n->wait_limit = polls ? polls : fwtc::WAIT_LIMIT;
-    // fw_correct_run's graph holds the old limit
-    if (n->cexec) {
-        cudaGraphExecDestroy(n->cexec);
-        n->cexec = nullptr;
-    }
+    n->drop_graph();  // it holds the old limit
     return FW_OK;
 }
 
@@ -728,7 +723,6 @@ int fw_net_destroy(fw_net *n) {
         if (p) cudaFree(p);
     if (n->loss) cudaFree(n->loss);
     if (n->img) cudaFree(n->img);
-    if (n->cexec) cudaGraphExecDestroy(n->cexec);
     if (n->status) cudaFree(n->status);
     delete n;
     return FW_OK;
@@ -817,11 +811,9 @@ int fw_correct_run(fw_ctx *c, fw_net *n, int nsteps, double max_corr, int *statu
         return r;
     };
     for (int s2 = 0; s2 + 2 <= nsteps; s2 += 2) {
-        const bool stale = !n->cexec || n->cctx != c || n->cstate != fw::buffer_state(c) ||
-                           std::memcmp(n->ctune, c->tune, sizeof(n->ctune)) != 0 || n->cmax != max_corr;
+        const bool stale = !n->cexec || n->cepoch != c->epoch || n->cstate != fw::buffer_state(c) || n->cmax != max_corr;
         if (stale) {
-            if (n->cexec) cudaGraphExecDestroy(n->cexec);
-            n->cexec = nullptr;
+            n->drop_graph();
             const long long st = fw::buffer_state(c);
             cudaGraph_t gr;
             if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -843,9 +835,8 @@ int fw_correct_run(fw_ctx *c, fw_net *n, int nsteps, double max_corr, int *statu
                 n->cexec = nullptr;
                 return FW_ERR_CUDA;
             }
-            n->cctx = c;
+            n->cepoch = c->epoch;
             n->cstate = st;
-            std::memcpy(n->ctune, c->tune, sizeof(n->ctune));
             n->cmax = max_corr;
         }
         if (cudaGraphLaunch(n->cexec, c->stream) != cudaSuccess) {
