@@ -362,6 +362,7 @@ constexpr int IMG_N[NL + 3] = {32, 32, 32, 16, 32, 32, 32};
 size_t img_elems(int i) { return (size_t)9 * IMG_CINC[i] * IMG_N[i] * 8; }
 
 void free_ws(fw_net *n) {
+    n->drop_graph();  // it holds these buffers
     for (auto &a : n->act) {
         if (a) cudaFree(a);
         a = nullptr;

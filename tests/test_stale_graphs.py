@@ -1,7 +1,7 @@
 """What an ensemble's or a network's captured graph was made with may change:
 a context is initialised again (new wavemaker tables), a scalar is set, the
-solver is another one.  The next run then gives what stepping gives, bit for
-bit."""
+solver is another one, the network's workspace grows.  The next run then
+gives what stepping gives, bit for bit."""
 import numpy as np
 import pytest
 
@@ -50,8 +50,9 @@ def test_ensemble_after_a_change(fw, what):
     e.close()
 
 
-@pytest.mark.parametrize("what", ["T_brk", "init", "other"])
+@pytest.mark.parametrize("what", ["T_brk", "init", "other", "workspace"])
 def test_correct_run_after_a_change(fw, what):
+    import torch
     p, d, ph = _case(fw, 1)
     net, ref = fw.learned.Net(seed=7), fw.learned.Net(seed=7)
     a, b = fw.Solver(p, precision="MIXED"), fw.Solver(p, precision="MIXED")
@@ -73,12 +74,15 @@ def test_correct_run_after_a_change(fw, what):
     elif what == "init":
         for s in (a, b):
             _init(fw, s, d, _case(fw, 9)[2], 4)
-    else:  # another solver, the same sizes, at the same addresses or not
+    elif what == "other":  # the same sizes, at the same addresses or not
         for s in (a, b):
             s.close()
         p, d, ph = _case(fw, 1, DX=1.25, DY=1.5)
         a = fw.Solver(p, precision="MIXED")
         _init(fw, a, d, ph, 5)
+    else:
+        net.forward(torch.zeros(2, 300, 400, 5, device="cuda"))
+        torch.cuda.synchronize()
     net.correct_run(a, 6)
     if what == "other":
         b = fw.Solver(p, precision="MIXED")
