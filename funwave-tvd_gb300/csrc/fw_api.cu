@@ -821,6 +821,7 @@ int fw_init(fw_ctx *c, const double *depth, const double *eta, const double *u, 
         std::copy(hc.jon_phases.begin(), hc.jon_phases.end(), h.begin() + 2 * mf * mt);
         std::copy(hc.jon_betagen.begin(), hc.jon_betagen.end(), h.begin() + 3 * mf * mt);
         rc = upload_array(c, tab, h.data(), ntab * sizeof(double));
+        if (rc == FW_OK) rc = cuda_status(c, cudaMemsetAsync((char *)Cm + nb, 0, nwm, c->stream));
         const int i0 = hc.ilo - (NG + 1), j0 = hc.jlo - (NG + 1);  // I-Ibeg, J-Jbeg of the band's first cell
         if (d) {
             c->fd.Cm = (double *)Cm;
@@ -1546,11 +1547,15 @@ int fw_restore(fw_ctx *c, const char *path) {
     // band tables: (re)allocate to the saved size
     void *nb[2] = {nullptr, nullptr};
     if (h.band_bytes) {
-        // (wm_band behind Cm)
-        if (cudaMalloc(&nb[0], h.band_bytes + h.band_bytes / c->p.nfreq) != cudaSuccess || cudaMalloc(&nb[1], h.band_bytes) != cudaSuccess) {
+        const size_t nwm = h.band_bytes / c->p.nfreq;  // (wm_band behind Cm)
+        if (cudaMalloc(&nb[0], h.band_bytes + nwm) != cudaSuccess || cudaMalloc(&nb[1], h.band_bytes) != cudaSuccess) {
             cudaGetLastError();
             if (nb[0]) cudaFree(nb[0]);
             return FW_ERR_OOM;
+        }
+        if ((e = cudaMemsetAsync((char *)nb[0] + h.band_bytes, 0, nwm, c->stream)) != cudaSuccess) {
+            for (void *b : nb) cudaFree(b);
+            return cuda_status(c, e);
         }
     }
     PinnedBuf pin(std::min(kCkChunk, std::max(h.arena_bytes, (uint64_t)1)));

@@ -1272,7 +1272,7 @@ __device__ __forceinline__ T wavemaker_mass(const Grid &g, const Fields<T> &f, i
 // whole step sums the band's frequencies once, beside the first stage's
 // dispersion, into the words behind Cm.  Summed in every stage's k_update, the
 // warps of the band kept the others waiting (k_update at 2048 x 2048 128 ->
-// 112 us, 1024 x 1024 50 -> 37).
+// 112 us, 1024 x 1024 50 -> 37).  The words are zero until a first whole step.
 template <typename T> __host__ __device__ __forceinline__ T *wm_band(const Grid &g, const Fields<T> &f) {
     return f.Cm + (size_t)g.nfreq * (size_t)(g.ihi - g.ilo + 1) * (size_t)(g.jhi - g.jlo + 1);
 }
@@ -4699,16 +4699,18 @@ template <typename T> static void launch_disp_a(fw_ctx *c) {
     k_disp_a<T><<<gr, b, 0, c->stream>>>(
         g, f, ahead_of<T>(g, b, gr.x, AHEAD_A_PMB, 2 * 152, {f.U, f.V, f.Depth, f.Eta, f.P, f.Q}));
 }
-// whether this step's launches leave the wavemaker's mass to k_wm_band
-template <typename T> static bool wm_in_band(fw_ctx *c) {
-    return c->whole_step && c->g.wavemaker == FW_WK_JON_2D && c->F<T>().Cm != nullptr;
+// whether whole steps leave the wavemaker's mass to k_wm_band, and whether the
+// launches under way are of one
+template <typename T> static bool wm_has_band(fw_ctx *c) {
+    return c->g.wavemaker == FW_WK_JON_2D && c->F<T>().Cm != nullptr;
 }
-template <typename T, bool RAD> static void launch_update(fw_ctx *c, T al, T be) {
+template <typename T> static bool wm_in_band(fw_ctx *c) { return c->whole_step && wm_has_band<T>(c); }
+template <typename T, bool RAD> static void launch_update(fw_ctx *c, T al, T be, bool band) {
     const Grid &g = c->g;
     const Fields<T> &f = c->F<T>();
     const dim3 b = c->blk(TK_UPDATE);
     const dim3 gr = grid2(g.Mloc, g.Nloc, b);
-    auto kern = wm_in_band<T>(c) ? k_update<T, RAD, true> : k_update<T, RAD, false>;
+    auto kern = band ? k_update<T, RAD, true> : k_update<T, RAD, false>;
     kern<<<gr, b, 0, c->stream>>>(
         g, f, al, be,
         ahead_of<T>(g, b, gr.x, AHEAD_UPDATE, 2 * 152, {f.Eta0, f.Ubar0, f.Vbar0, f.Eta, f.Ubar, f.Vbar, f.P, f.Q, f.Fx, f.Fy, f.Gx, f.Gy,
@@ -5085,9 +5087,9 @@ template <typename T> static void launch_estimate_huv_opt(fw_ctx *c, int istage,
     // previous exchange in the ghost corners (bc.F:735-740), so the last
     // stage's corners hold the second stage's values
     if (istage >= 2 && g.track_rad)
-        launch_update<T, true>(c, al, be);
+        launch_update<T, true>(c, al, be, wm_in_band<T>(c));
     else
-        launch_update<T, false>(c, al, be);
+        launch_update<T, false>(c, al, be, wm_in_band<T>(c));
     note(c);
     if (g.dispersion) {
         if (!branch && kept_factors<T>(c)) launch_factors<T>(c);
@@ -5326,7 +5328,7 @@ template <typename T> int launch_by_name(fw_ctx *c, const char *name) {
     else if (is("disp_b")) { launch_disp_b<T>(c); return 0; }
     else if (is("flux_x")) { launch_flux<T, 0>(c); return 0; }
     else if (is("flux_y")) { launch_flux<T, 1>(c); return 0; }
-    else if (is("update")) launch_update<T, false>(c, (T)0.75, (T)0.25);
+    else if (is("update")) launch_update<T, false>(c, (T)0.75, (T)0.25, wm_has_band<T>(c));  // as in a whole step
     else if (is("post_mask_break")) launch_pmb<T>(c);
     else if (is("tri_x")) { launch_tri<T, 0, false>(c, c->px); return 0; }
     else if (is("tri_y")) {

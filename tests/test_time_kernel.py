@@ -35,7 +35,7 @@ def test_breaking_candidates_do_not_pile_up(fw, name, precision):
     """Every cell a candidate of the breaking sweep (0.35 sqrt(g H) <= ETAT <
     0.65 sqrt(g H), AGE 0), launched 60 times without the sweep: the list
     keeps to its place in memory, and the run goes on as after two launches."""
-    p, depth, phases, _ = fw.cases.barred_beach(200, 24, 1.0, seed=3, wk_from_shore=60.0)
+    p, depth, phases, _ = fw.cases.barred_beach(200, 24, 1.0, seed=3, wk_from_shore=120.0, shore_from_east=40.0)
     depth = np.asfortranarray(np.full_like(depth, 1.0))
     p = fw.with_defaults(p)
     sea = fw.cases.random_state(*depth.shape, seed=6)
@@ -53,3 +53,21 @@ def test_breaking_candidates_do_not_pile_up(fw, name, precision):
     for a, b in zip(*got):
         assert np.array_equal(a, b)
     assert np.abs(got[0][0]).max() > 0
+
+
+@pytest.mark.parametrize("precision", ["MIXED", "FP64"])
+def test_update_is_timed_as_a_step_runs_it(fw, precision):
+    """JON_2D: a step takes the wavemaker's mass from k_wm_band, so k_update's
+    time does not grow with the frequencies (summed in every band cell, 4000 of
+    them take tens of times the kernel's few microseconds)."""
+    times = []
+    for nf in (2, 4000):
+        p, depth, phases, _ = fw.cases.barred_beach(200, 24, 1.0, seed=3, wk_from_shore=120.0, shore_from_east=40.0,
+                                                    nfreq=nf, ntheta=1)
+        s = fw.Solver(fw.with_defaults(p), precision=precision)
+        s.init(depth, phases=phases)
+        s.step(2)
+        assert 0 < s.scalar("ihi") - s.scalar("ilo") < 200
+        times.append(min(s.time_kernel("update", 20) for _ in range(3)))
+        s.close()
+    assert times[1] < 2.0 * times[0], times
