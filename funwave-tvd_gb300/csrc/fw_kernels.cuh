@@ -4920,9 +4920,8 @@ static LsfShape lsf_shape(int dir, const Grid &g, const LinePart &lp) {
         if (S.nc == 1)
             while (S.nline > 2 && (g.ie + S.nline) / S.nline < SMS) S.nline /= 2;
         S.nch = (PT + S.nc - 1) / S.nc;
-        // the last chunk and its remainder rows in the same block (P is then
-        // no multiple of nch; nch stays below 32 where it grows)
-        if (PT > lp.P && lp.P % S.nch == 0) S.nch++;
+        // (the last chunk and its remainder rows fall into the same block: with
+        // them, P is no multiple of nch for any length up to 4096)
         S.slots = S.nline / S.nc;
         S.nblk = (g.ie + S.nline) / S.nline * S.nc;  // columns 0 .. ie
     }
