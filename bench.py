@@ -64,12 +64,11 @@ KERNEL_BYTES = {
     "begin": lambda T: 8 * T + 1 + 9 * T,
 }
 # DRAM bytes per unit (dram__bytes_read.sum + dram__bytes_write.sum of one
-# ncu capture of the 2048 x 2048 mixed step, per launch / units; the tri_y
-# figure sums the partitioned y-solve kernels of one stage), taken with
-# the launch shapes pinned to the autotuner's choice
+# ncu capture of the 2048 x 2048 mixed step, per launch / units), taken with
+# the default launch shapes
 TRAFFIC_PER_UNIT_MIXED = {
-    "tri_x": 49.4, "update": 137.4, "flux_x": 41.0, "flux_y": 41.6, "disp_b": 72.6, "disp_a": 42.7,
-    "maskmul": 30.8, "tri_y": 95.2, "post_mask_break": 42.5,
+    "tri_x": 54.3, "update": 137.3, "flux_x": 42.0, "flux_y": 43.5, "disp_b": 73.1, "disp_a": 44.1,
+    "maskmul": 33.4, "tri_y": 54.5, "post_mask_break": 42.8,
 }
 # kernel launches per stage (tri_* count the partitioned solve as one)
 PER_STAGE = ["disp_a", "disp_b", "flux_x", "flux_y", "update", "tri_x", "tri_y", "post_mask_break", "post",

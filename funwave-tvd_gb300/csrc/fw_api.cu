@@ -1229,7 +1229,8 @@ int ens_build(fw_ensemble *e) {
         err = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
         // one branch: the other runs fill the GPU beside it (16 runs of uneven
-        // size, 4 steps: 7.9 ms, with two branches each 8.0)
+        // size, 4 steps: 7.9 ms, with two branches each 8.0; not measured with
+        // 512, where the runs' own two-branch graphs are 6 % ahead of this)
         c->one_branch = true;
         for (int s = 0; s < 2; s++) {
             if (c->p.precision == FW_PREC_FP64) enqueue_step<double>(c);

@@ -1272,7 +1272,7 @@ __device__ __forceinline__ T wavemaker_mass(const Grid &g, const Fields<T> &f, i
 // whole step sums the band's frequencies once, beside the first stage's
 // dispersion, into the words behind Cm.  Summed in every stage's k_update, the
 // warps of the band kept the others waiting (k_update at 2048 x 2048 128 ->
-// 112 us, 1024 x 1024 50 -> 37).  The words are zero until a first whole step.
+// 110 us, 1024 x 1024 50 -> 37).  The words are zero until a first whole step.
 template <typename T> __host__ __device__ __forceinline__ T *wm_band(const Grid &g, const Fields<T> &f) {
     return f.Cm + (size_t)g.nfreq * (size_t)(g.ihi - g.ilo + 1) * (size_t)(g.jhi - g.jlo + 1);
 }
@@ -2493,7 +2493,9 @@ __device__ __forceinline__ void fac_b_body(const Grid &g, const Fields<T> &f, co
 }
 
 // The multipliers of the parallel cyclic reduction of a line's reduced rows,
-// constant like the factors: per step a and b (n4 words each), then the last
+// constant like the factors (and computed with them: where MASK9 moves, at most
+// stages; with k_linesolve such a step of 1024 x 1024 takes 2522 us, 2701 with
+// the solves before it and no multipliers): per step a and b (n4 words each), then the last
 // diagonal; the operations are pcr_solve's.  They lie in the planes that only
 // the FP64 mode's dispersion terms use (eight consecutive planes from Uxx; at
 // most 19/8 words per cell and direction), x lines first.

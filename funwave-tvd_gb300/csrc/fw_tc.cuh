@@ -155,10 +155,10 @@ template <int M, int N> __host__ __device__ constexpr uint32_t idesc_bf16() {
 }
 
 // Issued by one lane of a warp that runs through it together: `me` is true on
-// that lane.  With the operands the same on every lane they stay in
-// uniform registers; issued from a branch that one lane takes, every operand
-// of every MMA is first moved there (about 100 cycles an MMA against 43: the
-// forward pass at 1 x 1024 x 1024 takes 156 us against 197).
+// that lane.  Issued from a branch that one lane takes, the forward pass at
+// 1 x 1024 x 1024 takes 197 us, like this 156 (a 32 -> 32 layer 102 cycles for
+// each of a CTA's MMAs, now 84; the likely cause, which no counter shows, is
+// that operands that are the same on every lane stay in uniform registers).
 __device__ __forceinline__ void tc_mma_by(uint32_t me, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
     asm volatile(
         "{\n.reg .pred p, q;\n"

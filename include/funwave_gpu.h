@@ -347,10 +347,12 @@ int fw_host_free(void *ptr);
 long long fw_launch_count(fw_ctx *ctx);
 /* Time nrep back-to-back launches of one kernel of the step with CUDA events
  * on the context stream; *ms_per_launch = average duration.  Names:
- * "disp_a","disp_b","flux_x","flux_y","update","tri_x","tri_y","post",
- * "mask","break_a","ghost","maskmul","begin".  Kernels that update state in
- * place (update, post, mask, maskmul, begin) change the state: time them on
- * a context whose state is disposable.  No reference counterpart. */
+ * "disp_a","disp_b","flux_x","flux_y","update","tri_x","tri_y",
+ * "post_mask_break","post","mask","break_a","ghost","maskmul","begin"
+ * ("maskmul" and "begin" with the ghost cells, as a step runs them; tri_* with
+ * their factorisation's early exit).  Kernels that update state in place
+ * (update, post, post_mask_break, mask, maskmul, begin) change the state: time
+ * them on a context whose state is disposable.  No reference counterpart. */
 int fw_time_kernel(fw_ctx *ctx, const char *name, int nrep, double *ms_per_launch);
 /* CUDA stream of the context, as a void* (cudaStream_t). */
 void *fw_stream(fw_ctx *ctx);
@@ -361,8 +363,8 @@ void *fw_stream(fw_ctx *ctx);
  * (bx a multiple of 32, bx*by <= 256), then the heights of the x-face and the
  * y-face flux kernels (8, 16 or 32 in MIXED; 8 or 16 in FP64), then how those
  * two work (0: by lines of a row and strips of a column, whose height sets the
- * rows of an x block and bounds a y strip; 1: by tiles of that height, staged
- * in shared memory by TMA tensor loads).  Every choice computes the same
+ * rows of an x block and bounds a y strip, in FP64 at twice the height; 1: by
+ * tiles of that height, staged in shared memory by TMA tensor loads).  Every choice computes the same
  * values bit for bit; only the speed differs.  Defaults: 32 x 8 blocks,
  * heights 8 and 32 (16 in FP64). */
 #define FW_TUNE_LEN 14
